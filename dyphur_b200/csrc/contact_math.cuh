@@ -432,4 +432,165 @@ __device__ __forceinline__ int solve_contact_reg(const GlobalBodies& B, const Co
     return res;
 }
 
+// ── one contact on two lanes ────────────────────────────────────────────────
+// Contact solves wait for one another in long chains of few contacts each, so
+// a solve's latency counts and lanes are idle. solve_contact's work is the same
+// on its two bodies up to sign, with a few scalars of both in between: lane
+// pair (2 i, 2 i + 1) takes contact i, each lane one body held in registers,
+// and the scalars cross by shuffles. Half the instructions per contact and no
+// shared-memory round trip between its steps. Every float is computed by the
+// same operations in the same order as in solve_contact (negating a factor or
+// a summand is exact), so the results are bit-identical.
+struct SideBody {
+    float px, py, pz, qw, qx, qy, qz, vx, vy, vz, wx, wy, wz;
+    float m, ixx, iyy, izz, ixy, ixz, iyz;
+};
+
+template <class Bodies>
+__device__ __forceinline__ SideBody load_side(const Bodies& B, uint32_t i) {
+    return SideBody{B.px(i), B.py(i), B.pz(i), B.qw(i), B.qx(i), B.qy(i), B.qz(i), B.vx(i), B.vy(i), B.vz(i),
+                    B.wx(i), B.wy(i), B.wz(i), B.im(i), B.ixx(i), B.iyy(i), B.izz(i), B.ixy(i), B.ixz(i), B.iyz(i)};
+}
+
+template <class Bodies>
+__device__ __forceinline__ void store_side(const Bodies& B, uint32_t i, const SideBody& s) {
+    B.px(i) = s.px; B.py(i) = s.py; B.pz(i) = s.pz;
+    B.qw(i) = s.qw; B.qx(i) = s.qx; B.qy(i) = s.qy; B.qz(i) = s.qz;
+    B.vx(i) = s.vx; B.vy(i) = s.vy; B.vz(i) = s.vz;
+    B.wx(i) = s.wx; B.wy(i) = s.wy; B.wz(i) = s.wz;
+}
+
+// World rotation rows of the body and the world inverse inertia times a vector
+// (world_inv_inertia).
+struct SideRot {
+    float R00, R01, R02, R10, R11, R12, R20, R21, R22;
+};
+__device__ __forceinline__ SideRot side_rot(const SideBody& b) {
+    const float qw = b.qw, qx = b.qx, qy = b.qy, qz = b.qz;
+    SideRot r;
+    r.R00 = 1.f - 2.f * (qy * qy + qz * qz); r.R01 = 2.f * (qx * qy + qz * qw); r.R02 = 2.f * (qx * qz - qy * qw);
+    r.R10 = 2.f * (qx * qy - qz * qw); r.R11 = 1.f - 2.f * (qx * qx + qz * qz); r.R12 = 2.f * (qy * qz + qx * qw);
+    r.R20 = 2.f * (qx * qz + qy * qw); r.R21 = 2.f * (qy * qz - qx * qw); r.R22 = 1.f - 2.f * (qx * qx + qy * qy);
+    return r;
+}
+__device__ __forceinline__ void side_inv_inertia(const SideRot& r, const SideBody& b, float vx, float vy, float vz,
+                                                 float& ox, float& oy, float& oz) {
+    const float lx = r.R00 * vx + r.R10 * vy + r.R20 * vz;
+    const float ly = r.R01 * vx + r.R11 * vy + r.R21 * vz;
+    const float lz = r.R02 * vx + r.R12 * vy + r.R22 * vz;
+    const float ilx = b.ixx * lx + b.ixy * ly + b.ixz * lz;
+    const float ily = b.ixy * lx + b.iyy * ly + b.iyz * lz;
+    const float ilz = b.ixz * lx + b.iyz * ly + b.izz * lz;
+    ox = r.R00 * ilx + r.R01 * ily + r.R02 * ilz;
+    oy = r.R10 * ilx + r.R11 * ily + r.R12 * ilz;
+    oz = r.R20 * ilx + r.R21 * ily + r.R22 * ilz;
+}
+
+// The other lane's value, and a pair's (body a's, body b's) values.
+__device__ __forceinline__ float other_side(float x) { return __shfl_xor_sync(0xffffffffu, x, 1); }
+__device__ __forceinline__ void both_sides(bool is_b, float mine, float& a, float& b) {
+    const float o = other_side(mine);
+    a = is_b ? o : mine;
+    b = is_b ? mine : o;
+}
+
+// solve_contact by lane pairs: `is_b` lanes hold body b in S, the others body
+// a. The whole warp calls it; pairs with `valid` false do nothing. Both lanes
+// of a pair return the same code, lambda and flags.
+__device__ __forceinline__ int solve_contact_side(bool valid, bool is_b, SideBody& S, const Contact& ct, float mu,
+                                                  float& lc, float dt, uint32_t* flags = nullptr) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const float depth = ct.depth;
+    const float remaining = depth - lc;
+    const bool wanted = valid && !(depth <= 0.f) && !(remaining <= 1e-6f);
+    if (!__any_sync(kAll, wanted)) return kSolveSkipped;
+    const float nx = ct.nx, ny = ct.ny, nz = ct.nz;
+    const float m = S.m, ms = is_b ? -m : m;  // the impulse acts with opposite signs
+    const bool dynamic = m != 0.f;
+    const float rx = ct.px - S.px, ry = ct.py - S.py, rz = ct.pz - S.pz;
+    const float rnx = ry * nz - rz * ny, rny = rz * nx - rx * nz, rnz = rx * ny - ry * nx;
+    float ix, iy, iz;
+    side_inv_inertia(side_rot(S), S, rnx, rny, rnz, ix, iy, iz);
+    float wa, wb, wa_ang, wb_ang;
+    both_sides(is_b, m, wa, wb);
+    both_sides(is_b, rnx * ix + rny * iy + rnz * iz, wa_ang, wb_ang);
+    const float w_total = wa + wb + wa_ang + wb_ang;
+    const bool act = wanted && !(w_total < 1e-10f);
+    uint32_t fl = act ? kSfActive : 0u;
+    if (act) {
+        const float dl = __fdiv_rn(remaining, w_total);
+        lc += remaining;
+        if (dynamic) {
+            S.px += ms * dl * nx; S.py += ms * dl * ny; S.pz += ms * dl * nz;
+            const float sdl = is_b ? -dl : dl;
+            const float ax = sdl * ix, ay = sdl * iy, az = sdl * iz;
+            const float qw = S.qw, qx = S.qx, qy = S.qy, qz = S.qz;
+            S.qw += 0.5f * (-ax * qx - ay * qy - az * qz);
+            S.qx += 0.5f * (ax * qw + ay * qz - az * qy);
+            S.qy += 0.5f * (-ax * qz + ay * qw + az * qx);
+            S.qz += 0.5f * (ax * qy - ay * qx + az * qw);
+        }
+    }
+    const SideRot rot = side_rot(S);
+    {
+        float vax, vbx, vay, vby, vaz, vbz;
+        both_sides(is_b, S.vx + S.wy * rz - S.wz * ry, vax, vbx);
+        both_sides(is_b, S.vy + S.wz * rx - S.wx * rz, vay, vby);
+        both_sides(is_b, S.vz + S.wx * ry - S.wy * rx, vaz, vbz);
+        const float vrel_n = (vax - vbx) * nx + (vay - vby) * ny + (vaz - vbz) * nz;
+        if (act && vrel_n < 0.f) {
+            fl |= kSfNormal;
+            if (dynamic) {
+                const float j_n = __fdiv_rn(-vrel_n, w_total);
+                float dx, dy, dz;
+                side_inv_inertia(rot, S, rnx, rny, rnz, dx, dy, dz);
+                const float sj = is_b ? -j_n : j_n;
+                S.vx += ms * j_n * nx; S.vy += ms * j_n * ny; S.vz += ms * j_n * nz;
+                S.wx += sj * dx; S.wy += sj * dy; S.wz += sj * dz;
+            }
+        }
+    }
+    if (mu > 0.f) {
+        float vax, vbx, vay, vby, vaz, vbz;
+        both_sides(is_b, S.vx + S.wy * rz - S.wz * ry, vax, vbx);
+        both_sides(is_b, S.vy + S.wz * rx - S.wx * rz, vay, vby);
+        both_sides(is_b, S.vz + S.wx * ry - S.wy * rx, vaz, vbz);
+        const float rvx = vax - vbx, rvy = vay - vby, rvz = vaz - vbz;
+        const float rvn = rvx * nx + rvy * ny + rvz * nz;
+        const float vt_x = rvx - rvn * nx, vt_y = rvy - rvn * ny, vt_z = rvz - rvn * nz;
+        const float vt2 = vt_x * vt_x + vt_y * vt_y + vt_z * vt_z;
+        const bool slides = act && vt2 > 1e-12f;
+        if (__any_sync(kAll, slides)) {
+            float vt_len = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
+            if (slides) {
+                vt_len = __fsqrt_rn(vt2);
+                tx = __fdiv_rn(vt_x, vt_len);
+                ty = __fdiv_rn(vt_y, vt_len);
+                tz = __fdiv_rn(vt_z, vt_len);
+            }
+            const float rtx = ry * tz - rz * ty, rty = rz * tx - rx * tz, rtz = rx * ty - ry * tx;
+            float fx, fy, fz;
+            side_inv_inertia(rot, S, rtx, rty, rtz, fx, fy, fz);
+            float ax, bx, ay, by, az, bz;
+            both_sides(is_b, rtx * fx, ax, bx);
+            both_sides(is_b, rty * fy, ay, by);
+            both_sides(is_b, rtz * fz, az, bz);
+            const float wt = wa + wb + ax + ay + az + bx + by + bz;
+            if (slides && wt > 1e-10f) {
+                const float j_n_static = __fdiv_rn(lc, dt * w_total);
+                float j_t = __fdiv_rn(vt_len, wt);
+                fl |= kSfFriction | (mu * j_n_static < j_t ? kSfClamped : 0u);
+                j_t = fminf(j_t, mu * j_n_static);
+                if (dynamic) {
+                    const float sj = is_b ? j_t : -j_t;
+                    S.vx -= ms * j_t * tx; S.vy -= ms * j_t * ty; S.vz -= ms * j_t * tz;
+                    S.wx += sj * fx; S.wy += sj * fy; S.wz += sj * fz;
+                }
+            }
+        }
+    }
+    if (flags) *flags = fl;
+    return act ? kSolveDone : (wanted ? kSolveDeferred : kSolveSkipped);
+}
+
 }  // namespace dyph
