@@ -27,26 +27,41 @@ namespace dyph {
 namespace {
 
 // Per-body rows the fused frame adds after the solver's rows: shape type and
-// flags, half extents (3), leaf box (6 floats).
-constexpr uint32_t kFrameBodyRows = 10;
+// flags, half extents (3), leaf box (4 words, see PairBox).
+constexpr uint32_t kFrameBodyRows = 8;
 
 __host__ __device__ __forceinline__ uint32_t frame_body_bytes(uint32_t nb) {
     const uint32_t ldb = (nb + 3u) & ~3u;
     return scene_body_bytes(nb) + kFrameBodyRows * 4u * ldb;
 }
 
-// Overlap bits of the candidate-pair search: body a has ceil((nb - 1 - a) /
-// 32) words, one per chunk of 32 partners b > a, laid out by ascending a.
-// S(t) = sum over u = 1..t of ceil(u / 32) = 16 q (q + 1) + (q + 1) r, t = 32 q + r.
-__host__ __device__ __forceinline__ uint32_t chunk_prefix(uint32_t t) {
-    const uint32_t q = t >> 5, r = t & 31u;
-    return 16u * q * (q + 1u) + (q + 1u) * r;
+// Overlap bits of the candidate-pair search: bit j of word (c, a) says whether
+// bodies a and b = 32 c + j > a overlap, for chunks c >= a / 32. Chunk c's words
+// are consecutive in a (a warp's lanes take consecutive a), 32 (c + 1) of them.
+__host__ __device__ __forceinline__ uint32_t overlap_chunks(uint32_t nb) { return (nb + 31u) >> 5; }
+__host__ __device__ __forceinline__ uint32_t overlap_mask_base(uint32_t c) { return 16u * c * (c + 1u); }
+
+// A leaf box for the pair search: the six fp16 bounds of leaf_box as
+// (mnx, mny), (mnz, -mxx), (-mxy, -mxz), so that the traversal's inclusive test
+// (core/src/broadphase.cpp:322-325) is six "greater than" comparisons of one
+// box's bounds with the other's facing ones, two to an instruction. The bounds
+// are fp16 numbers, so comparing them as fp16 is exact.
+__device__ __forceinline__ uint4 pair_box(uint4 leaf) {
+    return make_uint4(leaf.x, leaf.y ^ 0x80000000u, leaf.z ^ 0x80008000u, 0u);
 }
-__host__ __device__ __forceinline__ uint32_t overlap_mask_words(uint32_t nb) {
-    return nb ? chunk_prefix(nb - 1u) : 0u;
+// The facing bounds (mxx, mxy), (mxz, -mnx), (-mny, -mnz) of a pair box.
+__device__ __forceinline__ uint3 facing_box(uint4 p) {
+    const uint32_t mxx = (p.y >> 16) ^ 0x8000u, mxy = (p.z & 0xFFFFu) ^ 0x8000u, mxz = (p.z >> 16) ^ 0x8000u;
+    const uint32_t nx = (p.x & 0xFFFFu) ^ 0x8000u, ny = (p.x >> 16) ^ 0x8000u, nz = (p.y & 0xFFFFu) ^ 0x8000u;
+    return make_uint3(mxx | (mxy << 16), mxz | (nx << 16), ny | (nz << 16));
 }
-__host__ __device__ __forceinline__ uint32_t overlap_mask_base(uint32_t nb, uint32_t a) {
-    return chunk_prefix(nb - 1u) - chunk_prefix(nb - 1u - a);
+__device__ __forceinline__ __half2 half2_bits(uint32_t v) {
+    return __halves2half2(__ushort_as_half(static_cast<unsigned short>(v & 0xFFFFu)),
+                          __ushort_as_half(static_cast<unsigned short>(v >> 16)));
+}
+__device__ __forceinline__ bool pair_overlap(uint4 n, uint3 q) {
+    return (__hgt2_mask(half2_bits(n.x), half2_bits(q.x)) | __hgt2_mask(half2_bits(n.y), half2_bits(q.y)) |
+            __hgt2_mask(half2_bits(n.z), half2_bits(q.z))) == 0u;
 }
 
 struct FrameBufs {
@@ -148,7 +163,7 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
     const SceneSolverRows R = scene_solver_rows(fb, ldb);
     uint32_t* info = R.cnt + ldb;
     float* half = reinterpret_cast<float*>(info + ldb);
-    float* box = half + 3 * ldb;  // rows mnx, mny, mnz, mxx, mxy, mxz
+    uint4* box = reinterpret_cast<uint4*>(half + 3 * ldb);  // [ldb] pair boxes
     const SceneBodiesShaped SB{{fb, ldb}};
     const SceneShapes SS{info, half, ldb};
     const uint32_t pcap = F.pair_base[s + 1] - F.pair_base[s];
@@ -176,38 +191,47 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
             const float v[7] = {SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i)};
             for (int j = 0; j < 7; ++j) r[static_cast<size_t>(j) * adj->n_stride] = v[j];
         }
-        // leaf box from the integrated pose, kept as the exact floats of its fp16 bounds
-        const BoxF bx = unpack_box(leaf_box(SS.type(i), SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i),
-                                            SB.qy(i), SB.qz(i), SS.hx(i), SS.hy(i), SS.hz(i)));
-        box[i] = bx.mnx; box[ldb + i] = bx.mny; box[2 * ldb + i] = bx.mnz;
-        box[3 * ldb + i] = bx.mxx; box[4 * ldb + i] = bx.mxy; box[5 * ldb + i] = bx.mxz;
+        box[i] = pair_box(leaf_box(SS.type(i), SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
+                                   SS.hx(i), SS.hy(i), SS.hz(i)));
+        R.cnt[i] = 0u;
     }
     T.sync();
     phase_mark(T, P_, 0, t0);
     // ── candidate pairs: per body a, the partners b > a in ascending order ──
-    // The count pass keeps each 32-partner chunk's overlap bits at the end of
-    // the team's shared memory when they fit there, so the write pass reads
-    // them instead of testing the boxes again.
-    const uint32_t mask_words = overlap_mask_words(nb);
+    // Every (a, b) is tested: a lane holds one body a and meets 32 partners one
+    // after another, whose boxes the warp reads as broadcasts; the answers are
+    // the bits of one word and nothing waits inside the 32. A warp takes 32
+    // bodies and 32 partners at a time, so the triangle of pairs is split evenly
+    // over the team. Alone on its SM a 512-body scene takes 30 us for this phase
+    // and a 256-body one 10 us; with a warp on one body and a ballot per 32
+    // partners, each waiting for six loads, they took 222 and 64 us.
+    // The words go to the end of the team's shared memory when they fit there,
+    // so the write pass reads them instead of testing the boxes again.
+    const uint32_t chunks = overlap_chunks(nb), mask_words = overlap_mask_base(chunks);
     const uint32_t mask_off = (smem_bytes - 4u * mask_words) & ~15u;
     const bool keep_masks = 4u * mask_words <= smem_bytes && frame_body_bytes(nb) <= mask_off;
     uint32_t* masks = reinterpret_cast<uint32_t*>(smem + mask_off);
-    for (uint32_t a = T.warp(); a < nb; a += T.warps()) {
-        const BoxF q{box[a], box[ldb + a], box[2 * ldb + a], box[3 * ldb + a], box[4 * ldb + a], box[5 * ldb + a]};
-        uint32_t c = 0, w = overlap_mask_base(nb, a);
-        for (uint32_t j0 = a + 1; j0 < nb; j0 += 32u, ++w) {
-            const uint32_t j = j0 + lane;
-            bool ov = false;
-            if (j < nb) {
-                const BoxF n{box[j], box[ldb + j], box[2 * ldb + j], box[3 * ldb + j], box[4 * ldb + j],
-                             box[5 * ldb + j]};
-                ov = box_overlap(n, q);
-            }
-            const unsigned bal = __ballot_sync(0xffffffffu, ov);
-            if (keep_masks && lane == 0) masks[w] = bal;
-            c += __popc(bal);
+    // word (c, a) of this lane's a; partners past the scene's end do not overlap
+    auto overlap_word = [&](uint32_t c, uint32_t a, const uint3& q) -> uint32_t {
+        const uint32_t n_b = min(32u, nb - 32u * c);
+        uint32_t w = 0;
+        if (n_b == 32u) {
+#pragma unroll 8
+            for (uint32_t j = 0; j < 32u; ++j) w |= pair_overlap(box[32u * c + j], q) ? 1u << j : 0u;
+        } else {
+#pragma unroll 4
+            for (uint32_t j = 0; j < n_b; ++j) w |= pair_overlap(box[32u * c + j], q) ? 1u << j : 0u;
         }
-        if (lane == 0) R.cnt[a] = c;
+        if ((a >> 5) == c) w &= ~((2u << lane) - 1u);  // b > a
+        return a < nb ? w : 0u;
+    };
+    for (uint32_t c = 0, ga = T.warp();; ga += T.warps()) {
+        while (c < chunks && ga > c) ga -= ++c;  // chunk c meets body groups 0..c
+        if (c >= chunks) break;
+        const uint32_t a = 32u * ga + lane;
+        const uint32_t w = overlap_word(c, a, facing_box(box[min(a, nb - 1u)]));
+        if (keep_masks) masks[overlap_mask_base(c) + a] = w;
+        if (w) atomicAdd(&R.cnt[a], __popc(w));
     }
     if (T.leader()) sh.carry = 0u;
     T.sync();
@@ -235,27 +259,26 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
                            in_smem ? ldc : F.words_stride};
     // the masks survive the write pass unless the pairs themselves reach them
     const bool use_masks = keep_masks && (!in_smem || body_bytes + 4u * pwords <= mask_off);
-    for (uint32_t a = T.warp(); a < nb; a += T.warps()) {
-        const BoxF q{box[a], box[ldb + a], box[2 * ldb + a], box[3 * ldb + a], box[4 * ldb + a], box[5 * ldb + a]};
-        uint32_t pos = R.off[a], w = overlap_mask_base(nb, a);
-        for (uint32_t j0 = a + 1; j0 < nb && pos < P; j0 += 32u, ++w) {
-            const uint32_t j = j0 + lane;
-            unsigned bal;
-            if (use_masks) {
-                bal = masks[w];
-            } else {
-                bool ov = false;
-                if (j < nb) {
-                    const BoxF n{box[j], box[ldb + j], box[2 * ldb + j], box[3 * ldb + j], box[4 * ldb + j],
-                                 box[5 * ldb + j]};
-                    ov = box_overlap(n, q);
+    // a lane writes its body's partners; a word with many (a ground that comes
+    // first meets everything) is written by the whole warp
+    for (uint32_t ga = T.warp(); ga < chunks; ga += T.warps()) {
+        const uint32_t a = 32u * ga + lane;
+        const uint3 q = facing_box(box[min(a, nb - 1u)]);
+        uint32_t pos = a < nb ? R.off[a] : 0u;
+        for (uint32_t c = ga; c < chunks; ++c) {
+            uint32_t w = use_masks ? masks[overlap_mask_base(c) + a] : overlap_word(c, a, q);
+            for (unsigned many = __ballot_sync(0xffffffffu, __popc(w) > 8); many; many &= many - 1u) {
+                const int src = __ffs(static_cast<int>(many)) - 1;
+                const uint32_t wa = __shfl_sync(0xffffffffu, w, src), at0 = __shfl_sync(0xffffffffu, pos, src);
+                const uint32_t at = at0 + __popc(wa & ((1u << lane) - 1u));
+                if (((wa >> lane) & 1u) && at < P) pairs[at] = (32u * ga + src) | ((32u * c + lane) << 16);
+                if (static_cast<int>(lane) == src) {
+                    pos += __popc(w);
+                    w = 0u;
                 }
-                bal = __ballot_sync(0xffffffffu, ov);
             }
-            const bool ov = (bal >> lane) & 1u;
-            const uint32_t at = pos + __popc(bal & ((1u << lane) - 1u));
-            if (ov && at < P) pairs[at] = a | (j << 16);
-            pos += __popc(bal);
+            for (; w; w &= w - 1u, ++pos)
+                if (pos < P) pairs[pos] = a | ((32u * c + static_cast<uint32_t>(__ffs(static_cast<int>(w))) - 1u) << 16);
         }
     }
     T.sync();
