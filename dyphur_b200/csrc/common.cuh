@@ -50,7 +50,9 @@ __device__ __forceinline__ void raise_error(uint32_t code, uint32_t site = 0u) {
     if (atomicCAS(&g_device_error, 0u, code) == 0u) g_device_error_site = site;
 }
 
-__device__ __forceinline__ float rsqrt_ieee(float x) { return __fdiv_rn(1.0f, __fsqrt_rn(x)); }
+// 1 / sqrt(x), both correctly rounded (the correctly rounded reciprocal is the
+// correctly rounded quotient of 1).
+__device__ __forceinline__ float rsqrt_ieee(float x) { return __frcp_rn(__fsqrt_rn(x)); }
 
 __device__ __forceinline__ uint16_t f2h_bits(float f) { return __half_as_ushort(__float2half_rn(f)); }
 __device__ __forceinline__ float h2f_bits(uint16_t h) { return __half2float(__ushort_as_half(h)); }

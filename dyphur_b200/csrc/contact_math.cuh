@@ -23,32 +23,47 @@ __device__ __forceinline__ bool box_box_centroid(float acx, float acy, float acz
                                                  const float Be[3][3], const float Bh[3], Contact& out,
                                                  uint32_t* br = nullptr) {
     const float eps_par = 1e-5f;
-    float C[3][3];
-    float dx = bcx - acx, dy = bcy - acy, dz = bcz - acz;
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) C[i][j] = Ae[i][0] * Be[j][0] + Ae[i][1] * Be[j][1] + Ae[i][2] * Be[j][2];
+    const float dx = bcx - acx, dy = bcy - acy, dz = bcz - acz;
     SatBest best{1e30f, -1, 0, 0, 0.f, 1.f, 0.f};
+    // The axes of a group are tested together and a separating one ends the
+    // pair after it, so a group's square roots and sums overlap in time: the
+    // result is the same as that of a return at the first separating axis.
+    {
+        float ov[6], dl[6];
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-        if (!sat_axis(Ae[i][0], Ae[i][1], Ae[i][2], Ae, Ah, Be, Bh, dx, dy, dz, 0, i, 0, best)) return false;
+        for (int i = 0; i < 3; ++i) {
+            ov[i] = sat_overlap(Ae[i][0], Ae[i][1], Ae[i][2], Ae, Ah, Be, Bh, dx, dy, dz, dl[i]);
+            ov[3 + i] = sat_overlap(Be[i][0], Be[i][1], Be[i][2], Ae, Ah, Be, Bh, dx, dy, dz, dl[3 + i]);
+        }
+        if (ov[0] <= 0.f || ov[1] <= 0.f || ov[2] <= 0.f || ov[3] <= 0.f || ov[4] <= 0.f || ov[5] <= 0.f)
+            return false;
 #pragma unroll
-    for (int i = 0; i < 3; ++i)
-        if (!sat_axis(Be[i][0], Be[i][1], Be[i][2], Ae, Ah, Be, Bh, dx, dy, dz, 1, i, 0, best)) return false;
+        for (int i = 0; i < 3; ++i) sat_keep(ov[i], dl[i], Ae[i][0], Ae[i][1], Ae[i][2], 0, i, 0, best);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) sat_keep(ov[3 + i], dl[3 + i], Be[i][0], Be[i][1], Be[i][2], 1, i, 0, best);
+    }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
+        float ov[3], dl[3], l[3][3];
+        bool apart = false;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
-            float cx = Ae[i][1] * Be[j][2] - Ae[i][2] * Be[j][1];
-            float cy = Ae[i][2] * Be[j][0] - Ae[i][0] * Be[j][2];
-            float cz = Ae[i][0] * Be[j][1] - Ae[i][1] * Be[j][0];
-            float len2 = cx * cx + cy * cy + cz * cz;
-            if (len2 < eps_par * eps_par) continue;
-            float inv_l = rsqrt_ieee(len2);
-            if (!sat_axis(cx * inv_l, cy * inv_l, cz * inv_l, Ae, Ah, Be, Bh, dx, dy, dz, 2, i, j, best))
-                return false;
+            const float cx = Ae[i][1] * Be[j][2] - Ae[i][2] * Be[j][1];
+            const float cy = Ae[i][2] * Be[j][0] - Ae[i][0] * Be[j][2];
+            const float cz = Ae[i][0] * Be[j][1] - Ae[i][1] * Be[j][0];
+            const float len2 = cx * cx + cy * cy + cz * cz;
+            const bool parallel = len2 < eps_par * eps_par;  // no axis
+            const float inv_l = rsqrt_ieee(parallel ? 1.f : len2);
+            l[j][0] = cx * inv_l;
+            l[j][1] = cy * inv_l;
+            l[j][2] = cz * inv_l;
+            const float o = sat_overlap(l[j][0], l[j][1], l[j][2], Ae, Ah, Be, Bh, dx, dy, dz, dl[j]);
+            apart = apart || (!parallel && o <= 0.f);
+            ov[j] = parallel ? 1e30f : o;
         }
+        if (apart) return false;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) sat_keep(ov[j], dl[j], l[j][0], l[j][1], l[j][2], 2, i, j, best);
     }
     const float bnx = best.nx, bny = best.ny, bnz = best.nz;
     float sx_acc = 0.f, sy_acc = 0.f, sz_acc = 0.f, sd_acc = 0.f;
@@ -58,12 +73,20 @@ __device__ __forceinline__ bool box_box_centroid(float acx, float acy, float acz
                     (static_cast<uint32_t>(best.j) << 4);
     if (best_type == 0 || best_type == 1) {
         if (best_type == 0) {
-            int t0A = (best_i + 1) % 3, t1A = (best_i + 2) % 3;
+            // the B face most parallel to A's axis, if it is larger
+            const float ax = pick3(best_i, Ae[0][0], Ae[1][0], Ae[2][0]);
+            const float ay = pick3(best_i, Ae[0][1], Ae[1][1], Ae[2][1]);
+            const float az = pick3(best_i, Ae[0][2], Ae[1][2], Ae[2][2]);
+            const float c0 = fabsf(ax * Be[0][0] + ay * Be[0][1] + az * Be[0][2]);
+            const float c1 = fabsf(ax * Be[1][0] + ay * Be[1][1] + az * Be[1][2]);
+            const float c2 = fabsf(ax * Be[2][0] + ay * Be[2][1] + az * Be[2][2]);
             int j_best = 0;
-            for (int j = 1; j < 3; ++j)
-                if (fabsf(C[best_i][j]) > fabsf(C[best_i][j_best])) j_best = j;
-            int t0B = (j_best + 1) % 3, t1B = (j_best + 2) % 3;
-            if (Bh[t0B] * Bh[t1B] > Ah[t0A] * Ah[t1A]) { best_type = 1; best_i = j_best; }
+            if (c1 > c0) j_best = 1;
+            if (c2 > (j_best == 1 ? c1 : c0)) j_best = 2;
+            // products of the two other half extents, in (axis + 1, axis + 2) order
+            const float area_b = pick3(j_best, Bh[1] * Bh[2], Bh[2] * Bh[0], Bh[0] * Bh[1]);
+            const float area_a = pick3(best_i, Ah[1] * Ah[2], Ah[2] * Ah[0], Ah[0] * Ah[1]);
+            if (area_b > area_a) { best_type = 1; best_i = j_best; }
         }
         const bool a_is_ref = (best_type == 0);
         const int ref_ax = best_i;
@@ -81,59 +104,81 @@ __device__ __forceinline__ bool box_box_centroid(float acx, float acy, float acz
             Ih[r] = a_is_ref ? Bh[r] : Ah[r];
         }
         const float icx = a_is_ref ? bcx : acx, icy = a_is_ref ? bcy : acy, icz = a_is_ref ? bcz : acz;
-        const int t0 = (ref_ax + 1) % 3, t1 = (ref_ax + 2) % 3;
         const float rc_dot_n3 = rcx * bnx + rcy * bny + rcz * bnz;
         const float sign_depth = a_is_ref ? 1.f : -1.f;
-        float Rh_ref = Rh[0], Rh_t0 = Rh[1], Rh_t1 = Rh[2];
-        if (ref_ax == 1) { Rh_ref = Rh[1]; Rh_t0 = Rh[2]; Rh_t1 = Rh[0]; }
-        if (ref_ax == 2) { Rh_ref = Rh[2]; Rh_t0 = Rh[0]; Rh_t1 = Rh[1]; }
+        const float Rh_ref = pick3(ref_ax, Rh[0], Rh[1], Rh[2]);
+        const float Rh_t0 = pick3(ref_ax, Rh[1], Rh[2], Rh[0]), Rh_t1 = pick3(ref_ax, Rh[2], Rh[0], Rh[1]);
         float Rt0[3], Rt1[3];
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-            Rt0[q] = (t0 == 0) ? Re[0][q] : (t0 == 1 ? Re[1][q] : Re[2][q]);
-            Rt1[q] = (t1 == 0) ? Re[0][q] : (t1 == 1 ? Re[1][q] : Re[2][q]);
+            Rt0[q] = pick3(ref_ax, Re[1][q], Re[2][q], Re[0][q]);
+            Rt1[q] = pick3(ref_ax, Re[2][q], Re[0][q], Re[1][q]);
         }
+        // half edges of the incident box: a vertex is its centre plus or minus
+        // each (the reference's sign factors are exact, so a subtraction is the
+        // same float)
+        float E[3][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+            for (int q = 0; q < 3; ++q) E[r][q] = Ih[r] * Ie[r][q];
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-            float sx = (k & 1) ? 1.f : -1.f, sy = (k & 2) ? 1.f : -1.f, sz = (k & 4) ? 1.f : -1.f;
-            float vx = icx + sx * Ih[0] * Ie[0][0] + sy * Ih[1] * Ie[1][0] + sz * Ih[2] * Ie[2][0];
-            float vy = icy + sx * Ih[0] * Ie[0][1] + sy * Ih[1] * Ie[1][1] + sz * Ih[2] * Ie[2][1];
-            float vz = icz + sx * Ih[0] * Ie[0][2] + sy * Ih[1] * Ie[1][2] + sz * Ih[2] * Ie[2][2];
-            float v_dot_n = vx * bnx + vy * bny + vz * bnz;
-            float dv = Rh_ref + sign_depth * (v_dot_n - rc_dot_n3);
-            if (dv <= 0.f) continue;
-            float vx_rel = vx - rcx, vy_rel = vy - rcy, vz_rel = vz - rcz;
-            float qt0 = vx_rel * Rt0[0] + vy_rel * Rt0[1] + vz_rel * Rt0[2];
-            float qt1 = vx_rel * Rt1[0] + vy_rel * Rt1[1] + vz_rel * Rt1[2];
-            if (fabsf(qt0) > Rh_t0 + 1e-3f) continue;
-            if (fabsf(qt1) > Rh_t1 + 1e-3f) continue;
-            if (n_out < 4) {
-                word |= 1u << (10 + k);
-                // centroid accumulation in the reference's order (cx += opx[k] ...)
-                sx_acc += vx - sign_depth * dv * bnx;
-                sy_acc += vy - sign_depth * dv * bny;
-                sz_acc += vz - sign_depth * dv * bnz;
-                sd_acc += dv;
-                ++n_out;
-            }
+            float vx = (k & 1) ? icx + E[0][0] : icx - E[0][0];
+            float vy = (k & 1) ? icy + E[0][1] : icy - E[0][1];
+            float vz = (k & 1) ? icz + E[0][2] : icz - E[0][2];
+            vx = (k & 2) ? vx + E[1][0] : vx - E[1][0];
+            vy = (k & 2) ? vy + E[1][1] : vy - E[1][1];
+            vz = (k & 2) ? vz + E[1][2] : vz - E[1][2];
+            vx = (k & 4) ? vx + E[2][0] : vx - E[2][0];
+            vy = (k & 4) ? vy + E[2][1] : vy - E[2][1];
+            vz = (k & 4) ? vz + E[2][2] : vz - E[2][2];
+            const float v_dot_n = vx * bnx + vy * bny + vz * bnz;
+            const float dv = Rh_ref + sign_depth * (v_dot_n - rc_dot_n3);
+            const float vx_rel = vx - rcx, vy_rel = vy - rcy, vz_rel = vz - rcz;
+            const float qt0 = vx_rel * Rt0[0] + vy_rel * Rt0[1] + vz_rel * Rt0[2];
+            const float qt1 = vx_rel * Rt1[0] + vy_rel * Rt1[1] + vz_rel * Rt1[2];
+            const bool keep = !(dv <= 0.f) && !(fabsf(qt0) > Rh_t0 + 1e-3f) && !(fabsf(qt1) > Rh_t1 + 1e-3f) && n_out < 4;
+            // centroid accumulation in the reference's order (cx += opx[k] ...)
+            const float cx = sx_acc + (vx - sign_depth * dv * bnx);
+            const float cy = sy_acc + (vy - sign_depth * dv * bny);
+            const float cz = sz_acc + (vz - sign_depth * dv * bnz);
+            const float cd = sd_acc + dv;
+            sx_acc = keep ? cx : sx_acc;
+            sy_acc = keep ? cy : sy_acc;
+            sz_acc = keep ? cz : sz_acc;
+            sd_acc = keep ? cd : sd_acc;
+            word |= keep ? 1u << (10 + k) : 0u;
+            n_out += keep ? 1 : 0;
         }
     } else {
         const int i = best.i, j = best.j;
-        const int t0A = (i + 1) % 3, t1A = (i + 2) % 3;
-        const float s0A = (-bnx * Ae[t0A][0] - bny * Ae[t0A][1] - bnz * Ae[t0A][2]) >= 0.f ? 1.f : -1.f;
-        const float s1A = (-bnx * Ae[t1A][0] - bny * Ae[t1A][1] - bnz * Ae[t1A][2]) >= 0.f ? 1.f : -1.f;
-        float pAx = acx + s0A * Ah[t0A] * Ae[t0A][0] + s1A * Ah[t1A] * Ae[t1A][0];
-        float pAy = acy + s0A * Ah[t0A] * Ae[t0A][1] + s1A * Ah[t1A] * Ae[t1A][1];
-        float pAz = acz + s0A * Ah[t0A] * Ae[t0A][2] + s1A * Ah[t1A] * Ae[t1A][2];
-        const int t0B = (j + 1) % 3, t1B = (j + 2) % 3;
-        const float s0B = (bnx * Be[t0B][0] + bny * Be[t0B][1] + bnz * Be[t0B][2]) >= 0.f ? 1.f : -1.f;
-        const float s1B = (bnx * Be[t1B][0] + bny * Be[t1B][1] + bnz * Be[t1B][2]) >= 0.f ? 1.f : -1.f;
-        float pBx = bcx + s0B * Bh[t0B] * Be[t0B][0] + s1B * Bh[t1B] * Be[t1B][0];
-        float pBy = bcy + s0B * Bh[t0B] * Be[t0B][1] + s1B * Bh[t1B] * Be[t1B][1];
-        float pBz = bcz + s0B * Bh[t0B] * Be[t0B][2] + s1B * Bh[t1B] * Be[t1B][2];
-        float uAx = Ae[i][0], uAy = Ae[i][1], uAz = Ae[i][2];
-        float uBx = Be[j][0], uBy = Be[j][1], uBz = Be[j][2];
-        float b12 = C[i][j];
+        // the edges' directions and the two other axes of each box, in (axis + 1, axis + 2) order
+        float uA[3], uB[3], a0[3], a1[3], b0[3], b1[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            uA[q] = pick3(i, Ae[0][q], Ae[1][q], Ae[2][q]);
+            a0[q] = pick3(i, Ae[1][q], Ae[2][q], Ae[0][q]);
+            a1[q] = pick3(i, Ae[2][q], Ae[0][q], Ae[1][q]);
+            uB[q] = pick3(j, Be[0][q], Be[1][q], Be[2][q]);
+            b0[q] = pick3(j, Be[1][q], Be[2][q], Be[0][q]);
+            b1[q] = pick3(j, Be[2][q], Be[0][q], Be[1][q]);
+        }
+        const float Ah0 = pick3(i, Ah[1], Ah[2], Ah[0]), Ah1 = pick3(i, Ah[2], Ah[0], Ah[1]);
+        const float Bh0 = pick3(j, Bh[1], Bh[2], Bh[0]), Bh1 = pick3(j, Bh[2], Bh[0], Bh[1]);
+        const float s0A = (-bnx * a0[0] - bny * a0[1] - bnz * a0[2]) >= 0.f ? 1.f : -1.f;
+        const float s1A = (-bnx * a1[0] - bny * a1[1] - bnz * a1[2]) >= 0.f ? 1.f : -1.f;
+        float pAx = acx + s0A * Ah0 * a0[0] + s1A * Ah1 * a1[0];
+        float pAy = acy + s0A * Ah0 * a0[1] + s1A * Ah1 * a1[1];
+        float pAz = acz + s0A * Ah0 * a0[2] + s1A * Ah1 * a1[2];
+        const float s0B = (bnx * b0[0] + bny * b0[1] + bnz * b0[2]) >= 0.f ? 1.f : -1.f;
+        const float s1B = (bnx * b1[0] + bny * b1[1] + bnz * b1[2]) >= 0.f ? 1.f : -1.f;
+        float pBx = bcx + s0B * Bh0 * b0[0] + s1B * Bh1 * b1[0];
+        float pBy = bcy + s0B * Bh0 * b0[1] + s1B * Bh1 * b1[1];
+        float pBz = bcz + s0B * Bh0 * b0[2] + s1B * Bh1 * b1[2];
+        const float uAx = uA[0], uAy = uA[1], uAz = uA[2];
+        const float uBx = uB[0], uBy = uB[1], uBz = uB[2];
+        float b12 = uAx * uBx + uAy * uBy + uAz * uBz;
         float denom = 1.f - b12 * b12;
         float wx = pAx - pBx, wy = pAy - pBy, wz = pAz - pBz;
         float d1 = wx * uAx + wy * uAy + wz * uAz;
@@ -155,7 +200,7 @@ __device__ __forceinline__ bool box_box_centroid(float acx, float acy, float acz
     }
     if (n_out == 0) return false;
     if (br) *br = word;
-    float inv = __fdiv_rn(1.f, static_cast<float>(n_out));
+    float inv = __frcp_rn(static_cast<float>(n_out));
     out.px = sx_acc * inv; out.py = sy_acc * inv; out.pz = sz_acc * inv;
     out.nx = bnx; out.ny = bny; out.nz = bnz;
     out.depth = sd_acc * inv;
@@ -172,20 +217,17 @@ __device__ __forceinline__ bool process_pair(const Bodies& B, const Shapes& S, u
     c.a = ia; c.b = ib;
     if (ta == kShapeSphere && tb == kShapeSphere)
         return sphere_sphere(B.px(ia), B.py(ia), B.pz(ia), S.hx(sha), B.px(ib), B.py(ib), B.pz(ib), S.hx(shb), c, br);
-    if (ta == kShapeSphere && tb == kShapeBox) {
-        float Be[3][3];
-        make_axes(B.qw(ib), B.qx(ib), B.qy(ib), B.qz(ib), Be);
-        if (!sphere_box(B.px(ia), B.py(ia), B.pz(ia), S.hx(sha), B.px(ib), B.py(ib), B.pz(ib), Be, S.hx(shb),
-                        S.hy(shb), S.hz(shb), c, br))
+    if ((ta == kShapeSphere && tb == kShapeBox) || (ta == kShapeBox && tb == kShapeSphere)) {
+        // one path for both orders, the normal flipped when the sphere comes first
+        const bool first = ta == kShapeSphere;
+        const uint32_t is = first ? ia : ib, ibx = first ? ib : ia, shs = first ? sha : shb, shx = first ? shb : sha;
+        float E[3][3];
+        make_axes(B.qw(ibx), B.qx(ibx), B.qy(ibx), B.qz(ibx), E);
+        if (!sphere_box(B.px(is), B.py(is), B.pz(is), S.hx(shs), B.px(ibx), B.py(ibx), B.pz(ibx), E, S.hx(shx),
+                        S.hy(shx), S.hz(shx), c, br))
             return false;
-        c.nx = -c.nx; c.ny = -c.ny; c.nz = -c.nz;
+        if (first) { c.nx = -c.nx; c.ny = -c.ny; c.nz = -c.nz; }
         return true;
-    }
-    if (ta == kShapeBox && tb == kShapeSphere) {
-        float Ae[3][3];
-        make_axes(B.qw(ia), B.qx(ia), B.qy(ia), B.qz(ia), Ae);
-        return sphere_box(B.px(ib), B.py(ib), B.pz(ib), S.hx(shb), B.px(ia), B.py(ia), B.pz(ia), Ae, S.hx(sha),
-                          S.hy(sha), S.hz(sha), c, br);
     }
     if (ta == kShapeBox && tb == kShapeBox) {
         float Ae[3][3], Be[3][3];

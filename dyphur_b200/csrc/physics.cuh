@@ -192,7 +192,7 @@ __device__ __forceinline__ bool sphere_sphere(float acx, float acy, float acz, f
     float dist = __fsqrt_rn(dist2);
     if (br) *br = dist < 1e-8f ? 1u : 0u;
     if (dist < 1e-8f) { c.nx = 0.f; c.ny = 1.f; c.nz = 0.f; }
-    else { float inv = __fdiv_rn(1.f, dist); c.nx = dx * inv; c.ny = dy * inv; c.nz = dz * inv; }
+    else { float inv = __frcp_rn(dist); c.nx = dx * inv; c.ny = dy * inv; c.nz = dz * inv; }
     c.depth = sum_r - dist;
     float sa = acx - c.nx * ra, sb = bcx + c.nx * rb;
     c.px = 0.5f * (sa + sb);
@@ -246,7 +246,7 @@ __device__ __forceinline__ bool sphere_box(float scx, float scy, float scz, floa
         *br = (q0 < -bh0 ? 16u : 0u) | (q0 > bh0 ? 32u : 0u) | (q1 < -bh1 ? 64u : 0u) | (q1 > bh1 ? 128u : 0u) |
               (q2 < -bh2 ? 256u : 0u) | (q2 > bh2 ? 512u : 0u);
     float dist = __fsqrt_rn(dist2);
-    float inv_d = __fdiv_rn(1.f, dist);
+    float inv_d = __frcp_rn(dist);
     float wx = lx * e0x + ly * e1x + lz * e2x;
     float wy = lx * e0y + ly * e1y + lz * e2y;
     float wz = lx * e0z + ly * e1z + lz * e2z;
@@ -258,32 +258,37 @@ __device__ __forceinline__ bool sphere_box(float scx, float scy, float scz, floa
     return true;
 }
 
-// One SAT axis: the SAT_TEST macro (narrowphase.cpp:158-175) and the edge
-// block (:192-208) evaluate the same expressions.
-struct SatBest {
-    float ov;
-    int type, i, j;
-    float nx, ny, nz;
-};
-__device__ __forceinline__ bool sat_axis(float lx, float ly, float lz, const float Ae[3][3], const float Ah[3],
-                                         const float Be[3][3], const float Bh[3], float dx, float dy, float dz,
-                                         int type, int i, int j, SatBest& best) {
+// One SAT axis l: the SAT_TEST macro (narrowphase.cpp:158-175) and the edge
+// block (:192-208) evaluate the same expressions. Returns the overlap and d . l.
+__device__ __forceinline__ float sat_overlap(float lx, float ly, float lz, const float Ae[3][3], const float Ah[3],
+                                             const float Be[3][3], const float Bh[3], float dx, float dy, float dz,
+                                             float& dl) {
     float rA = Ah[0] * fabsf(lx * Ae[0][0] + ly * Ae[0][1] + lz * Ae[0][2]) +
                Ah[1] * fabsf(lx * Ae[1][0] + ly * Ae[1][1] + lz * Ae[1][2]) +
                Ah[2] * fabsf(lx * Ae[2][0] + ly * Ae[2][1] + lz * Ae[2][2]);
     float rB = Bh[0] * fabsf(lx * Be[0][0] + ly * Be[0][1] + lz * Be[0][2]) +
                Bh[1] * fabsf(lx * Be[1][0] + ly * Be[1][1] + lz * Be[1][2]) +
                Bh[2] * fabsf(lx * Be[2][0] + ly * Be[2][1] + lz * Be[2][2]);
-    float t = fabsf(dx * lx + dy * ly + dz * lz);
-    float ov = rA + rB - t;
-    if (ov <= 0.f) return false;
-    if (ov < best.ov) {
-        best.ov = ov;
-        best.type = type; best.i = i; best.j = j;
-        float sgn = (dx * lx + dy * ly + dz * lz) >= 0.f ? -1.f : 1.f;
-        best.nx = sgn * lx; best.ny = sgn * ly; best.nz = sgn * lz;
-    }
-    return true;
+    dl = dx * lx + dy * ly + dz * lz;
+    return rA + rB - fabsf(dl);
 }
+
+// The axis of least overlap so far (strictly less, so the first of equals).
+struct SatBest {
+    float ov;
+    int type, i, j;
+    float nx, ny, nz;
+};
+__device__ __forceinline__ void sat_keep(float ov, float dl, float lx, float ly, float lz, int type, int i, int j,
+                                         SatBest& best) {
+    if (ov < best.ov) {
+        const float sgn = dl >= 0.f ? -1.f : 1.f;
+        best = SatBest{ov, type, i, j, sgn * lx, sgn * ly, sgn * lz};
+    }
+}
+
+// v[i] of three values in registers (an array indexed at run time would live
+// in local memory).
+__device__ __forceinline__ float pick3(int i, float v0, float v1, float v2) { return i == 0 ? v0 : (i == 1 ? v1 : v2); }
 
 }  // namespace dyph
