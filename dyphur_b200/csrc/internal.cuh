@@ -28,6 +28,10 @@ struct BvhBuffers {
     // left child (internal) or body (leaf); [2j+1] = lo, hi, escape node, 0.
     uint4* trav;            // [2(2n-1)]
     uint32_t* big;          // [2n-1] 1 when the subtree holds a static body's leaf
+    // Tiled pair search (single scenes):
+    uint4* leaf_box;        // [32 tiles] pair box and body of each leaf; bit 31 of the body word: a wide leaf
+    uint4* tile_box;        // [tiles] pair box around the tile's leaves that are not wide
+    uint32_t* wide;         // [n] wide leaves
     uint32_t* bucket_cnt;   // [n] candidate partners b > a found for body a
     uint32_t* bucket;       // [n * kBucket] first kBucket partners of body a (unordered)
     // Batched scenes only (null for one scene):
@@ -48,9 +52,10 @@ struct dyph_broadphase {
     uint32_t* codes = nullptr;   // Morton codes, sorted in place
     dyph::BvhBuffers bvh{};
     dyph_pair* pairs = nullptr;  // [max_pairs]
-    uint32_t* counts = nullptr;  // [0] stored pairs, [1] true pairs, [2] tile counter, [3] subtree queue length
+    uint32_t* counts = nullptr;  // [0] stored pairs, [1] true pairs, [2] tile counter, [3] subtree queue length / wide leaves,
+                                 // [4] 1 when a leaf box holds a NaN
     uint2* queue = nullptr;      // [16 max_bodies] (leaf, subtree) items of the pair search's second pass
-    uint32_t* tstatus = nullptr; // traversal look-back status, one word per 256 bodies
+    uint32_t* tstatus = nullptr; // pair writer's look-back status, one word per 64 bodies
     void* sort_ws = nullptr;
     size_t sort_ws_bytes = 0;
     uint32_t n_scenes = 0;              // 0: one scene (bounds passed per build)

@@ -171,6 +171,29 @@ __device__ __forceinline__ bool box_overlap(const BoxF& n, const BoxF& q) {
              n.mxz < q.mnz);
 }
 
+// A leaf box for the pair searches: the six fp16 bounds of leaf_box as
+// (mnx, mny), (mnz, -mxx), (-mxy, -mxz), so that the traversal's inclusive test
+// (core/src/broadphase.cpp:322-325) is six "greater than" comparisons of one
+// box's bounds with the other's facing ones, two to an instruction. The bounds
+// are fp16 numbers, so comparing them as fp16 is exact.
+__device__ __forceinline__ uint4 pair_box(uint4 leaf) {
+    return make_uint4(leaf.x, leaf.y ^ 0x80000000u, leaf.z ^ 0x80008000u, 0u);
+}
+// The facing bounds (mxx, mxy), (mxz, -mnx), (-mny, -mnz) of a pair box.
+__device__ __forceinline__ uint3 facing_box(uint4 p) {
+    const uint32_t mxx = (p.y >> 16) ^ 0x8000u, mxy = (p.z & 0xFFFFu) ^ 0x8000u, mxz = (p.z >> 16) ^ 0x8000u;
+    const uint32_t nx = (p.x & 0xFFFFu) ^ 0x8000u, ny = (p.x >> 16) ^ 0x8000u, nz = (p.y & 0xFFFFu) ^ 0x8000u;
+    return make_uint3(mxx | (mxy << 16), mxz | (nx << 16), ny | (nz << 16));
+}
+__device__ __forceinline__ __half2 half2_bits(uint32_t v) {
+    return __halves2half2(__ushort_as_half(static_cast<unsigned short>(v & 0xFFFFu)),
+                          __ushort_as_half(static_cast<unsigned short>(v >> 16)));
+}
+__device__ __forceinline__ bool pair_overlap(uint4 n, uint3 q) {
+    return (__hgt2_mask(half2_bits(n.x), half2_bits(q.x)) | __hgt2_mask(half2_bits(n.y), half2_bits(q.y)) |
+            __hgt2_mask(half2_bits(n.z), half2_bits(q.z))) == 0u;
+}
+
 // ── narrowphase primitives (core/src/narrowphase.cpp) ───────────────────────
 
 // make_axes (narrowphase.cpp:913-917): row k = body axis k in world space.
