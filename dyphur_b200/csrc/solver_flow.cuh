@@ -40,6 +40,12 @@ __device__ __forceinline__ uint64_t ld_relaxed_u64(const unsigned long long* p) 
     asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void ld_relaxed_2u64(const unsigned long long* p, uint64_t& a, uint64_t& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_relaxed_2u64(unsigned long long* p, uint64_t a, uint64_t b) {
+    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
+}
 __device__ __forceinline__ void st_relaxed_u32(uint32_t* p, uint32_t v) {
     asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -73,55 +79,51 @@ struct FlowBufs {
     uint32_t* partial;           // [kFlowMaxBlocks] per-block sums of the offset scan
 };
 
-constexpr uint32_t kSeqOneBlock = 2048;  // sequential order up to this many contacts: the one-block kernel
+// Sequential order up to this many contacts: the one-block kernel, which has no
+// grid barriers but runs the chain in global memory. Frames with it and with the
+// dataflow kernel: 133 and 123 us at 129 contacts of a box stack, 265 and 169 at
+// 350, 677 and 294 at 1,833.
+constexpr uint32_t kSeqOneBlock = 128;
 constexpr int kFlowMaxBlocks = 4096;
 
-constexpr int kHandWords = 16;  // record stride (13 words used): 128 bytes
+constexpr int kHandWords = 16;  // record stride (14 words written): 128 bytes
 
 __device__ __forceinline__ uint64_t hand_word(uint32_t tag, float v) {
     return (static_cast<uint64_t>(tag) << 32) | __float_as_uint(v);
 }
 
-// Load a record into body slot j of L; true when all 13 words carry `tag`.
-// The last word is written last, so it is polled alone first: a waiting
-// contact then costs one 8-byte load per pass, not thirteen.
-__device__ __forceinline__ bool load_hand(const unsigned long long* r, uint32_t tag, LocalPair& L, int j) {
+// Load a record into S; true when all 13 words carry `tag`. The last word is
+// polled alone first: a waiting contact then costs one 8-byte load per pass.
+// Words go two to an access (each 8 bytes carry their own tag, so the halves
+// need not arrive together).
+__device__ __forceinline__ bool load_hand(const unsigned long long* r, uint32_t tag, SideBody& S) {
     if (static_cast<uint32_t>(ld_relaxed_u64(r + 12) >> 32) != tag) return false;
-    uint64_t w[13];
+    uint64_t w[14];
 #pragma unroll
-    for (int i = 0; i < 13; ++i) w[i] = ld_relaxed_u64(r + i);
+    for (int i = 0; i < 14; i += 2) ld_relaxed_2u64(r + i, w[i], w[i + 1]);
     bool ok = true;
 #pragma unroll
     for (int i = 0; i < 13; ++i) ok = ok && static_cast<uint32_t>(w[i] >> 32) == tag;
-    L.p[j][0] = __uint_as_float(static_cast<uint32_t>(w[0]));
-    L.p[j][1] = __uint_as_float(static_cast<uint32_t>(w[1]));
-    L.p[j][2] = __uint_as_float(static_cast<uint32_t>(w[2]));
-    L.q[j][0] = __uint_as_float(static_cast<uint32_t>(w[3]));
-    L.q[j][1] = __uint_as_float(static_cast<uint32_t>(w[4]));
-    L.q[j][2] = __uint_as_float(static_cast<uint32_t>(w[5]));
-    L.q[j][3] = __uint_as_float(static_cast<uint32_t>(w[6]));
-    L.v[j][0] = __uint_as_float(static_cast<uint32_t>(w[7]));
-    L.v[j][1] = __uint_as_float(static_cast<uint32_t>(w[8]));
-    L.v[j][2] = __uint_as_float(static_cast<uint32_t>(w[9]));
-    L.w[j][0] = __uint_as_float(static_cast<uint32_t>(w[10]));
-    L.w[j][1] = __uint_as_float(static_cast<uint32_t>(w[11]));
-    L.w[j][2] = __uint_as_float(static_cast<uint32_t>(w[12]));
+    auto f = [&](int i) { return __uint_as_float(static_cast<uint32_t>(w[i])); };
+    S.px = f(0); S.py = f(1); S.pz = f(2);
+    S.qw = f(3); S.qx = f(4); S.qy = f(5); S.qz = f(6);
+    S.vx = f(7); S.vy = f(8); S.vz = f(9);
+    S.wx = f(10); S.wy = f(11); S.wz = f(12);
     return ok;
 }
 
-__device__ __forceinline__ void store_hand(unsigned long long* r, uint32_t tag, const LocalPair& L, int j) {
-    const float f[13] = {L.p[j][0], L.p[j][1], L.p[j][2], L.q[j][0], L.q[j][1], L.q[j][2], L.q[j][3],
-                         L.v[j][0], L.v[j][1], L.v[j][2], L.w[j][0], L.w[j][1], L.w[j][2]};
+__device__ __forceinline__ void store_hand(unsigned long long* r, uint32_t tag, const SideBody& S) {
+    const float f[14] = {S.px, S.py, S.pz, S.qw, S.qx, S.qy, S.qz, S.vx, S.vy, S.vz, S.wx, S.wy, S.wz, 0.f};
 #pragma unroll
-    for (int i = 0; i < 13; ++i) st_relaxed_u64(r + i, hand_word(tag, f[i]));
+    for (int i = 0; i < 14; i += 2) st_relaxed_2u64(r + i, hand_word(tag, f[i]), hand_word(tag, f[i + 1]));
 }
 
 // The 13 state floats of body bi from the SoA arrays.
-__device__ __forceinline__ void load_state(const GlobalBodies& B, uint32_t bi, LocalPair& L, int j) {
-    L.p[j][0] = B.px(bi); L.p[j][1] = B.py(bi); L.p[j][2] = B.pz(bi);
-    L.q[j][0] = B.qw(bi); L.q[j][1] = B.qx(bi); L.q[j][2] = B.qy(bi); L.q[j][3] = B.qz(bi);
-    L.v[j][0] = B.vx(bi); L.v[j][1] = B.vy(bi); L.v[j][2] = B.vz(bi);
-    L.w[j][0] = B.wx(bi); L.w[j][1] = B.wy(bi); L.w[j][2] = B.wz(bi);
+__device__ __forceinline__ void load_state(const GlobalBodies& B, uint32_t bi, SideBody& S) {
+    S.px = B.px(bi); S.py = B.py(bi); S.pz = B.pz(bi);
+    S.qw = B.qw(bi); S.qx = B.qx(bi); S.qy = B.qy(bi); S.qz = B.qz(bi);
+    S.vx = B.vx(bi); S.vy = B.vy(bi); S.vz = B.vz(bi);
+    S.wx = B.wx(bi); S.wy = B.wy(bi); S.wz = B.wz(bi);
 }
 
 // Sort a thread's items (at most kFlowItems) by key, ascending.
@@ -438,70 +440,72 @@ __global__ void __launch_bounds__(kFlowThreads) flow_solve_kernel(dyph_contacts 
             stamp(meta, gtid, 2);
         }
         n_items = 0;
-        for (uint32_t k = gtid; k < nc; k += gstride) item[n_items++] = k;
+        // a lane pair's contacts lie half a stride apart: one that waits holds up
+        // only contacts far after it
+        for (uint32_t k = (gtid >> 1) + (gtid & 1u) * (gstride >> 1); k < nc; k += gstride) {
+            item[n_items] = k;
+            key[n_items++] = k;
+        }
         if (!link_sequential(F, cv, B, nc, nb, bar, s_red, s_scan, gtid, gstride)) return;
     }
     stamp(meta, gtid, 3);
 
     // ── sweeps: each contact after the lower-colour contacts of its two bodies ──
-    // A contact takes each dynamic body's state from its list predecessor's
-    // record (or from the arrays when it is first), solves on registers, and
-    // publishes the two bodies' new states in its own records. A record is
-    // complete when all its words carry the pass's tag: no flag, no fence.
+    // A lane pair takes a contact, one body each (solve_contact_side): each lane
+    // takes its body's state from its list predecessor's record (or from the
+    // arrays when it is first), and publishes the new state in its own record.
+    // A record is complete when all its words carry the pass's tag: no flag, no
+    // fence. The pair works through both lanes' contacts in ascending key order.
     bool deferred_any = false;
+    const bool is_b = threadIdx.x & 1u;
     for (int iter = 0; iter < n_iters; ++iter) {
         if (iter == 0 || deferred_any) {
             const uint32_t tag = tag_base + static_cast<uint32_t>(iter) + 1u;
             int cur = 0;
-            bool have = false, got_a = false, got_b = false;
-            uint32_t k = 0, la = kNoLink, lb = kNoLink;
-            bool da = false, db = false;
+            bool have = false, got = false, dynamic = false;
+            uint32_t k = 0, link = kNoLink;
             float lc = 0.f;
             Contact ct{};
-            LocalPair L;
+            SideBody S{};
             uint32_t idle = 0;
-            while (__any_sync(0xffffffffu, cur < n_items)) {
-                bool progressed = false;
-                if (cur < n_items) {
-                    if (!have) {
-                        k = item[cur];
-                        ct = load_contact(cv, k);
-                        L.m[0] = B.im(ct.a);
-                        L.m[1] = B.im(ct.b);
-                        da = L.m[0] != 0.f;
-                        db = L.m[1] != 0.f;
-                        L.I[0][0] = B.ixx(ct.a); L.I[0][1] = B.iyy(ct.a); L.I[0][2] = B.izz(ct.a);
-                        L.I[0][3] = B.ixy(ct.a); L.I[0][4] = B.ixz(ct.a); L.I[0][5] = B.iyz(ct.a);
-                        L.I[1][0] = B.ixx(ct.b); L.I[1][1] = B.iyy(ct.b); L.I[1][2] = B.izz(ct.b);
-                        L.I[1][3] = B.ixy(ct.b); L.I[1][4] = B.ixz(ct.b); L.I[1][5] = B.iyz(ct.b);
-                        la = da ? F.link[2 * k] : kNoLink;
-                        lb = db ? F.link[2 * k + 1] : kNoLink;
-                        got_a = la == kNoLink;
-                        got_b = lb == kNoLink;
-                        if (got_a) load_state(B, ct.a, L, 0);
-                        if (got_b) load_state(B, ct.b, L, 1);
-                        lc = lambda[k];
-                        have = true;
-                    }
-                    if (!got_a) got_a = load_hand(F.hand + static_cast<size_t>(la) * kHandWords, tag, L, 0);
-                    if (!got_b) got_b = load_hand(F.hand + static_cast<size_t>(lb) * kHandWords, tag, L, 1);
-                    if (got_a && got_b) {
-                        if (ct.depth > 0.f && ct.depth - lc > 1e-6f) {
-                            Contact lct = ct;
-                            lct.a = 0u;
-                            lct.b = 1u;
-                            if (solve_contact(LocalPairRef{&L}, lct, mu, lc, dt) == kSolveDeferred)
-                                meta[kMetaDeferred] = 1u;
-                            lambda[k] = lc;
-                        }
-                        if (da) store_hand(F.hand + static_cast<size_t>(2 * k) * kHandWords, tag, L, 0);
-                        if (db) store_hand(F.hand + static_cast<size_t>(2 * k + 1) * kHandWords, tag, L, 1);
-                        ++cur;
-                        have = false;
-                        progressed = true;
-                    }
+            while (true) {
+                // the pair's next contact: the lower of its lanes' next keys
+                const bool more = cur < n_items;
+                const uint32_t next = more ? item[cur] : kNoLink, next_key = more ? key[cur] : kNoLink;
+                const uint32_t o_next = __shfl_xor_sync(0xffffffffu, next, 1);
+                const uint32_t o_key = __shfl_xor_sync(0xffffffffu, next_key, 1);
+                if (!__any_sync(0xffffffffu, have || more)) break;
+                if (!have && (next != kNoLink || o_next != kNoLink)) {
+                    const bool lower = o_next == kNoLink || (next != kNoLink && (is_b ? next_key < o_key : next_key <= o_key));
+                    k = lower ? next : o_next;
+                    cur += lower ? 1 : 0;
+                    ct = load_contact(cv, k);
+                    const uint32_t bi = is_b ? ct.b : ct.a;
+                    S.m = B.im(bi);
+                    S.ixx = B.ixx(bi); S.iyy = B.iyy(bi); S.izz = B.izz(bi);
+                    S.ixy = B.ixy(bi); S.ixz = B.ixz(bi); S.iyz = B.iyz(bi);
+                    dynamic = S.m != 0.f;
+                    link = dynamic ? F.link[2 * k + (is_b ? 1u : 0u)] : kNoLink;
+                    got = link == kNoLink;
+                    if (got) load_state(B, bi, S);
+                    lc = lambda[k];
+                    have = true;
                 }
-                if (__any_sync(0xffffffffu, progressed)) {
+                if (have && !got) got = load_hand(F.hand + static_cast<size_t>(link) * kHandWords, tag, S);
+                const bool o_got = __shfl_xor_sync(0xffffffffu, static_cast<int>(got), 1) != 0;
+                const bool ready = have && got && o_got;
+                if (__any_sync(0xffffffffu, ready)) {
+                    const int res = solve_contact_side(ready, is_b, S, ct, mu, lc, dt);
+                    if (ready) {
+                        if (dynamic)
+                            store_hand(F.hand + static_cast<size_t>(2 * k + (is_b ? 1u : 0u)) * kHandWords, tag, S);
+                        if (!is_b) {
+                            if (res == kSolveDeferred) meta[kMetaDeferred] = 1u;
+                            if (res == kSolveDone) lambda[k] = lc;
+                        }
+                        have = false;
+                        got = false;
+                    }
                     idle = 0;
                 } else {
                     if (++idle > spin_limit()) {
@@ -517,9 +521,9 @@ __global__ void __launch_bounds__(kFlowThreads) flow_solve_kernel(dyph_contacts 
             // Each body's final state is its list tail's record.
             for (uint32_t x = gtid; x < nb; x += gstride) {
                 if (B.im(x) == 0.f || F.body_cnt[x] == 0u) continue;
-                LocalPair T;
-                load_hand(F.hand + static_cast<size_t>(F.tail[x]) * kHandWords, tag, T, 0);
-                store_local(B, x, T, 0);
+                SideBody T;
+                load_hand(F.hand + static_cast<size_t>(F.tail[x]) * kHandWords, tag, T);
+                store_side(B, x, T);
             }
         }
         if (!deferred_any) {
