@@ -386,8 +386,7 @@ __device__ __forceinline__ int solve_contact(const Bodies& B, const Contact& ct,
 namespace dyph {
 
 // The two bodies of one contact held in registers (index 0 = body a, 1 = body
-// b), so solve_contact's read-modify-writes stay on chip; only the 13 state
-// floats of a dynamic body are written back.
+// b), the reverse pass's pre-solve states.
 struct LocalPair {
     float p[2][3], q[2][4], v[2][3], w[2][3], m[2], I[2][6];
     __device__ __forceinline__ float& px(uint32_t i) { return p[i][0]; }
@@ -411,68 +410,6 @@ struct LocalPair {
     __device__ __forceinline__ float ixz(uint32_t i) const { return I[i][4]; }
     __device__ __forceinline__ float iyz(uint32_t i) const { return I[i][5]; }
 };
-
-// LocalPair's accessors are non-const; solve_contact takes `const Bodies&`,
-// so it is driven through this thin reference wrapper.
-struct LocalPairRef {
-    LocalPair* s;
-    __device__ __forceinline__ float& px(uint32_t i) const { return s->p[i][0]; }
-    __device__ __forceinline__ float& py(uint32_t i) const { return s->p[i][1]; }
-    __device__ __forceinline__ float& pz(uint32_t i) const { return s->p[i][2]; }
-    __device__ __forceinline__ float& qw(uint32_t i) const { return s->q[i][0]; }
-    __device__ __forceinline__ float& qx(uint32_t i) const { return s->q[i][1]; }
-    __device__ __forceinline__ float& qy(uint32_t i) const { return s->q[i][2]; }
-    __device__ __forceinline__ float& qz(uint32_t i) const { return s->q[i][3]; }
-    __device__ __forceinline__ float& vx(uint32_t i) const { return s->v[i][0]; }
-    __device__ __forceinline__ float& vy(uint32_t i) const { return s->v[i][1]; }
-    __device__ __forceinline__ float& vz(uint32_t i) const { return s->v[i][2]; }
-    __device__ __forceinline__ float& wx(uint32_t i) const { return s->w[i][0]; }
-    __device__ __forceinline__ float& wy(uint32_t i) const { return s->w[i][1]; }
-    __device__ __forceinline__ float& wz(uint32_t i) const { return s->w[i][2]; }
-    __device__ __forceinline__ float im(uint32_t i) const { return s->m[i]; }
-    __device__ __forceinline__ float ixx(uint32_t i) const { return s->I[i][0]; }
-    __device__ __forceinline__ float iyy(uint32_t i) const { return s->I[i][1]; }
-    __device__ __forceinline__ float izz(uint32_t i) const { return s->I[i][2]; }
-    __device__ __forceinline__ float ixy(uint32_t i) const { return s->I[i][3]; }
-    __device__ __forceinline__ float ixz(uint32_t i) const { return s->I[i][4]; }
-    __device__ __forceinline__ float iyz(uint32_t i) const { return s->I[i][5]; }
-};
-
-__device__ __forceinline__ void load_local(const GlobalBodies& B, uint32_t bi, LocalPair& L, int j) {
-    L.p[j][0] = B.px(bi); L.p[j][1] = B.py(bi); L.p[j][2] = B.pz(bi);
-    L.q[j][0] = B.qw(bi); L.q[j][1] = B.qx(bi); L.q[j][2] = B.qy(bi); L.q[j][3] = B.qz(bi);
-    L.v[j][0] = B.vx(bi); L.v[j][1] = B.vy(bi); L.v[j][2] = B.vz(bi);
-    L.w[j][0] = B.wx(bi); L.w[j][1] = B.wy(bi); L.w[j][2] = B.wz(bi);
-    L.m[j] = B.im(bi);
-    L.I[j][0] = B.ixx(bi); L.I[j][1] = B.iyy(bi); L.I[j][2] = B.izz(bi);
-    L.I[j][3] = B.ixy(bi); L.I[j][4] = B.ixz(bi); L.I[j][5] = B.iyz(bi);
-}
-
-__device__ __forceinline__ void store_local(const GlobalBodies& B, uint32_t bi, const LocalPair& L, int j) {
-    B.px(bi) = L.p[j][0]; B.py(bi) = L.p[j][1]; B.pz(bi) = L.p[j][2];
-    B.qw(bi) = L.q[j][0]; B.qx(bi) = L.q[j][1]; B.qy(bi) = L.q[j][2]; B.qz(bi) = L.q[j][3];
-    B.vx(bi) = L.v[j][0]; B.vy(bi) = L.v[j][1]; B.vz(bi) = L.v[j][2];
-    B.wx(bi) = L.w[j][0]; B.wy(bi) = L.w[j][1]; B.wz(bi) = L.w[j][2];
-}
-
-// solve_contact on register copies of the two bodies: the same arithmetic in
-// the same order, so the results are bit-identical to the global-memory form.
-__device__ __forceinline__ int solve_contact_reg(const GlobalBodies& B, const Contact& ct, float mu, float& lc,
-                                                 float dt) {
-    if (ct.depth <= 0.f || ct.depth - lc <= 1e-6f) return kSolveSkipped;
-    LocalPair L;
-    load_local(B, ct.a, L, 0);
-    load_local(B, ct.b, L, 1);
-    Contact lct = ct;
-    lct.a = 0u;
-    lct.b = 1u;
-    const int res = solve_contact(LocalPairRef{&L}, lct, mu, lc, dt);
-    if (res == kSolveDone) {
-        if (L.m[0] != 0.f) store_local(B, ct.a, L, 0);
-        if (L.m[1] != 0.f) store_local(B, ct.b, L, 1);
-    }
-    return res;
-}
 
 // ── one contact on two lanes ────────────────────────────────────────────────
 // Contact solves wait for one another in long chains of few contacts each, so
@@ -538,7 +475,11 @@ __device__ __forceinline__ void both_sides(bool is_b, float mine, float& a, floa
 
 // solve_contact by lane pairs: `is_b` lanes hold body b in S, the others body
 // a. The whole warp calls it; pairs with `valid` false do nothing. Both lanes
-// of a pair return the same code, lambda and flags.
+// of a pair return the same code, lambda and flags. kAhead takes the quotients
+// by w_total together before the position correction (the relative velocity
+// needs none of it): a shorter chain for more work, for callers that latency
+// bounds.
+template <bool kAhead = false>
 __device__ __forceinline__ int solve_contact_side(bool valid, bool is_b, SideBody& S, const Contact& ct, float mu,
                                                   float& lc, float dt, uint32_t* flags = nullptr) {
     constexpr unsigned kAll = 0xffffffffu;
@@ -559,8 +500,24 @@ __device__ __forceinline__ int solve_contact_side(bool valid, bool is_b, SideBod
     const float w_total = wa + wb + wa_ang + wb_ang;
     const bool act = wanted && !(w_total < 1e-10f);
     uint32_t fl = act ? kSfActive : 0u;
+    // contact velocities of a minus b along the normal
+    auto normal_velocity = [&]() {
+        float vax, vbx, vay, vby, vaz, vbz;
+        both_sides(is_b, S.vx + S.wy * rz - S.wz * ry, vax, vbx);
+        both_sides(is_b, S.vy + S.wz * rx - S.wx * rz, vay, vby);
+        both_sides(is_b, S.vz + S.wx * ry - S.wy * rx, vaz, vbz);
+        return (vax - vbx) * nx + (vay - vby) * ny + (vaz - vbz) * nz;
+    };
+    float vrel_n = 0.f, dl = 0.f, j_n = 0.f, j_n_static = 0.f;
+    if (kAhead) {
+        vrel_n = normal_velocity();
+        const float w_div = act ? w_total : 1.f;  // an idle pair divides by 1
+        dl = __fdiv_rn(act ? remaining : 1.f, w_div);
+        j_n = __fdiv_rn(act ? -vrel_n : 1.f, w_div);
+        j_n_static = __fdiv_rn(act ? lc + remaining : 1.f, act ? dt * w_div : 1.f);
+    }
     if (act) {
-        const float dl = __fdiv_rn(remaining, w_total);
+        if (!kAhead) dl = __fdiv_rn(remaining, w_total);
         lc += remaining;
         if (dynamic) {
             S.px += ms * dl * nx; S.py += ms * dl * ny; S.pz += ms * dl * nz;
@@ -574,22 +531,16 @@ __device__ __forceinline__ int solve_contact_side(bool valid, bool is_b, SideBod
         }
     }
     const SideRot rot = side_rot(S);
-    {
-        float vax, vbx, vay, vby, vaz, vbz;
-        both_sides(is_b, S.vx + S.wy * rz - S.wz * ry, vax, vbx);
-        both_sides(is_b, S.vy + S.wz * rx - S.wx * rz, vay, vby);
-        both_sides(is_b, S.vz + S.wx * ry - S.wy * rx, vaz, vbz);
-        const float vrel_n = (vax - vbx) * nx + (vay - vby) * ny + (vaz - vbz) * nz;
-        if (act && vrel_n < 0.f) {
-            fl |= kSfNormal;
-            if (dynamic) {
-                const float j_n = __fdiv_rn(-vrel_n, w_total);
-                float dx, dy, dz;
-                side_inv_inertia(rot, S, rnx, rny, rnz, dx, dy, dz);
-                const float sj = is_b ? -j_n : j_n;
-                S.vx += ms * j_n * nx; S.vy += ms * j_n * ny; S.vz += ms * j_n * nz;
-                S.wx += sj * dx; S.wy += sj * dy; S.wz += sj * dz;
-            }
+    if (!kAhead) vrel_n = normal_velocity();
+    if (act && vrel_n < 0.f) {
+        fl |= kSfNormal;
+        if (dynamic) {
+            if (!kAhead) j_n = __fdiv_rn(-vrel_n, w_total);
+            float dx, dy, dz;
+            side_inv_inertia(rot, S, rnx, rny, rnz, dx, dy, dz);
+            const float sj = is_b ? -j_n : j_n;
+            S.vx += ms * j_n * nx; S.vy += ms * j_n * ny; S.vz += ms * j_n * nz;
+            S.wx += sj * dx; S.wy += sj * dy; S.wz += sj * dz;
         }
     }
     if (mu > 0.f) {
@@ -619,7 +570,7 @@ __device__ __forceinline__ int solve_contact_side(bool valid, bool is_b, SideBod
             both_sides(is_b, rtz * fz, az, bz);
             const float wt = wa + wb + ax + ay + az + bx + by + bz;
             if (slides && wt > 1e-10f) {
-                const float j_n_static = __fdiv_rn(lc, dt * w_total);
+                if (!kAhead) j_n_static = __fdiv_rn(lc, dt * w_total);
                 float j_t = __fdiv_rn(vt_len, wt);
                 fl |= kSfFriction | (mu * j_n_static < j_t ? kSfClamped : 0u);
                 j_t = fminf(j_t, mu * j_n_static);

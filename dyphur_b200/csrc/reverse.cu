@@ -23,14 +23,22 @@
 namespace dyph {
 namespace {
 
+// The frames of a segment, last first: scenes do not depend on one another, so
+// a team takes its scene through all of them without waiting for the others.
 __global__ void __launch_bounds__(kSceneThreads, 2) scene_frame_reverse_kernel(SceneBufs S, FrameBufs F,
-                                                                               FrameParams P_, AdjRun A, AdjKeep K,
+                                                                               FrameParams P_, AdjSegment D,
                                                                                AdjFrame G,
                                                                                const uint32_t* __restrict__ items,
                                                                                uint32_t n_items) {
     for_each_item(items, n_items, S.smem_bytes,
-                  [&](const auto& T, uint32_t s, unsigned char* smem, uint32_t bytes, SceneShared& sh) {
-                      reverse_scene(T, s, smem, bytes, sh, S, F, P_, A, K, G);
+                  [&](Team& T, uint32_t s, unsigned char* smem, uint32_t bytes, SceneShared& sh) {
+                      const uint32_t len = P_.n_frames;
+                      for (uint32_t f = len; f-- > 0u;) {
+                          const float* st0 = f ? D.state1 + static_cast<size_t>(f - 1u) * 13u * D.n_stride : D.state0;
+                          const AdjSet& k = D.sets[f];
+                          reverse_scene(T, s, f + 1u == len, st0, smem, bytes, sh, S, F, P_, segment_run(D, f, len),
+                                        AdjKeep{k.words, k.mg}, G);
+                      }
                   });
 }
 

@@ -43,9 +43,8 @@ __device__ __forceinline__ void process_pair_adj(uint32_t ta, uint32_t tb, F3 xa
 }
 
 struct AdjFrame {
-    const float* gin;   // [13][n_stride] adjoint of the state at the frame's end
-    float* gout;        // [13][n_stride] adjoint of the state at the frame's start (work array)
-    float* gim;         // [n] inverse-mass adjoints, accumulated
+    float* g;    // [13][n_stride] adjoint of the state at the frame's end, then at its start
+    float* gim;  // [n] inverse-mass adjoints, accumulated
 };
 
 __device__ __forceinline__ float& grow(float* g, uint32_t stride, int r, uint32_t i) {
@@ -58,15 +57,42 @@ struct AdjKeep {
     uint32_t* mg;     // [2 n_scenes] contacts and groups of every scene
 };
 
+// One frame's record set.
+struct AdjSet {
+    float* rec;       // [kRecWords][rec_stride], AdjRun::rec
+    float* pose1;     // [7][n_stride]
+    float* qs;        // [4][n_stride]
+    uint32_t* words;  // AdjKeep::words
+    uint32_t* mg;     // AdjKeep::mg
+};
+
+// A segment of frames, one launch of the recording kernel and one of the
+// reverse kernel: frame j's record set is sets[j]; its start state is state0
+// for j = 0 and state1 + (j - 1) [13][n_stride] after that, which the recording
+// of frame j - 1 stores when `store` is set (else it is there already).
+struct AdjSegment {
+    const AdjSet* sets;
+    uint32_t rec_stride, n_stride;
+    uint32_t* flag;
+    const float* state0;
+    float* state1;
+    uint32_t store;
+};
+__device__ __forceinline__ AdjRun segment_run(const AdjSegment& D, uint32_t j, uint32_t len) {
+    const AdjSet& k = D.sets[j];
+    float* next = D.store && j + 1u < len ? D.state1 + static_cast<size_t>(j) * 13u * D.n_stride : nullptr;
+    return AdjRun{k.rec, D.rec_stride, k.pose1, k.qs, D.n_stride, D.flag, next};
+}
+
 // Recomputation of scene s's frame with recording (team T, `smem_bytes` of
 // shared memory at smem); F.words is K.words, so a scene whose words spill
 // writes them in place and the others copy theirs out.
-template <class Team>
-__device__ void record_scene(const Team& T, uint32_t s, unsigned char* smem, uint32_t smem_bytes, SceneShared& sh,
+template <bool kAhead>
+__device__ void record_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem, uint32_t smem_bytes, SceneShared& sh,
                              const SceneBufs& S, const FrameBufs& F, const FrameParams& P_, const AdjRun& A,
                              const AdjKeep& K) {
     FrameOut fo{};
-    const bool ok = frame_scene<true>(T, s, smem, smem_bytes, sh, S, F, P_, &A, &fo);
+    const bool ok = frame_scene<true, kAhead>(T, s, f, smem, smem_bytes, sh, S, F, P_, &A, &fo);
     const uint32_t m = ok ? fo.m : 0u, groups = ok ? fo.groups : 0u;
     const SceneContacts dst{K.words + F.contact_base[s] + s, F.words_stride};
     const SceneContacts& SC = fo.SC;
@@ -86,9 +112,10 @@ __device__ void record_scene(const Team& T, uint32_t s, unsigned char* smem, uin
     T.sync();
 }
 
-// The reverse pass of scene s's recorded frame by team T.
-template <class Team>
-__device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, uint32_t smem_bytes, SceneShared& sh,
+// The reverse pass of scene s's recorded frame by team T, from the state st0
+// ([13][n_stride]) at the frame's start. The first frame that a launch reverses
+// (`first`) stages the bodies' constant rows, the next ones find them.
+__device__ void reverse_scene(Team& T, uint32_t s, bool first, const float* st0, unsigned char* smem, uint32_t smem_bytes, SceneShared& sh,
                               const SceneBufs& S, const FrameBufs& F, const FrameParams& P_, const AdjRun& A,
                               const AdjKeep& K, const AdjFrame& G) {
     const uint32_t ns = A.n_stride, rs = A.rec_stride;
@@ -100,7 +127,7 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
     uint32_t* info = R.cnt + ldb;
     float* half = reinterpret_cast<float*>(info + ldb);
     // the bodies' constant rows, shape types, flags and half extents
-    {
+    if (first) {
         const GlobalBodies B{P_.gb};
         for (uint32_t i = T.rank(); i < nb; i += T.size()) {
             const uint32_t g = b0 + i, sh_i = P_.gb.shape[g];
@@ -143,10 +170,6 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
             recb[static_cast<size_t>(row) * ldc + k] = A.rec[cbase + k + static_cast<size_t>(row) * rs];
         }
     T.sync();
-    // ── adjoint of the frame's end state ──
-    for (uint32_t i = T.rank(); i < nb; i += T.size())
-        for (int r = 0; r < 13; ++r) grow(G.gout, ns, r, b0 + i) = G.gin[static_cast<size_t>(r) * ns + b0 + i];
-    T.sync();
     if (m > 0) {
         // ── renormalisations: q_end = renorm^n_iters(q_sweeps) ──
         for (uint32_t i = T.rank(); i < nb; i += T.size()) {
@@ -160,14 +183,14 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
                 ++kept;
             }
             if (n_it > 10) atomicOr(A.flag, 2u);
-            float g[4] = {grow(G.gout, ns, 3, b0 + i), grow(G.gout, ns, 4, b0 + i), grow(G.gout, ns, 5, b0 + i),
-                          grow(G.gout, ns, 6, b0 + i)};
+            float g[4] = {grow(G.g, ns, 3, b0 + i), grow(G.g, ns, 4, b0 + i), grow(G.g, ns, 5, b0 + i),
+                          grow(G.g, ns, 6, b0 + i)};
             for (int it = kept - 1; it >= 0; --it) {
                 float gi[4];
                 normalize_adj(chain[it], g, gi);
                 for (int c = 0; c < 4; ++c) g[c] = gi[c];
             }
-            for (int c = 0; c < 4; ++c) grow(G.gout, ns, 3 + c, b0 + i) = g[c];
+            for (int c = 0; c < 4; ++c) grow(G.g, ns, 3 + c, b0 + i) = g[c];
         }
         T.sync();
         // ── contact solves, last group first ──
@@ -196,10 +219,10 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
                 for (int j = 0; j < 2; ++j) {
                     const uint32_t gi = b0 + (j ? ib : ia);
                     BodyBar& Gj = *Gs[j];
-                    Gj.x = f3(grow(G.gout, ns, 0, gi), grow(G.gout, ns, 1, gi), grow(G.gout, ns, 2, gi));
-                    for (int c = 0; c < 4; ++c) Gj.q[c] = grow(G.gout, ns, 3 + c, gi);
-                    Gj.v = f3(grow(G.gout, ns, 7, gi), grow(G.gout, ns, 8, gi), grow(G.gout, ns, 9, gi));
-                    Gj.w = f3(grow(G.gout, ns, 10, gi), grow(G.gout, ns, 11, gi), grow(G.gout, ns, 12, gi));
+                    Gj.x = f3(grow(G.g, ns, 0, gi), grow(G.g, ns, 1, gi), grow(G.g, ns, 2, gi));
+                    for (int c = 0; c < 4; ++c) Gj.q[c] = grow(G.g, ns, 3 + c, gi);
+                    Gj.v = f3(grow(G.g, ns, 7, gi), grow(G.g, ns, 8, gi), grow(G.g, ns, 9, gi));
+                    Gj.w = f3(grow(G.g, ns, 10, gi), grow(G.g, ns, 11, gi), grow(G.g, ns, 12, gi));
                     Gj.im = 0.f;
                 }
                 F3 pb = f3(0.f, 0.f, 0.f), nb3 = pb;
@@ -210,13 +233,13 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
                     if (L.m[j] == 0.f) continue;  // a static body's state is not a variable
                     const uint32_t gi = b0 + (j ? ib : ia);
                     const BodyBar& Gj = *Gs[j];
-                    grow(G.gout, ns, 0, gi) = Gj.x.x; grow(G.gout, ns, 1, gi) = Gj.x.y;
-                    grow(G.gout, ns, 2, gi) = Gj.x.z;
-                    for (int c = 0; c < 4; ++c) grow(G.gout, ns, 3 + c, gi) = Gj.q[c];
-                    grow(G.gout, ns, 7, gi) = Gj.v.x; grow(G.gout, ns, 8, gi) = Gj.v.y;
-                    grow(G.gout, ns, 9, gi) = Gj.v.z;
-                    grow(G.gout, ns, 10, gi) = Gj.w.x; grow(G.gout, ns, 11, gi) = Gj.w.y;
-                    grow(G.gout, ns, 12, gi) = Gj.w.z;
+                    grow(G.g, ns, 0, gi) = Gj.x.x; grow(G.g, ns, 1, gi) = Gj.x.y;
+                    grow(G.g, ns, 2, gi) = Gj.x.z;
+                    for (int c = 0; c < 4; ++c) grow(G.g, ns, 3 + c, gi) = Gj.q[c];
+                    grow(G.g, ns, 7, gi) = Gj.v.x; grow(G.g, ns, 8, gi) = Gj.v.y;
+                    grow(G.g, ns, 9, gi) = Gj.v.z;
+                    grow(G.g, ns, 10, gi) = Gj.w.x; grow(G.g, ns, 11, gi) = Gj.w.y;
+                    grow(G.g, ns, 12, gi) = Gj.w.z;
                     G.gim[gi] += Gj.im;
                 }
                 float* w = recb + k;
@@ -243,21 +266,19 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
             if (SB.im(a) != 0.f) atomicAdd(&R.cnt[a], 1u);
             if (SB.im(b) != 0.f) atomicAdd(&R.cnt[b], 1u);
         }
-        if (T.leader()) sh.carry = 0u;
         T.sync();
+        uint32_t entries = 0;
         for (uint32_t base = 0; base < nb; base += T.size()) {
             const uint32_t i = base + T.rank();
             uint32_t tot;
             const uint32_t ex = T.exclusive_scan(i < nb ? R.cnt[i] : 0u, sh.scan, tot);
             if (i < nb) {
-                R.off[i] = sh.carry + ex;
+                R.off[i] = entries + ex;
                 R.cnt[i] = 0u;
             }
-            T.sync();
-            if (T.leader()) sh.carry += tot;
-            T.sync();
+            entries += tot;
         }
-        if (T.leader()) R.off[nb] = sh.carry;
+        if (T.leader()) R.off[nb] = entries;
         T.sync();
         for (uint32_t k = T.rank(); k < m; k += T.size()) {
             if (recb[k + 35ull * rst] == 0.f) continue;
@@ -312,7 +333,7 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
             const uint32_t gx = b0 + x;
             float acc[7];
 #pragma unroll
-            for (int c = 0; c < 7; ++c) acc[c] = grow(G.gout, ns, c, gx);
+            for (int c = 0; c < 7; ++c) acc[c] = grow(G.g, ns, c, gx);
             for (uint32_t e = lo; e < hi; ++e) {
                 const uint32_t k = entry(e);
                 const uint32_t side = (SC.ab(k) & 0xFFFFu) == x ? 0u : 7u;
@@ -321,56 +342,45 @@ __device__ void reverse_scene(const Team& T, uint32_t s, unsigned char* smem, ui
                 for (int c = 0; c < 7; ++c) acc[c] += r[static_cast<size_t>(side + c) * rst];
             }
 #pragma unroll
-            for (int c = 0; c < 7; ++c) grow(G.gout, ns, c, gx) = acc[c];
+            for (int c = 0; c < 7; ++c) grow(G.g, ns, c, gx) = acc[c];
         }
         T.sync();
     }
     // ── integration, from the state at the frame's start ──
-    const GlobalBodies B0{P_.gb};
+    auto row = [&](uint32_t r, uint32_t i) { return st0[static_cast<size_t>(r) * ns + i]; };
     for (uint32_t i = T.rank(); i < nb; i += T.size()) {
         const uint32_t gi = b0 + i;
         if (SB.im(i) == 0.f) {
-            for (int r = 0; r < 13; ++r) grow(G.gout, ns, r, gi) = 0.f;
+            for (int r = 0; r < 13; ++r) grow(G.g, ns, r, gi) = 0.f;
             continue;
         }
         if ((info[i] >> 8) & kFlagSleeping) continue;  // not integrated: identity
-        const Pose p0{B0.px(gi), B0.py(gi), B0.pz(gi), B0.qw(gi), B0.qx(gi), B0.qy(gi), B0.qz(gi),
-                      B0.vx(gi), B0.vy(gi), B0.vz(gi)};
-        F3 xb = f3(grow(G.gout, ns, 0, gi), grow(G.gout, ns, 1, gi), grow(G.gout, ns, 2, gi));
-        float qb[4] = {grow(G.gout, ns, 3, gi), grow(G.gout, ns, 4, gi), grow(G.gout, ns, 5, gi),
-                       grow(G.gout, ns, 6, gi)};
-        F3 vb = f3(grow(G.gout, ns, 7, gi), grow(G.gout, ns, 8, gi), grow(G.gout, ns, 9, gi));
-        F3 wb = f3(grow(G.gout, ns, 10, gi), grow(G.gout, ns, 11, gi), grow(G.gout, ns, 12, gi));
-        if (!integrate_body_adj(p0, B0.wx(gi), B0.wy(gi), B0.wz(gi), P_.gx, P_.gy, P_.gz, P_.sub_dt, P_.half_dt,
+        const Pose p0{row(0, gi), row(1, gi), row(2, gi), row(3, gi), row(4, gi),
+                      row(5, gi), row(6, gi), row(7, gi), row(8, gi), row(9, gi)};
+        F3 xb = f3(grow(G.g, ns, 0, gi), grow(G.g, ns, 1, gi), grow(G.g, ns, 2, gi));
+        float qb[4] = {grow(G.g, ns, 3, gi), grow(G.g, ns, 4, gi), grow(G.g, ns, 5, gi),
+                       grow(G.g, ns, 6, gi)};
+        F3 vb = f3(grow(G.g, ns, 7, gi), grow(G.g, ns, 8, gi), grow(G.g, ns, 9, gi));
+        F3 wb = f3(grow(G.g, ns, 10, gi), grow(G.g, ns, 11, gi), grow(G.g, ns, 12, gi));
+        if (!integrate_body_adj(p0, row(10, gi), row(11, gi), row(12, gi), P_.gx, P_.gy, P_.gz, P_.sub_dt, P_.half_dt,
                                 P_.n_substeps, xb, qb, vb, wb))
             atomicOr(A.flag, 4u);
-        grow(G.gout, ns, 0, gi) = xb.x; grow(G.gout, ns, 1, gi) = xb.y; grow(G.gout, ns, 2, gi) = xb.z;
-        for (int c = 0; c < 4; ++c) grow(G.gout, ns, 3 + c, gi) = qb[c];
-        grow(G.gout, ns, 7, gi) = vb.x; grow(G.gout, ns, 8, gi) = vb.y; grow(G.gout, ns, 9, gi) = vb.z;
-        grow(G.gout, ns, 10, gi) = wb.x; grow(G.gout, ns, 11, gi) = wb.y; grow(G.gout, ns, 12, gi) = wb.z;
+        grow(G.g, ns, 0, gi) = xb.x; grow(G.g, ns, 1, gi) = xb.y; grow(G.g, ns, 2, gi) = xb.z;
+        for (int c = 0; c < 4; ++c) grow(G.g, ns, 3 + c, gi) = qb[c];
+        grow(G.g, ns, 7, gi) = vb.x; grow(G.g, ns, 8, gi) = vb.y; grow(G.g, ns, 9, gi) = vb.z;
+        grow(G.g, ns, 10, gi) = wb.x; grow(G.g, ns, 11, gi) = wb.y; grow(G.g, ns, 12, gi) = wb.z;
     }
     T.sync();
 }
 
-// Work items as for scene_frame_kernel: a large scene per block, two
-// mid-size scenes on two warps each, or up to four small scenes, one per warp.
+// Work items as for scene_frame_kernel.
 template <class Fn>
 __device__ __forceinline__ void for_each_item(const uint32_t* items, uint32_t n_items, uint32_t smem_bytes, Fn&& fn) {
     extern __shared__ __align__(16) unsigned char scene_smem[];
-    __shared__ SceneShared sh[kSceneThreads / 32];
-    const uint32_t warp = threadIdx.x >> 5;
-    const uint32_t share = (smem_bytes / 4u) & ~15u;
+    __shared__ SceneShared sh[4];
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const uint32_t kind = items[4 * it + 1];
-        if (kind == kItemBlock) {
-            fn(BlockTeam{}, items[4 * it], scene_smem, smem_bytes, sh[0]);
-        } else if (kind == kItemHalf) {
-            const uint32_t half = warp >> 1, s = items[4 * it + 2 * half];
-            if (s != kItemEmpty) fn(HalfTeam{half}, s, scene_smem + half * 2u * share, 2u * share, sh[2 * half]);
-        } else {
-            const uint32_t s = items[4 * it + warp];
-            if (s != kItemEmpty) fn(WarpTeam{}, s, scene_smem + warp * share, share, sh[warp]);
-        }
+        ItemTeam t = item_team(items + 4 * it, smem_bytes);
+        if (t.scene != kItemEmpty) fn(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared]);
         __syncthreads();
     }
 }

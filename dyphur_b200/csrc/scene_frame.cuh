@@ -1,6 +1,7 @@
-// Batched scenes, fused: one thread block runs a whole frame of one scene —
+// Batched scenes, fused: one thread block runs whole frames of one scene —
 // integrate, pair search, narrowphase and contact solve — on the scene's
-// bodies in shared memory, and writes the bodies back once. Included by
+// bodies in shared memory, frame after frame, and writes the bodies back once
+// per launch. Included by
 // world.cu (after solver.cu in the library's translation unit).
 //
 // Every stage is the single-scene stage restated for one block:
@@ -69,17 +70,32 @@ struct SceneBodiesShaped : SceneBodies {
     __device__ __forceinline__ uint32_t shape(uint32_t i) const { return i; }
 };
 
-// Per-frame parameters of the fused kernel.
+// Words a launch's last frame leaves for frame_run_stats_kernel, which moves
+// them to the solver's meta words and clears them: largest colour + 1, JP
+// rounds, some scene coloured, some scene solved.
+constexpr int kAccMaxColor = 0, kAccRounds = 1, kAccColored = 2, kAccSolved = 3, kAccWords = 4;
+
+// Frames of one launch at most (the per-frame count words).
+constexpr uint32_t kMaxRunFrames = 256;
+
+// Parameters of the fused kernels, one launch.
 struct FrameParams {
     dyph_bodies gb;
     dyph_shapes gs;
     float gx, gy, gz, sub_dt, half_dt, mu, dt;
     int n_substeps, mode, n_iters;
-    uint32_t* meta;
-    uint32_t* bp_counts;
-    uint32_t* np_counts;
+    uint32_t* acc;     // [kAccWords]
+    uint32_t* counts;  // [4][n_frames] stored / true pairs, stored / true contacts of every frame, over all scenes
     uint32_t* status;
     unsigned long long* phase_ns;  // null, or [kFramePhases] device-clock ns summed over scenes
+    uint32_t n_frames;             // frames of this launch
+    uint32_t keep;                 // 1: the last frame's lists and statistics are kept (a call's last launch)
+    // Poses after frame traj_first + j traj_every, j < traj_count: row j of traj, [n][7].
+    float* traj;
+    uint32_t traj_first, traj_every, traj_count;
+    // State before frame ckpt_first + j ckpt_every: rows [13][n] at j of ckpt.
+    float* ckpt;
+    uint32_t ckpt_first, ckpt_every;
 };
 
 // Phases of a scene's fused frame, timed per scene by its team leader when
@@ -94,7 +110,6 @@ __device__ __forceinline__ uint64_t global_ns() {
     return t;
 }
 
-template <class Team>
 __device__ __forceinline__ void phase_mark(const Team& T, const FrameParams& P_, int k, uint64_t& t0) {
     if (P_.phase_ns && T.leader()) {
         const uint64_t t = global_ns();
@@ -117,19 +132,45 @@ struct AdjRun {
     float* store;        // [13][n_stride] the frame's end state (x, q, v, w), or null
 };
 
+// The 13 state rows of a scene's bodies into a [13][stride] buffer.
+__device__ __forceinline__ void scene_store_state(const Team& T, float* out, uint32_t stride, uint32_t b0, uint32_t nb,
+                                                  const SceneBodies& SB) {
+    for (uint32_t i = T.rank(); i < nb; i += T.size()) {
+        const float v[13] = {SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
+                             SB.vx(i), SB.vy(i), SB.vz(i), SB.wx(i), SB.wy(i), SB.wz(i)};
+#pragma unroll
+        for (int r = 0; r < 13; ++r) out[static_cast<size_t>(r) * stride + b0 + i] = v[r];
+    }
+}
+
+// The .trajectory rows (x, y, z, w, qx, qy, qz per body,
+// examples/stress_test_blocks/main.cpp:191-197) of a scene's bodies.
+__device__ __forceinline__ void scene_store_poses(const Team& T, float* out, uint32_t nb, const SceneBodies& SB) {
+    for (uint32_t i = T.rank(); i < nb; i += T.size()) {
+        const float v[7] = {SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i)};
+#pragma unroll
+        for (int r = 0; r < 7; ++r) out[7u * i + r] = v[r];
+    }
+}
+
 // What the adjoint pass needs of a recomputed frame.
 struct FrameOut {
     SceneContacts SC;
     uint32_t m, groups;
 };
 
-// One frame of scene s by team T with `smem_bytes` of shared memory at smem.
+// Frame f of P_.n_frames of scene s by team T with `smem_bytes` of shared
+// memory at smem. The first frame loads the scene's bodies, the next ones find
+// them in shared memory as the frame before left them, and the last one writes
+// them back; the lists in global memory and the solver's statistics are those
+// of a call's last frame, so the frames before it do not write them.
 // Returns false after raising an error. kRecord compiles the adjoint's
 // recording in (`adj_in`, `out`); the forward frame is built without it.
-template <bool kRecord = false, class Team>
-__device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint32_t smem_bytes, SceneShared& sh,
-                            const SceneBufs& S, const FrameBufs& F, const FrameParams& P_,
+template <bool kRecord, bool kAhead>
+__device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem, uint32_t smem_bytes,
+                            SceneShared& sh, const SceneBufs& S, const FrameBufs& F, const FrameParams& P_,
                             const AdjRun* adj_in = nullptr, FrameOut* out = nullptr) {
+    const bool end = f + 1u == P_.n_frames, last = end && P_.keep;
     const AdjRun* const adj = kRecord ? adj_in : nullptr;
     const GlobalBodies B{P_.gb};
     const uint32_t lane = threadIdx.x & 31u;
@@ -146,13 +187,21 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
     const uint32_t pcap = F.pair_base[s + 1] - F.pair_base[s];
     const uint32_t ccap = F.contact_base[s + 1] - F.contact_base[s];
     // ── stage and integrate ──
-    scene_load_bodies(T, B, b0, nb, fb, ldb);
+    if (f == 0u) {
+        scene_load_bodies(T, B, b0, nb, fb, ldb);
+        for (uint32_t i = T.rank(); i < nb; i += T.size()) {
+            const uint32_t g = b0 + i, sh_i = P_.gb.shape[g];
+            info[i] = P_.gs.type[sh_i] | (P_.gb.flags[g] << 8);
+            half[i] = P_.gs.half_x[sh_i];
+            half[ldb + i] = P_.gs.half_y[sh_i];
+            half[2 * ldb + i] = P_.gs.half_z[sh_i];
+        }
+    }
+    if (!adj && P_.ckpt && f >= P_.ckpt_first && (f - P_.ckpt_first) % P_.ckpt_every == 0u) {
+        const uint32_t j = (f - P_.ckpt_first) / P_.ckpt_every;
+        scene_store_state(T, P_.ckpt + static_cast<size_t>(j) * 13u * P_.gb.n, P_.gb.n, b0, nb, SB);
+    }
     for (uint32_t i = T.rank(); i < nb; i += T.size()) {
-        const uint32_t g = b0 + i, sh_i = P_.gb.shape[g];
-        info[i] = P_.gs.type[sh_i] | (P_.gb.flags[g] << 8);
-        half[i] = P_.gs.half_x[sh_i];
-        half[ldb + i] = P_.gs.half_y[sh_i];
-        half[2 * ldb + i] = P_.gs.half_z[sh_i];
         if (SB.im(i) != 0.f && !((info[i] >> 8) & kFlagSleeping)) {
             Pose p{SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
                    SB.vx(i), SB.vy(i), SB.vz(i)};
@@ -210,19 +259,17 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
         if (keep_masks) masks[overlap_mask_base(c) + a] = w;
         if (w) atomicAdd(&R.cnt[a], __popc(w));
     }
-    if (T.leader()) sh.carry = 0u;
     T.sync();
+    uint32_t p_true = 0;
     for (uint32_t base = 0; base < nb; base += T.size()) {
         const uint32_t i = base + T.rank();
         const uint32_t v = i < nb ? R.cnt[i] : 0u;
         uint32_t tot;
         const uint32_t ex = T.exclusive_scan(v, sh.scan, tot);
-        if (i < nb) R.off[i] = sh.carry + ex;
-        T.sync();
-        if (T.leader()) sh.carry += tot;
-        T.sync();
+        if (i < nb) R.off[i] = p_true + ex;
+        p_true += tot;
     }
-    const uint32_t p_true = sh.carry;
+    T.sync();
     const uint32_t P = min(p_true, pcap);
     // ── layout of the pairs and the contact words: shared memory if they fit ──
     const uint32_t cc = min(P, ccap);
@@ -259,13 +306,13 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
         }
     }
     T.sync();
-    if (in_smem && !adj)
+    if (in_smem && !adj && last)
         for (uint32_t p = T.rank(); p < P; p += T.size()) F.pair_raw[F.pair_base[s] + p] = pairs[p];
     phase_mark(T, P_, 1, t0);
     // ── narrowphase: contacts in pair order ──
     for (uint32_t i = T.rank(); i < nb; i += T.size()) R.cnt[i] = 0u;
-    if (T.leader()) sh.carry = 0u;
     T.sync();
+    uint32_t m_true = 0;
     const uint32_t cbase = F.contact_base[s];
     for (uint32_t base = 0; base < P; base += T.size()) {
         const uint32_t p = base + T.rank();
@@ -277,8 +324,8 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
             hit = process_pair(SB, SS, ab & 0xFFFFu, ab >> 16, c, adj ? &br : nullptr);
         }
         uint32_t tot;
-        const uint32_t ex = T.exclusive_scan(hit ? 1u : 0u, sh.scan, tot);
-        const uint32_t k = sh.carry + ex;
+        const uint32_t k = m_true + T.count_before(hit, sh.scan, tot);
+        m_true += tot;
         if (hit && k < cc) {
             SC.ab(k) = c.a | (c.b << 16);
             SC.lam(k) = 0.f;
@@ -290,7 +337,7 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
             const uint32_t slot = cbase + k, st = F.contact_slots;
             if (adj) {
                 adj->rec[27ull * adj->rec_stride + slot] = __uint_as_float(br);
-            } else {
+            } else if (last) {
                 F.contact_raw[slot] = b0 + c.a;
                 F.contact_raw[st + slot] = b0 + c.b;
                 F.contact_raw[2 * st + slot] = __float_as_uint(c.px);
@@ -302,21 +349,20 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
                 F.contact_raw[8 * st + slot] = __float_as_uint(c.depth);
             }
         }
-        T.sync();
-        if (T.leader()) sh.carry += tot;
-        T.sync();
     }
-    const uint32_t m_true = sh.carry, m = min(m_true, cc);
-    T.sync();  // every thread has read the count before scene_solve reuses sh.carry
+    const uint32_t m = min(m_true, cc);
+    T.sync();
     if (T.leader() && !adj) {
-        F.counts[4 * s + 0] = P;
-        F.counts[4 * s + 1] = p_true;
-        F.counts[4 * s + 2] = m;
-        F.counts[4 * s + 3] = m_true;
-        atomicAdd(&P_.bp_counts[0], P);
-        atomicAdd(&P_.bp_counts[1], p_true);
-        atomicAdd(&P_.np_counts[0], m);
-        atomicAdd(&P_.np_counts[1], m_true);
+        if (last) {
+            F.counts[4 * s + 0] = P;
+            F.counts[4 * s + 1] = p_true;
+            F.counts[4 * s + 2] = m;
+            F.counts[4 * s + 3] = m_true;
+        }
+        atomicAdd(&P_.counts[f], P);
+        atomicAdd(&P_.counts[P_.n_frames + f], p_true);
+        atomicAdd(&P_.counts[2u * P_.n_frames + f], m);
+        atomicAdd(&P_.counts[3u * P_.n_frames + f], m_true);
         // a scene past its own capacity keeps its ordered prefix, as it does alone
         if (p_true > pcap) atomicCAS(P_.status, 0u, static_cast<uint32_t>(DYPH_ERR_PAIR_OVERFLOW));
         if (m_true > ccap) atomicCAS(P_.status, 0u, static_cast<uint32_t>(DYPH_ERR_CONTACT_OVERFLOW));
@@ -329,71 +375,94 @@ __device__ bool frame_scene(const Team& T, uint32_t s, unsigned char* smem, uint
         SolveRecord rec{};
         if (adj) rec = SolveRecord{adj->rec, adj->rec_stride, cbase, adj->qs, adj->n_stride, b0, adj->flag};
         uint64_t t_sweep = 0;
-        if (!scene_solve<kRecord>(T, nb, m, SB, R, SC, P_.mode, P_.n_iters, P_.mu, P_.dt, sh, colored, n_colors, rounds,
+        if (!scene_solve<kRecord, kAhead>(T, nb, m, SB, R, SC, P_.mode, P_.n_iters, P_.mu, P_.dt, sh, colored, n_colors, rounds,
                          adj ? &rec : nullptr, &groups, P_.phase_ns ? &t_sweep : nullptr))
             return false;
         if (P_.phase_ns && T.leader()) {
             atomicAdd(&P_.phase_ns[3], static_cast<unsigned long long>(t_sweep - t0));
             t0 = t_sweep;
         }
-        if (!adj) {
+        if (!adj && last) {
             for (uint32_t k = T.rank(); k < m; k += T.size())
                 F.color_raw[cbase + k] = colored ? SC.done(k) : kUncolored;
-            scene_stats(T, P_.meta, colored, n_colors, rounds);
+            if (T.leader()) {
+                if (colored) {
+                    atomicMax(&P_.acc[kAccMaxColor], n_colors);
+                    P_.acc[kAccColored] = 1u;
+                }
+                atomicMax(&P_.acc[kAccRounds], rounds);
+                P_.acc[kAccSolved] = 1u;
+            }
         }
     }
     if (out) *out = FrameOut{SC, m, groups};
     phase_mark(T, P_, 4, t0);
     if (!adj) {
-        scene_store_bodies(T, B, b0, nb, SB);
-    } else if (adj->store) {
-        for (uint32_t i = T.rank(); i < nb; i += T.size()) {
-            const float v[13] = {SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
-                                 SB.vx(i), SB.vy(i), SB.vz(i), SB.wx(i), SB.wy(i), SB.wz(i)};
-#pragma unroll
-            for (int r = 0; r < 13; ++r) adj->store[static_cast<size_t>(r) * adj->n_stride + b0 + i] = v[r];
+        if (P_.traj && f >= P_.traj_first && (f - P_.traj_first) % P_.traj_every == 0u) {
+            const uint32_t j = (f - P_.traj_first) / P_.traj_every;
+            if (j < P_.traj_count)
+                scene_store_poses(T, P_.traj + (static_cast<size_t>(j) * P_.gb.n + b0) * 7u, nb, SB);
         }
+        if (end) scene_store_bodies(T, B, b0, nb, SB);
+    } else if (adj->store) {
+        scene_store_state(T, adj->store, adj->n_stride, b0, nb, SB);
     }
     T.sync();
     phase_mark(T, P_, 5, t0);
     return true;
 }
 
+// All frames of the launch of scene s: scenes do not depend on one another, so
+// a team takes its scene from frame to frame without waiting for the others.
+template <bool kAhead>
+__device__ __forceinline__ void run_scene(Team T, uint32_t s, unsigned char* smem, uint32_t smem_bytes,
+                                          SceneShared& sh, const SceneBufs& S, const FrameBufs& F,
+                                          const FrameParams& P_) {
+    for (uint32_t f = 0; f < P_.n_frames; ++f)
+        if (!frame_scene<false, kAhead>(T, s, f, smem, smem_bytes, sh, S, F, P_)) return;
+}
+
 // Work item i: items[4 i] a large scene solved by the whole block when
 // items[4 i + 1] == kItemBlock; two mid-size scenes items[4 i] and
-// items[4 i + 2], two warps and half the block's shared memory each, when
-// items[4 i + 1] == kItemHalf; otherwise up to four small scenes, one per
-// warp, each with a quarter of the shared memory. kItemEmpty marks an unused
-// team.
+// items[4 i + 2], half the block and its shared memory each, when
+// items[4 i + 1] == kItemHalf; otherwise up to four small scenes, a quarter of
+// the block and its shared memory each. kItemEmpty marks an unused team.
 constexpr uint32_t kItemEmpty = 0xFFFFFFFFu;
 constexpr uint32_t kItemBlock = 0xFFFFFFFEu;
 constexpr uint32_t kItemHalf = 0xFFFFFFFDu;
 
-// kMinBlocks is the register budget: 4 resident blocks per SM (128
-// registers a thread), 5 (96) or 6 (80, a few bytes spilled). Which one runs
-// best depends on the batch (dyph_world_autotune picks it with the shared
-// memory cap); all three compute the same frames.
-template <int kMinBlocks>
-__global__ void __launch_bounds__(kSceneThreads, kMinBlocks) scene_frame_kernel(SceneBufs S, FrameBufs F,
-                                                                                FrameParams P_,
-                                                                                const uint32_t* __restrict__ items,
-                                                                                uint32_t n_items) {
+// The calling thread's team of a work item: its scene, its part of the block's
+// shared memory and which of the block's SceneShared it uses.
+struct ItemTeam {
+    Team team;
+    uint32_t scene, smem, bytes, shared;
+};
+__device__ __forceinline__ ItemTeam item_team(const uint32_t* item, uint32_t smem_bytes) {
+    const uint32_t kind = item[1], share = (smem_bytes / 4u) & ~15u;
+    if (kind == kItemBlock) return ItemTeam{Team{blockDim.x, 0u}, item[0], 0u, smem_bytes, 0u};
+    const uint32_t quarter = threadIdx.x / (blockDim.x / 4u);
+    if (kind == kItemHalf) {
+        const uint32_t half = quarter >> 1;
+        return ItemTeam{Team{blockDim.x / 2u, 1u + half}, item[2 * half], half * 2u * share, 2u * share, 2u * half};
+    }
+    return ItemTeam{Team{blockDim.x / 4u, 3u + quarter}, item[quarter], quarter * share, share, quarter};
+}
+
+// kMinBlocks is the register budget: 4 resident blocks of kSceneThreads per SM
+// (128 registers a thread), 5 (96) or 6 (80, a few bytes spilled), or 2 of
+// kSceneWideThreads (128). Which one runs best depends on the batch
+// (dyph_world_autotune picks the budget with the shared memory cap; the wide
+// form's rule is in fused_threads); all compute the same frames.
+template <int kMinBlocks, int kThreads>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) scene_frame_kernel(SceneBufs S, FrameBufs F, FrameParams P_,
+                                                                           const uint32_t* __restrict__ items,
+                                                                           uint32_t n_items) {
     extern __shared__ __align__(16) unsigned char scene_smem[];
-    __shared__ SceneShared sh[kSceneThreads / 32];
-    const uint32_t warp = threadIdx.x >> 5;
-    const uint32_t share = (S.smem_bytes / 4u) & ~15u;
+    __shared__ SceneShared sh[4];
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-        const uint32_t kind = items[4 * it + 1];
-        if (kind == kItemBlock) {
-            frame_scene(BlockTeam{}, items[4 * it], scene_smem, S.smem_bytes, sh[0], S, F, P_);
-        } else if (kind == kItemHalf) {
-            const uint32_t half = warp >> 1, s = items[4 * it + 2 * half];
-            if (s != kItemEmpty)
-                frame_scene(HalfTeam{half}, s, scene_smem + half * 2u * share, 2u * share, sh[2 * half], S, F, P_);
-        } else {
-            const uint32_t s = items[4 * it + warp];
-            if (s != kItemEmpty) frame_scene(WarpTeam{}, s, scene_smem + warp * share, share, sh[warp], S, F, P_);
-        }
+        const ItemTeam t = item_team(items + 4 * it, S.smem_bytes);
+        if (t.scene != kItemEmpty)
+            run_scene<kThreads == kSceneWideThreads>(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared], S, F, P_);
         __syncthreads();
     }
 }

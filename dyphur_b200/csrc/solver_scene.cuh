@@ -29,7 +29,8 @@
 namespace dyph {
 namespace {
 
-constexpr int kSceneThreads = 128;
+constexpr int kSceneThreads = 128;      // threads of a block
+constexpr int kSceneWideThreads = 256;  // of the fused frame's larger form
 constexpr uint32_t kSceneNone = 0xFFFFFFFFu;
 constexpr uint32_t kSceneWords = 13;         // per-contact words (see SceneContacts)
 constexpr uint32_t kSceneMaxBodies = 65535;  // local body indices are 16 bits
@@ -115,30 +116,40 @@ struct SceneContacts {
     }
 };
 
-// A team of threads that runs one scene: the whole block (big scenes) or one
-// warp (small scenes, several to a block).
-struct BlockTeam {
-    __device__ __forceinline__ uint32_t rank() const { return threadIdx.x; }
-    __device__ __forceinline__ uint32_t size() const { return kSceneThreads; }
-    __device__ __forceinline__ uint32_t warp() const { return threadIdx.x >> 5; }
-    __device__ __forceinline__ uint32_t warps() const { return kSceneThreads / 32; }
-    __device__ __forceinline__ bool leader() const { return threadIdx.x == 0; }
-    __device__ __forceinline__ void sync() const { __syncthreads(); }
-    __device__ __forceinline__ bool any(bool p) const { return __syncthreads_or(p) != 0; }
-    __device__ __forceinline__ uint32_t exclusive_scan(uint32_t v, uint32_t* scratch, uint32_t& total) const {
-        return block_exclusive_scan<kSceneThreads>(v, scratch, total);
+// A team of threads that runs one scene: the whole block (big scenes), half of
+// it or a quarter (small scenes, several to a block). The size is a run-time
+// value, so that a kernel holds one copy of a frame's code: the teams of an SM
+// are in different phases of their frames, and a copy per kind of team pushed
+// one another out of the instruction cache. Teams are aligned to their size;
+// `bar` is the team's named barrier (0 the block's own, 1 and 2 the halves', 3
+// to 6 the quarters'; immediate ids, so that a kernel reserves seven).
+struct Team {
+    uint32_t n, bar;
+    uint32_t turn = 0;  // which scratch words the next scan takes
+    __device__ __forceinline__ uint32_t rank() const { return threadIdx.x & (n - 1u); }
+    __device__ __forceinline__ uint32_t size() const { return n; }
+    __device__ __forceinline__ uint32_t warp() const { return rank() >> 5; }
+    __device__ __forceinline__ uint32_t warps() const { return n >> 5; }
+    __device__ __forceinline__ bool leader() const { return rank() == 0u; }
+    __device__ __forceinline__ void sync() const {
+        if (n == 32u) {
+            __syncwarp();
+            return;
+        }
+        switch (bar) {
+            case 0: __syncthreads(); break;
+            case 1: asm volatile("bar.sync 1, %0;" ::"r"(n) : "memory"); break;
+            case 2: asm volatile("bar.sync 2, %0;" ::"r"(n) : "memory"); break;
+            case 3: asm volatile("bar.sync 3, %0;" ::"r"(n) : "memory"); break;
+            case 4: asm volatile("bar.sync 4, %0;" ::"r"(n) : "memory"); break;
+            case 5: asm volatile("bar.sync 5, %0;" ::"r"(n) : "memory"); break;
+            default: asm volatile("bar.sync 6, %0;" ::"r"(n) : "memory");
+        }
     }
-};
-
-struct WarpTeam {
-    __device__ __forceinline__ uint32_t rank() const { return threadIdx.x & 31u; }
-    __device__ __forceinline__ uint32_t size() const { return 32u; }
-    __device__ __forceinline__ uint32_t warp() const { return 0u; }
-    __device__ __forceinline__ uint32_t warps() const { return 1u; }
-    __device__ __forceinline__ bool leader() const { return (threadIdx.x & 31u) == 0u; }
-    __device__ __forceinline__ void sync() const { __syncwarp(); }
-    __device__ __forceinline__ bool any(bool p) const { return __any_sync(0xffffffffu, p) != 0; }
-    __device__ __forceinline__ uint32_t exclusive_scan(uint32_t v, uint32_t*, uint32_t& total) const {
+    // The exclusive prefix of v over the team and its total. A scan takes one
+    // barrier: two halves of the scratch alternate, and a thread that writes a
+    // half again has passed the barrier after everyone's reads of it.
+    __device__ __forceinline__ uint32_t exclusive_scan(uint32_t v, uint32_t* scratch, uint32_t& total) {
         const uint32_t lane = threadIdx.x & 31u;
         uint32_t x = v;
 #pragma unroll
@@ -146,64 +157,33 @@ struct WarpTeam {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
             if (lane >= static_cast<uint32_t>(d)) x += y;
         }
-        total = __shfl_sync(0xffffffffu, x, 31);
-        return x - v;
+        return finish_scan(x, x - v, scratch, total);
     }
-};
+    // The same of one bit per thread.
+    __device__ __forceinline__ uint32_t count_before(bool p, uint32_t* scratch, uint32_t& total) {
+        const uint32_t lane = threadIdx.x & 31u;
+        const unsigned m = __ballot_sync(0xffffffffu, p);
+        return finish_scan(__popc(m), __popc(m & ((1u << lane) - 1u)), scratch, total);
+    }
 
-// Two warps of a block (half 0: warps 0-1, half 1: warps 2-3), synchronised
-// on named barrier 1 + half; the block's own __syncthreads uses barrier 0.
-struct HalfTeam {
-    uint32_t half;
-    __device__ __forceinline__ uint32_t rank() const { return threadIdx.x & 63u; }
-    __device__ __forceinline__ uint32_t size() const { return 64u; }
-    __device__ __forceinline__ uint32_t warp() const { return (threadIdx.x >> 5) & 1u; }
-    __device__ __forceinline__ uint32_t warps() const { return 2u; }
-    __device__ __forceinline__ bool leader() const { return (threadIdx.x & 63u) == 0u; }
-    // Immediate barrier ids (the branch is uniform over the team), so the
-    // kernel reserves barriers 0-2 only.
-    __device__ __forceinline__ void sync() const {
-        if (half)
-            asm volatile("bar.sync 2, 64;" ::: "memory");
-        else
-            asm volatile("bar.sync 1, 64;" ::: "memory");
-    }
-    __device__ __forceinline__ bool any(bool p) const {
-        uint32_t r;
-        if (half)
-            asm volatile(
-                "{\n\t.reg .pred pin, pout;\n\t"
-                "setp.ne.u32 pin, %1, 0;\n\t"
-                "bar.red.or.pred pout, 2, 64, pin;\n\t"
-                "selp.u32 %0, 1, 0, pout;\n\t}"
-                : "=r"(r)
-                : "r"(static_cast<uint32_t>(p))
-                : "memory");
-        else
-            asm volatile(
-                "{\n\t.reg .pred pin, pout;\n\t"
-                "setp.ne.u32 pin, %1, 0;\n\t"
-                "bar.red.or.pred pout, 1, 64, pin;\n\t"
-                "selp.u32 %0, 1, 0, pout;\n\t}"
-                : "=r"(r)
-                : "r"(static_cast<uint32_t>(p))
-                : "memory");
-        return r != 0u;
-    }
-    __device__ __forceinline__ uint32_t exclusive_scan(uint32_t v, uint32_t* scratch, uint32_t& total) const {
-        const uint32_t lane = threadIdx.x & 31u, w = warp();
-        uint32_t x = v;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-            if (lane >= static_cast<uint32_t>(d)) x += y;
+private:
+    // last: the warp's total in its last lane; before: the prefix inside the warp
+    __device__ __forceinline__ uint32_t finish_scan(uint32_t last, uint32_t before, uint32_t* scratch,
+                                                    uint32_t& total) {
+        if (n == 32u) {
+            total = __shfl_sync(0xffffffffu, last, 31);
+            return before;
         }
-        if (lane == 31u) scratch[w] = x;
+        uint32_t* w = scratch + turn * (kSceneWideThreads / 32);
+        turn ^= 1u;
+        if ((threadIdx.x & 31u) == 31u) w[warp()] = last;
         sync();
-        const uint32_t t0 = scratch[0], t1 = scratch[1];
-        total = t0 + t1;
-        sync();  // the scratch words are free again for the next scan
-        return (w ? t0 : 0u) + x - v;
+        total = 0u;
+        for (uint32_t i = 0; i < warps(); ++i) {
+            if (i == warp()) before += total;
+            total += w[i];
+        }
+        return before;
     }
 };
 
@@ -220,32 +200,35 @@ struct HalfTeam {
 // always be finished, and each warp goes through its contacts in ascending
 // order, so the polls end. (A pass over all contacts between barriers took a
 // pass per level: 25 against 22 us of set-up on a 256-body stack.)
-template <class Team>
 __device__ uint32_t scene_levels(const Team& T, uint32_t m, const SceneContacts& SC, uint32_t* s_max) {
     for (uint32_t k = T.rank(); k < m; k += T.size()) SC.done(k) = 0u;
     if (T.leader()) *s_max = 0u;
     T.sync();
     uint32_t my_max = 0, spins = 0;
-    const volatile uint32_t* done = &SC.done(0);
+    volatile uint32_t* done = &SC.done(0);
+    const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t k0 = T.rank() & ~31u; k0 < m; k0 += T.size()) {
-        const uint32_t k = k0 + (threadIdx.x & 31u);
+        // a predecessor among the warp's 32 is read by a shuffle, an earlier one from its word
+        const uint32_t k = k0 + lane;
         const bool mine = k < m;
         const uint32_t pa = mine ? SC.pa(k) : kSceneNone, pb = mine ? SC.pb(k) : kSceneNone;
-        bool open = mine;
+        const bool in_a = pa != kSceneNone && pa >= k0, in_b = pb != kSceneNone && pb >= k0;
+        bool wait_a = pa != kSceneNone && !in_a, wait_b = pb != kSceneNone && !in_b, open = mine;
+        uint32_t level = 0, la = 0, lb = 0;
         while (__any_sync(0xffffffffu, open)) {
-            if (open) {
-                const uint32_t la = pa == kSceneNone ? 0u : done[pa];
-                const uint32_t lb = pb == kSceneNone ? 0u : done[pb];
-                if ((pa == kSceneNone || la != 0u) && (pb == kSceneNone || lb != 0u)) {
-                    const uint32_t l = max(la, lb) + 1u;
-                    const_cast<volatile uint32_t*>(done)[k] = l;
-                    my_max = max(my_max, l);
-                    open = false;
-                }
+            if (wait_a) wait_a = (la = done[pa]) == 0u;
+            if (wait_b) wait_b = (lb = done[pb]) == 0u;
+            const uint32_t sa = __shfl_sync(0xffffffffu, level, static_cast<int>(in_a ? pa - k0 : lane));
+            const uint32_t sb = __shfl_sync(0xffffffffu, level, static_cast<int>(in_b ? pb - k0 : lane));
+            if (open && !wait_a && !wait_b && (!in_a || sa != 0u) && (!in_b || sb != 0u)) {
+                level = max(in_a ? sa : la, in_b ? sb : lb) + 1u;
+                done[k] = level;
+                open = false;
             }
             if (++spins > kSpinLimit) break;
-            __syncwarp();
         }
+        my_max = max(my_max, level);
+        __syncwarp();
     }
     my_max = __reduce_max_sync(0xffffffffu, spins > kSpinLimit ? kSceneNone : my_max);
     if ((threadIdx.x & 31u) == 0u) atomicMax(s_max, my_max);
@@ -257,28 +240,31 @@ __device__ uint32_t scene_levels(const Team& T, uint32_t m, const SceneContacts&
 
 // Counting sort of the scene's contacts by group done(k) - base (a level or a
 // colour) into SC.ent; group g is SC.ent[SC.pa(g), SC.pa(g + 1)). The
-// predecessor rows are free once the groups are known.
-template <class Team>
-__device__ void scene_group(const Team& T, uint32_t m, uint32_t groups, uint32_t base, const SceneContacts& SC,
-                            uint32_t* s_scan, uint32_t* s_carry) {
+// predecessor rows are free once the groups are known. *s_passes receives the
+// groups' sixteens (see scene_sweep).
+__device__ void scene_group(Team& T, uint32_t m, uint32_t groups, uint32_t base, const SceneContacts& SC,
+                            uint32_t* s_scan, uint32_t* s_passes) {
     for (uint32_t g = T.rank(); g <= groups; g += T.size()) SC.pa(g) = 0u;
-    if (T.leader()) *s_carry = 0u;
+    if (T.leader()) *s_passes = 0u;
     T.sync();
     for (uint32_t k = T.rank(); k < m; k += T.size()) atomicAdd(&SC.pa(SC.done(k) - base), 1u);
     T.sync();
-    for (uint32_t g0 = 0; g0 <= groups; g0 += T.size()) {
+    uint32_t passes = 0;
+    for (uint32_t g0 = 0, carry = 0; g0 <= groups; g0 += T.size()) {
         const uint32_t g = g0 + T.rank();
         const uint32_t v = g <= groups ? SC.pa(g) : 0u;
+        passes += (v + 15u) >> 4;
         uint32_t tot;
         const uint32_t ex = T.exclusive_scan(v, s_scan, tot);
         if (g <= groups) {
-            SC.pa(g) = *s_carry + ex;
-            SC.pb(g) = *s_carry + ex;  // fill cursor
+            SC.pa(g) = carry + ex;
+            SC.pb(g) = carry + ex;  // fill cursor
         }
-        T.sync();
-        if (T.leader()) *s_carry += tot;
-        T.sync();
+        carry += tot;
     }
+    passes = __reduce_add_sync(0xffffffffu, passes);
+    if ((threadIdx.x & 31u) == 0u && passes) atomicAdd(s_passes, passes);
+    T.sync();
     for (uint32_t k = T.rank(); k < m; k += T.size()) SC.ent(atomicAdd(&SC.pb(SC.done(k) - base), 1u)) = k;
     T.sync();
 }
@@ -311,61 +297,97 @@ __device__ __forceinline__ void record_state(float* r, uint32_t stride, const Si
 // its renormalisation took 70 us with a contact per lane on a 256-body stack
 // alone on its SM, 44 us with a contact per lane pair; 41.6 and 27.9 us on the
 // 66-body push scenes. kRecord compiles the recording in; without it `rec` is
-// ignored.
-template <bool kRecord, class Team>
-__device__ void scene_sweep(const Team& T, uint32_t groups, const SceneBodies& SB, const SceneContacts& SC, float mu,
-                            float dt, int* s_flag, const SolveRecord* rec_in = nullptr, int iter = 0) {
+// ignored. kAhead, for kernels whose warps have their scheduler to themselves:
+// what does not depend on the group before (the next group's bounds, contact and
+// constant body rows) is loaded ahead of the barrier, and when almost every
+// group fits one warp (`passes`, the groups' sixteens, are hardly more than the
+// groups) the first warp sweeps alone. On full SMs the extra registers and
+// instructions cost more than they hide (455 against 440 us a frame on 4096
+// stacks; 76 against 80 us on two 256-body stacks).
+template <bool kRecord, bool kAhead>
+__device__ void scene_sweep(const Team& T, uint32_t groups, uint32_t passes, const SceneBodies& SB,
+                            const SceneContacts& SC, float mu, float dt, int* s_flag,
+                            const SolveRecord* rec_in = nullptr, int iter = 0) {
     const SolveRecord* const rec = kRecord ? rec_in : nullptr;
-    const bool is_b = T.rank() & 1u;
-    for (uint32_t g = 0; g < groups; ++g) {
-        const uint32_t end = SC.pa(g + 1);
-        for (uint32_t i0 = SC.pa(g) + ((T.rank() & ~31u) >> 1); i0 < end; i0 += T.size() >> 1) {  // warp-uniform
+    const bool is_b = T.rank() & 1u, alone = kAhead && T.size() > 32u && passes - groups <= groups / 16u;
+    const uint32_t first = alone ? 0u : (T.rank() & ~31u) >> 1, step = alone ? 16u : T.size() >> 1;
+    if (!alone || T.warp() == 0u) {
+        uint32_t k = 0, bi = 0;
+        Contact ct{};
+        SideBody S{};
+        float lc = 0.f;
+        // contact i0 + lane / 2 of a group that ends at `end`, and its body's constant rows
+        auto fetch = [&](uint32_t i0, uint32_t end) {
             const uint32_t i = i0 + ((T.rank() & 31u) >> 1);
-            const bool valid = i < end;
-            const uint32_t k = SC.ent(valid ? i : i0);
-            const Contact ct = SC.contact(k);
-            const uint32_t bi = is_b ? ct.b : ct.a;
-            float lc = SC.lam(k);
-            SideBody S = load_side(SB, bi);
-            int res;
-            if (rec) {
-                // The pre-solve state of the first sweep, the one the adjoint
-                // differentiates, marked as acted only if it did. A later sweep
-                // (after a deferral) must not overwrite it: it re-solves only the
-                // deferred contacts, and one of those that acts there is
-                // reported as a path the adjoint does not cover.
-                float* r = rec->rec + rec->base + k;
-                const float lc0 = lc;
-                if (iter == 0 && valid) record_state(r, rec->stride, S, is_b ? 13 : 0);
-                uint32_t fl = 0u;
-                res = solve_contact_side(valid, is_b, S, ct, mu, lc, dt, &fl);
-                if (valid && !is_b) {
-                    if (fl & kSfActive) {
-                        r[26ull * rec->stride] = lc0;
-                        r[35ull * rec->stride] = __uint_as_float(fl);
-                        if (iter > 0) atomicOr(rec->flag, 1u);  // acted after a renormalisation
-                    } else if (iter == 0) {
-                        r[35ull * rec->stride] = 0.f;
+            k = SC.ent(i < end ? i : i0);
+            ct = SC.contact(k);
+            lc = SC.lam(k);
+            bi = is_b ? ct.b : ct.a;
+            S.m = SB.im(bi);
+            S.ixx = SB.ixx(bi); S.iyy = SB.iyy(bi); S.izz = SB.izz(bi);
+            S.ixy = SB.ixy(bi); S.ixz = SB.ixz(bi); S.iyz = SB.iyz(bi);
+        };
+        uint32_t start = SC.pa(0), end = SC.pa(1);
+        if (kAhead && start + first < end) fetch(start + first, end);
+        for (uint32_t g = 0; g < groups; ++g) {
+            bool fetched = kAhead;
+            for (uint32_t i0 = start + first; i0 < end; i0 += step) {  // warp-uniform
+                if (!fetched) fetch(i0, end);
+                fetched = false;
+                const bool valid = i0 + ((T.rank() & 31u) >> 1) < end;
+                S.px = SB.px(bi); S.py = SB.py(bi); S.pz = SB.pz(bi);
+                S.qw = SB.qw(bi); S.qx = SB.qx(bi); S.qy = SB.qy(bi); S.qz = SB.qz(bi);
+                S.vx = SB.vx(bi); S.vy = SB.vy(bi); S.vz = SB.vz(bi);
+                S.wx = SB.wx(bi); S.wy = SB.wy(bi); S.wz = SB.wz(bi);
+                int res;
+                if (rec) {
+                    // The pre-solve state of the first sweep, the one the adjoint
+                    // differentiates, marked as acted only if it did. A later sweep
+                    // (after a deferral) must not overwrite it: it re-solves only the
+                    // deferred contacts, and one of those that acts there is
+                    // reported as a path the adjoint does not cover.
+                    float* r = rec->rec + rec->base + k;
+                    const float lc0 = lc;
+                    if (iter == 0 && valid) record_state(r, rec->stride, S, is_b ? 13 : 0);
+                    uint32_t fl = 0u;
+                    res = solve_contact_side<kAhead>(valid, is_b, S, ct, mu, lc, dt, &fl);
+                    if (valid && !is_b) {
+                        if (fl & kSfActive) {
+                            r[26ull * rec->stride] = lc0;
+                            r[35ull * rec->stride] = __uint_as_float(fl);
+                            if (iter > 0) atomicOr(rec->flag, 1u);  // acted after a renormalisation
+                        } else if (iter == 0) {
+                            r[35ull * rec->stride] = 0.f;
+                        }
                     }
+                } else {
+                    res = solve_contact_side<kAhead>(valid, is_b, S, ct, mu, lc, dt);
                 }
-            } else {
-                res = solve_contact_side(valid, is_b, S, ct, mu, lc, dt);
+                if (res == kSolveDone) {
+                    if (S.m != 0.f) store_side(SB, bi, S);
+                    if (!is_b) SC.lam(k) = lc;
+                } else if (res == kSolveDeferred) {
+                    *s_flag = 1;
+                }
             }
-            if (res == kSolveDone) {
-                if (S.m != 0.f) store_side(SB, bi, S);
-                if (!is_b) SC.lam(k) = lc;
-            } else if (res == kSolveDeferred) {
-                *s_flag = 1;
+            start = end;
+            if (g + 1u < groups) {
+                end = SC.pa(g + 2u);
+                if (kAhead && start + first < end) fetch(start + first, end);
             }
+            if (alone)
+                __syncwarp();
+            else
+                T.sync();
         }
-        T.sync();
     }
+    if (alone) T.sync();
 }
 
 // Block-shared scalars of one scene's solve.
 struct SceneShared {
-    uint32_t scan[kSceneThreads / 32];
-    uint32_t carry, rem, over, maxcol;
+    uint32_t scan[2 * (kSceneWideThreads / 32)];
+    uint32_t rem, over, maxcol, passes;
     int flag;
 };
 
@@ -386,7 +408,6 @@ __device__ __forceinline__ SceneSolverRows scene_solver_rows(float* fb, uint32_t
     return R;
 }
 
-template <class Team>
 __device__ __forceinline__ void scene_load_bodies(const Team& T, const GlobalBodies& B, uint32_t b0, uint32_t nb,
                                                   float* fb, uint32_t ldb) {
     const SceneBodies SB{fb, ldb};
@@ -402,7 +423,6 @@ __device__ __forceinline__ void scene_load_bodies(const Team& T, const GlobalBod
     }
 }
 
-template <class Team>
 __device__ __forceinline__ void scene_store_bodies(const Team& T, const GlobalBodies& B, uint32_t b0, uint32_t nb,
                                                    const SceneBodies& SB) {
     for (uint32_t i = T.rank(); i < nb; i += T.size()) {
@@ -414,37 +434,128 @@ __device__ __forceinline__ void scene_store_bodies(const Team& T, const GlobalBo
     }
 }
 
+// Jones–Plassmann colouring of a scene's contacts into SC.done: the rounds taken
+// in `rounds`, what is left uncoloured in sh.rem, sh.over when a body needs a 65th
+// colour, the largest colour in sh.maxcol.
+__device__ __forceinline__ void scene_color(const Team& T, uint32_t nb, uint32_t m, const SceneBodies& SB,
+                                      const SceneSolverRows& R, const SceneContacts& SC, SceneShared& sh,
+                                      uint32_t& rounds) {
+    // A contact's priority is hash(k) << 32 | k; the hash (murmur3's
+    // finaliser) is a bijection, so its 32 bits alone are distinct and in
+    // the same order, and shared memory has a native 32-bit maximum. A
+    // winner is the only one on its bodies, so it updates their masks
+    // without atomics. Each thread keeps its uncoloured contacts as bits
+    // (up to 64 of them, the rest by their colour word); priorities
+    // alternate between two rows, one cleared while the other is used.
+    // Set-up of a 512-body mixed scene alone: 80 us, 137 with 64-bit
+    // maxima over all contacts in every round.
+    // The bodies of a contact, 0xFFFF for a static one, wait in its list entry's
+    // word (free until the groups are made).
+    T.sync();  // the lists' last reads
+    for (uint32_t k = T.rank(); k < m; k += T.size()) {
+        const uint32_t ab = SC.ab(k);
+        SC.done(k) = kUncolored;
+        SC.ent(k) = ab | (SB.im(ab & 0xFFFFu) == 0.f ? 0xFFFFu : 0u) | (SB.im(ab >> 16) == 0.f ? 0xFFFF0000u : 0u);
+    }
+    for (uint32_t i = T.rank(); i < nb; i += T.size()) {
+        R.mask[i] = 0ull;
+        R.pri[i] = 0u;
+    }
+    if (T.leader()) {
+        sh.rem = m;
+        sh.over = 0u;
+        sh.maxcol = 0u;
+    }
+    const uint32_t mine = m > T.rank() ? (m - T.rank() + T.size() - 1u) / T.size() : 0u;
+    uint64_t open = mine >= 64u ? ~0ull : (1ull << mine) - 1ull;
+    // fn(k, bodies) for each of this thread's uncoloured contacts, four loads ahead
+    auto for_open = [&](auto&& fn) {
+        for (uint64_t o = open; o;) {
+            uint32_t j[4], ab[4];
+            int c = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                j[u] = o ? static_cast<uint32_t>(__ffsll(static_cast<long long>(o))) - 1u : 0u;
+                c += o ? 1 : 0;
+                o &= o - 1ull;
+                ab[u] = SC.ent(T.rank() + j[u] * T.size());
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (u < c && fn(T.rank() + j[u] * T.size(), ab[u])) open &= ~(1ull << j[u]);
+        }
+        for (uint32_t j = 64u; j < mine; ++j) {
+            const uint32_t k = T.rank() + j * T.size();
+            if (SC.done(k) == kUncolored) fn(k, SC.ent(k));
+        }
+    };
+    uint32_t my_max = 0u;
+    T.sync();
+    while (sh.rem > 0u && rounds < kMaxRounds) {
+        uint32_t* pri = R.pri + (rounds & 1u) * ((nb + 3u) & ~3u);
+        uint32_t* next = R.pri + (~rounds & 1u) * ((nb + 3u) & ~3u);
+        for_open([&](uint32_t k, uint32_t ab) {
+            const uint32_t a = ab & 0xFFFFu, b = ab >> 16, pk = hash_u32(k);
+            if (a != 0xFFFFu) atomicMax(&pri[a], pk);
+            if (b != 0xFFFFu) atomicMax(&pri[b], pk);
+            return false;
+        });
+        for (uint32_t i = T.rank(); i < nb; i += T.size()) next[i] = 0u;
+        T.sync();
+        uint32_t won = 0u;
+        for_open([&](uint32_t k, uint32_t ab) {
+            const uint32_t a = ab & 0xFFFFu, b = ab >> 16, pk = hash_u32(k);
+            const bool da = a != 0xFFFFu, db = b != 0xFFFFu;
+            if ((da && pri[a] != pk) || (db && pri[b] != pk)) return false;  // not a local maximum
+            const uint64_t used = (da ? R.mask[a] : 0ull) | (db ? R.mask[b] : 0ull);
+            if (~used == 0ull) {  // > 64 colours: the reference falls back to the serial order
+                sh.over = 1u;
+                return false;
+            }
+            const uint32_t col = static_cast<uint32_t>(__ffsll(static_cast<long long>(~used)) - 1);
+            SC.done(k) = col;
+            if (da) R.mask[a] |= 1ull << col;
+            if (db) R.mask[b] |= 1ull << col;
+            my_max = max(my_max, col);
+            ++won;
+            return true;
+        });
+        won = __reduce_add_sync(0xffffffffu, won);
+        if ((threadIdx.x & 31u) == 0u && won) atomicSub(&sh.rem, won);
+        T.sync();
+        ++rounds;
+    }
+    my_max = __reduce_max_sync(0xffffffffu, my_max);
+    if ((threadIdx.x & 31u) == 0u) atomicMax(&sh.maxcol, my_max);
+    T.sync();
+}
+
 // XpbdSolver::solve on one scene whose m >= 1 contacts sit in SC (rows ab,
 // lambda = 0, geometry; pb = none) with R.cnt[b] = the b-side contact count of
 // every dynamic body b. Leaves the bodies solved and renormalised in SB and
 // the colours (or UINT32_MAX) in SC.done. Returns false after raising an error.
-template <bool kRecord = false, class Team>
-__device__ bool scene_solve(const Team& T, uint32_t nb, uint32_t m, const SceneBodies& SB, const SceneSolverRows& R,
+template <bool kRecord = false, bool kAhead = false>
+__device__ bool scene_solve(Team& T, uint32_t nb, uint32_t m, const SceneBodies& SB, const SceneSolverRows& R,
                             const SceneContacts& SC, int mode, int n_iters, float mu, float dt, SceneShared& sh,
                             bool& colored_out, uint32_t& n_colors_out, uint32_t& rounds_out,
                             const SolveRecord* rec_in = nullptr, uint32_t* groups_out = nullptr,
                             uint64_t* sweep_start = nullptr) {
     const SolveRecord* const rec = kRecord ? rec_in : nullptr;
     // ── predecessors in contact order: b-side lists (scan, fill, sort) ──
-    if (T.leader()) {
-        sh.carry = 0u;
-        sh.flag = 0;
-    }
-    T.sync();
+    if (T.leader()) sh.flag = 0;
+    uint32_t entries = 0;
     for (uint32_t base = 0; base < nb; base += T.size()) {
         const uint32_t i = base + T.rank();
         const uint32_t v = i < nb ? R.cnt[i] : 0u;
         uint32_t tot;
         const uint32_t ex = T.exclusive_scan(v, sh.scan, tot);
         if (i < nb) {
-            R.off[i] = sh.carry + ex;
+            R.off[i] = entries + ex;
             R.cnt[i] = 0u;
         }
-        T.sync();
-        if (T.leader()) sh.carry += tot;
-        T.sync();
+        entries += tot;
     }
-    if (T.leader()) R.off[nb] = sh.carry;
+    if (T.leader()) R.off[nb] = entries;
     T.sync();
     for (uint32_t k = T.rank(); k < m; k += T.size()) {
         const uint32_t b = SC.ab(k) >> 16;
@@ -477,77 +588,7 @@ __device__ bool scene_solve(const Team& T, uint32_t nb, uint32_t m, const SceneB
                    ((mode == DYPH_SOLVER_REFERENCE || mode == DYPH_SOLVER_REFERENCE_ROUNDS) && m > kSerialThreshold);
     uint32_t n_colors = 0, rounds = 0;
     if (colored) {
-        // A contact's priority is hash(k) << 32 | k; the hash (murmur3's
-        // finaliser) is a bijection, so its 32 bits alone are distinct and in
-        // the same order, and shared memory has a native 32-bit maximum. A
-        // winner is the only one on its bodies, so it updates their masks
-        // without atomics. Each thread keeps its uncoloured contacts as bits
-        // (up to 64 of them, the rest by their colour word); priorities
-        // alternate between two rows, one cleared while the other is used.
-        // Set-up of a 512-body mixed scene alone: 80 us, 137 with 64-bit
-        // maxima over all contacts in every round.
-        for (uint32_t k = T.rank(); k < m; k += T.size()) SC.done(k) = kUncolored;
-        for (uint32_t i = T.rank(); i < nb; i += T.size()) {
-            R.mask[i] = 0ull;
-            R.pri[i] = 0u;
-        }
-        if (T.leader()) {
-            sh.rem = m;
-            sh.over = 0u;
-            sh.maxcol = 0u;
-        }
-        const uint32_t mine = m > T.rank() ? (m - T.rank() + T.size() - 1u) / T.size() : 0u;
-        uint64_t open = mine >= 64u ? ~0ull : (1ull << mine) - 1ull;
-        // fn(k) for each of this thread's uncoloured contacts
-        auto for_open = [&](auto&& fn) {
-            for (uint64_t o = open; o; o &= o - 1ull) {
-                const uint32_t j = static_cast<uint32_t>(__ffsll(static_cast<long long>(o))) - 1u;
-                if (fn(T.rank() + j * T.size())) open &= ~(1ull << j);
-            }
-            for (uint32_t j = 64u; j < mine; ++j) {
-                const uint32_t k = T.rank() + j * T.size();
-                if (SC.done(k) == kUncolored) fn(k);
-            }
-        };
-        uint32_t my_max = 0u;
-        T.sync();
-        while (sh.rem > 0u && rounds < kMaxRounds) {
-            uint32_t* pri = R.pri + (rounds & 1u) * ((nb + 3u) & ~3u);
-            uint32_t* next = R.pri + (~rounds & 1u) * ((nb + 3u) & ~3u);
-            for_open([&](uint32_t k) {
-                const uint32_t a = SC.ab(k) & 0xFFFFu, b = SC.ab(k) >> 16, pk = hash_u32(k);
-                if (SB.im(a) != 0.f) atomicMax(&pri[a], pk);
-                if (SB.im(b) != 0.f) atomicMax(&pri[b], pk);
-                return false;
-            });
-            for (uint32_t i = T.rank(); i < nb; i += T.size()) next[i] = 0u;
-            T.sync();
-            uint32_t won = 0u;
-            for_open([&](uint32_t k) {
-                const uint32_t a = SC.ab(k) & 0xFFFFu, b = SC.ab(k) >> 16, pk = hash_u32(k);
-                const bool da = SB.im(a) != 0.f, db = SB.im(b) != 0.f;
-                if ((da && pri[a] != pk) || (db && pri[b] != pk)) return false;  // not a local maximum
-                const uint64_t used = (da ? R.mask[a] : 0ull) | (db ? R.mask[b] : 0ull);
-                if (~used == 0ull) {  // > 64 colours: the reference falls back to the serial order
-                    sh.over = 1u;
-                    return false;
-                }
-                const uint32_t col = static_cast<uint32_t>(__ffsll(static_cast<long long>(~used)) - 1);
-                SC.done(k) = col;
-                if (da) R.mask[a] |= 1ull << col;
-                if (db) R.mask[b] |= 1ull << col;
-                my_max = max(my_max, col);
-                ++won;
-                return true;
-            });
-            won = __reduce_add_sync(0xffffffffu, won);
-            if ((threadIdx.x & 31u) == 0u && won) atomicSub(&sh.rem, won);
-            T.sync();
-            ++rounds;
-        }
-        my_max = __reduce_max_sync(0xffffffffu, my_max);
-        if ((threadIdx.x & 31u) == 0u) atomicMax(&sh.maxcol, my_max);
-        T.sync();
+        scene_color(T, nb, m, SB, R, SC, sh, rounds);
         colored = sh.rem == 0u && sh.over == 0u;
         n_colors = sh.maxcol + 1u;
         T.sync();
@@ -562,7 +603,7 @@ __device__ bool scene_solve(const Team& T, uint32_t nb, uint32_t m, const SceneB
             return false;
         }
     }
-    scene_group(T, m, groups, base, SC, sh.scan, &sh.carry);
+    scene_group(T, m, groups, base, SC, sh.scan, &sh.passes);
     if (sweep_start && T.leader()) {
         uint64_t t;
         asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -573,7 +614,7 @@ __device__ bool scene_solve(const Team& T, uint32_t nb, uint32_t m, const SceneB
     if (groups_out) *groups_out = groups;
     for (int iter = 0; iter < n_iters; ++iter) {
         if (iter == 0 || deferred) {
-            scene_sweep<kRecord>(T, groups, SB, SC, mu, dt, &sh.flag, rec, iter);
+            scene_sweep<kRecord, kAhead>(T, groups, sh.passes, SB, SC, mu, dt, &sh.flag, rec, iter);
             deferred = sh.flag != 0;
         }
         if (rec && iter == 0)
@@ -604,7 +645,6 @@ __device__ bool scene_solve(const Team& T, uint32_t nb, uint32_t m, const SceneB
     return true;
 }
 
-template <class Team>
 __device__ __forceinline__ void scene_stats(const Team& T, uint32_t* meta, bool colored, uint32_t n_colors,
                                             uint32_t rounds) {
     if (T.leader()) {
@@ -625,7 +665,7 @@ __global__ void __launch_bounds__(kSceneThreads, 4) scene_solve_kernel(dyph_cont
     extern __shared__ __align__(16) unsigned char scene_smem[];
     __shared__ SceneShared sh;
     const GlobalBodies B{gb};
-    const BlockTeam T;
+    Team T{kSceneThreads, 0u};
     for (uint32_t t = blockIdx.x; t < S.n_scenes; t += gridDim.x) {
         const uint32_t s = S.order[t];
         const uint32_t b0 = S.body_offset[s], nb = S.body_offset[s + 1] - b0;

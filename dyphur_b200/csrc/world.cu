@@ -1,11 +1,12 @@
-// The whole frame step behind one handle, replayed as a CUDA graph.
+// The whole frame step behind one handle.
 //
 // One frame is the reference's loop body (examples/stress_test_blocks/
 // main.cpp:264-279): integrate, build_and_query, sort_pairs (already sorted),
 // Narrowphase::run, XpbdSolver::solve. Every count stays on the device, so a
-// frame has no host round trip; the first step captures one frame into a CUDA
-// graph and every later frame replays it. A one-thread kernel at the end of
-// the frame folds the pair / contact counts into peak and overflow words.
+// frame has no host round trip. A single scene's first step captures one frame
+// into a CUDA graph and every later frame replays it; a batch whose scenes fit
+// a block's shared memory runs on fused kernels. A small kernel at the end folds
+// the pair / contact counts into peak and overflow words.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,7 +37,9 @@ struct dyph_world {
     float* traj_host = nullptr;
     uint32_t traj_every = 0, traj_max = 0;
     uint64_t traj_frame = 0;              // frames stepped by dyph_world_step since the last set-up
-    float* traj_stage[2] = {nullptr, nullptr};
+    float* traj_stage[2] = {nullptr, nullptr};  // [traj_slots][7 n] records each
+    uint32_t traj_slots = 0;
+    uint64_t traj_chunk = 0;              // staging buffers filled by fused steps since the last set-up
     cudaStream_t traj_stream = nullptr;
     cudaEvent_t traj_packed[2] = {nullptr, nullptr};
     cudaEvent_t traj_copied[2] = {nullptr, nullptr};
@@ -51,6 +54,7 @@ struct dyph_world {
     uint32_t* f_contact_raw = nullptr;
     uint32_t* f_color_raw = nullptr;
     uint32_t* f_counts = nullptr;        // [4 n_scenes]
+    uint32_t* f_run = nullptr;           // [kAccWords] + [4 kMaxRunFrames] a launch's statistics (zero between launches)
     uint32_t* f_words = nullptr;
     uint32_t* f_pos = nullptr;           // [2 n_scenes] gather positions
     uint32_t* f_items = nullptr;         // [4 f_n_items] work items of the fused kernel
@@ -65,7 +69,8 @@ struct dyph_world {
     std::vector<float*> a_qs;        // [4][n]
     std::vector<uint32_t*> a_words;  // [kSceneWords][f_words_stride]
     std::vector<uint32_t*> a_mg;     // [2 n_scenes]
-    float* a_g[2] = {nullptr, nullptr};  // [13][n] adjoint ping-pong
+    AdjSet* a_sets = nullptr;        // [a_rec.size()] the record sets, for the kernels
+    float* a_g = nullptr;            // [13][n] the state's adjoint
     float* a_seg[2] = {nullptr, nullptr};  // [a_seg_frames][13][n] states of frames 1.. of a segment (double buffer)
     uint32_t a_seg_frames = 0;
     uint32_t* a_pairs = nullptr;         // pair slots of spilled scenes, the recording's own
@@ -78,6 +83,8 @@ struct dyph_world {
     std::vector<uint32_t> h_body_offset;  // host copy of the scenes' body ranges
     uint32_t f_smem_cap = 0;              // shared memory cap per block (0 = what the largest scene needs)
     uint32_t f_teams = 2;                 // 0 blocks only, 1 + small scenes one per warp, 2 + mid-size two warps
+    uint32_t f_threads = kSceneThreads;   // threads of a block (fused_threads)
+    bool f_resident = false;              // all blocks of the batch fit the device at once
     uint32_t f_variant = 0;               // register budget: 4 (0), 5 (1) or 6 (2) blocks per SM
     uint32_t f_warp_scenes = 0, f_half_scenes = 0, f_block_scenes = 0;
     // Work items of the adjoint's reverse kernel, laid out on their own: its
@@ -97,15 +104,22 @@ namespace {
 
 constexpr uint32_t kHistory = 4096;
 
-// Frame f's recomputation with recording for the adjoint (record_scene), on
-// the fused kernel's work items.
-__global__ void __launch_bounds__(kSceneThreads, 4) scene_frame_record_kernel(SceneBufs S, FrameBufs F,
-                                                                              FrameParams P_, AdjRun A, AdjKeep K,
-                                                                              const uint32_t* __restrict__ items,
-                                                                              uint32_t n_items) {
+// The recomputation with recording of a segment's frames (record_scene), on the
+// fused kernel's work items.
+template <int kMinBlocks, int kThreads>
+__global__ void __launch_bounds__(kThreads, kMinBlocks) scene_frame_record_kernel(SceneBufs S, FrameBufs F,
+                                                                                  FrameParams P_, AdjSegment D,
+                                                                                  const uint32_t* __restrict__ items,
+                                                                                  uint32_t n_items) {
     for_each_item(items, n_items, S.smem_bytes,
-                  [&](const auto& T, uint32_t s, unsigned char* smem, uint32_t bytes, SceneShared& sh) {
-                      record_scene(T, s, smem, bytes, sh, S, F, P_, A, K);
+                  [&](Team& T, uint32_t s, unsigned char* smem, uint32_t bytes, SceneShared& sh) {
+                      for (uint32_t f = 0; f < P_.n_frames; ++f) {
+                          const AdjSet& k = D.sets[f];
+                          FrameBufs Ff = F;
+                          Ff.words = k.words;
+                          record_scene<kThreads == kSceneWideThreads>(T, s, f, smem, bytes, sh, S, Ff, P_, segment_run(D, f, P_.n_frames),
+                                       AdjKeep{k.words, k.mg});
+                      }
                   });
 }
 constexpr size_t kStatsWords = 8 + 2 * kHistory;
@@ -123,6 +137,59 @@ __global__ void frame_stats_kernel(const uint32_t* __restrict__ bp_counts, const
     stats[9 + 2 * (f % kHistory)] = c;
     if (p > max_pairs) atomicCAS(&stats[4], 0u, static_cast<uint32_t>(DYPH_ERR_PAIR_OVERFLOW));
     if (c > max_contacts) atomicCAS(&stats[4], 0u, static_cast<uint32_t>(DYPH_ERR_CONTACT_OVERFLOW));
+}
+
+// The statistics of a fused launch of n_frames <= kMaxRunFrames frames (one
+// block): the world's history, peaks and status as frame_stats_kernel keeps
+// them frame by frame, the stored-count words and the solver's meta words of
+// the last frame. Clears the launch's words for the next one.
+__global__ void __launch_bounds__(kMaxRunFrames) frame_run_stats_kernel(uint32_t* __restrict__ run, uint32_t n_frames,
+                                                                        uint32_t* __restrict__ bp_counts,
+                                                                        uint32_t* __restrict__ np_counts,
+                                                                        uint32_t* __restrict__ meta,
+                                                                        uint32_t max_pairs, uint32_t max_contacts,
+                                                                        uint32_t* __restrict__ stats) {
+    const uint32_t f = threadIdx.x;
+    uint32_t* counts = run + kAccWords;
+    const uint32_t total = stats[5];
+    uint32_t p = 0, c = 0;
+    if (f < n_frames) {
+        p = counts[n_frames + f];
+        c = counts[3u * n_frames + f];
+        stats[8 + 2 * ((total + f) % kHistory)] = p;
+        stats[9 + 2 * ((total + f) % kHistory)] = c;
+        atomicMax(&stats[2], p);
+        atomicMax(&stats[3], c);
+        if (f + 1u == n_frames) {
+            stats[0] = p;
+            stats[1] = c;
+            bp_counts[0] = counts[f];
+            bp_counts[1] = p;
+            np_counts[0] = counts[2u * n_frames + f];
+            np_counts[1] = c;
+        }
+    }
+    // the earliest frame past a capacity sets the status, its pairs before its contacts
+    __shared__ uint32_t s_first;
+    if (f == 0) s_first = kMaxRunFrames;
+    __syncthreads();
+    if (f < n_frames && (p > max_pairs || c > max_contacts)) atomicMin(&s_first, f);
+    __syncthreads();
+    if (f == s_first)
+        atomicCAS(&stats[4], 0u,
+                  static_cast<uint32_t>(p > max_pairs ? DYPH_ERR_PAIR_OVERFLOW : DYPH_ERR_CONTACT_OVERFLOW));
+    if (f < 16u) {
+        uint32_t v = 0u;
+        if (f == kMetaMaxColor && run[kAccMaxColor]) v = run[kAccMaxColor] - 1u;
+        if (f == kMetaRounds) v = run[kAccRounds];
+        if (f == kMetaSceneColored) v = run[kAccColored];
+        if (f == kMetaDecision) v = run[kAccSolved] ? kDecisionScenes : 0u;
+        meta[f] = v;
+    }
+    __syncthreads();
+    if (f == 0) stats[5] = total + n_frames;
+    if (f < static_cast<uint32_t>(kAccWords)) run[f] = 0u;
+    for (uint32_t i = f; i < 4u * n_frames; i += kMaxRunFrames) counts[i] = 0u;
 }
 
 // Pose rows of every body, interleaved per body as the .trajectory row
@@ -154,10 +221,11 @@ dyph_status enqueue_trajectory_record(dyph_world* w, cudaStream_t s, uint64_t re
     return DYPH_OK;
 }
 
-// Order every queued trajectory copy before the work that follows on s.
-dyph_status join_trajectory(dyph_world* w, cudaStream_t s, uint64_t last_rec) {
+// Order every queued trajectory copy, the last one out of staging buffer
+// `last`, before the work that follows on s.
+dyph_status join_trajectory(dyph_world* w, cudaStream_t s, uint64_t last) {
     if (!w->traj_pending) return DYPH_OK;
-    DYPH_CUDA_TRY(cudaStreamWaitEvent(s, w->traj_copied[last_rec & 1u], 0));
+    DYPH_CUDA_TRY(cudaStreamWaitEvent(s, w->traj_copied[last & 1u], 0));
     w->traj_pending = false;
     return DYPH_OK;
 }
@@ -173,6 +241,116 @@ dyph_status probe_record(void* ev, cudaStream_t s) {
     return DYPH_OK;
 }
 
+// What a fused launch does besides stepping: its frames' numbers, the
+// trajectory rows and the checkpoints it writes (see FrameParams).
+struct FusedRun {
+    uint32_t n_frames;  // <= kMaxRunFrames
+    bool keep = true;   // the last launch of a call
+    float* traj = nullptr;
+    uint32_t traj_first = 0, traj_count = 0;
+    float* ckpt = nullptr;
+    uint32_t ckpt_first = 0, ckpt_every = 1;
+};
+
+// The fused kernel's form that the world's settings ask for.
+struct FusedForm {
+    const void* kernel;
+    uint32_t threads;
+};
+FusedForm fused_form(const dyph_world* w) {
+    if (w->f_threads == static_cast<uint32_t>(kSceneWideThreads))
+        return {reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>), kSceneWideThreads};
+    switch (w->f_variant) {
+        case 1: return {reinterpret_cast<const void*>(scene_frame_kernel<5, kSceneThreads>), kSceneThreads};
+        case 2: return {reinterpret_cast<const void*>(scene_frame_kernel<6, kSceneThreads>), kSceneThreads};
+        default: return {reinterpret_cast<const void*>(scene_frame_kernel<4, kSceneThreads>), kSceneThreads};
+    }
+}
+
+// n_frames frames of every scene in one launch, and their statistics.
+dyph_status launch_run(dyph_world* w, const FusedRun& r, cudaStream_t s) {
+    const dyph_world_desc& d = w->desc;
+    const dyph_integrator_params& ip = d.integrator;
+    const float sub_dt = ip.dt / static_cast<float>(ip.n_substeps);
+    SceneBufs S{w->bp->body_offset, w->bp->bvh.scene_of, w->sv->scene_order, nullptr, nullptr, 0, w->bp->n_scenes,
+                w->frame_smem};
+    FrameBufs F{w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw,
+                w->f_counts, w->f_words, w->f_words_stride, w->f_contact_slots};
+    const FusedForm form = fused_form(w);
+    FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
+                  w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(w->sv->mode),
+                  w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->stats + 4, w->f_phase, r.n_frames,
+                  r.keep ? 1u : 0u, r.traj, r.traj_first, std::max(w->traj_every, 1u), r.traj_count, r.ckpt,
+                  r.ckpt_first, r.ckpt_every};
+    void* args[] = {&S, &F, &P, &w->f_items, &w->f_n_items};
+    DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(w->f_n_items), dim3(form.threads), args, w->frame_smem, s));
+    frame_run_stats_kernel<<<1, kMaxRunFrames, 0, s>>>(w->f_run, r.n_frames, w->bp->counts, w->np->counts, w->sv->meta,
+                                                      w->bp->max_pairs, w->np->max_contacts, w->stats);
+    DYPH_CUDA_TRY(cudaGetLastError());
+    return DYPH_OK;
+}
+
+// Frames [frame0, frame0 + n_frames) of a fused batch, frame numbers as the
+// trajectory counts them, in as few launches as the per-frame words and the
+// trajectory's staging buffers allow when all of the batch's blocks are
+// resident at once (no scene waits for the slowest of a frame: 67 against 79 us
+// a frame on 256 push scenes, 51 against 60 on 64 stacks). With more blocks than
+// that a frame is a launch: the queue's order, longest first, then balances
+// every frame (421 us against 480 on 4096 stacks). Records go to one of the two staging
+// buffers, traj_slots of them per launch, and from there to the host on the
+// side stream while the next launch runs; chunk counts the buffers filled,
+// live says whether a buffer's last copy has to be waited for (a capture may
+// only wait for events of its own). ckpt receives the state before every
+// ckpt_every-th frame of this call.
+dyph_status enqueue_run(dyph_world* w, cudaStream_t s, uint64_t frame0, uint32_t n_frames, uint64_t& chunk,
+                        bool live[2], float* ckpt = nullptr, uint32_t ckpt_every = 1) {
+    const size_t n = w->desc.bodies.n;
+    for (uint32_t done = 0; done < n_frames;) {
+        FusedRun r{std::min(n_frames - done, w->f_resident ? kMaxRunFrames : 1u)};
+        uint64_t rec0 = 0;
+        if (w->traj_host) {
+            const uint64_t every = w->traj_every, f = frame0 + done;
+            rec0 = (f + every - 1) / every;  // the first record at or after frame f
+            if (rec0 < w->traj_max) {
+                const uint64_t most = std::min<uint64_t>(w->traj_slots, w->traj_max - rec0);
+                // the launch ends with the record that fills the buffer
+                r.n_frames = static_cast<uint32_t>(
+                    std::min<uint64_t>(r.n_frames, rec0 * every - f + (most - 1) * every + 1));
+                const uint64_t past = (f + r.n_frames - 1) / every + 1;  // one past the last record
+                if (past > rec0) {
+                    r.traj = w->traj_stage[chunk & 1u];
+                    r.traj_first = static_cast<uint32_t>(rec0 * every - f);
+                    r.traj_count = static_cast<uint32_t>(past - rec0);
+                }
+            }
+        }
+        if (ckpt) {
+            const uint32_t c = (done + ckpt_every - 1) / ckpt_every;
+            r.ckpt = ckpt + static_cast<size_t>(c) * 13 * n;
+            r.ckpt_first = c * ckpt_every - done;
+            r.ckpt_every = ckpt_every;
+        }
+        r.keep = done + r.n_frames == n_frames;
+        const int k = static_cast<int>(chunk & 1u);
+        if (r.traj && live[k]) DYPH_CUDA_TRY(cudaStreamWaitEvent(s, w->traj_copied[k], 0));
+        const dyph_status st = launch_run(w, r, s);
+        if (st != DYPH_OK) return st;
+        if (r.traj) {
+            DYPH_CUDA_TRY(cudaEventRecord(w->traj_packed[k], s));
+            DYPH_CUDA_TRY(cudaStreamWaitEvent(w->traj_stream, w->traj_packed[k], 0));
+            DYPH_CUDA_TRY(cudaMemcpyAsync(w->traj_host + rec0 * 7 * n, w->traj_stage[k],
+                                          r.traj_count * 7 * n * sizeof(float), cudaMemcpyDeviceToHost,
+                                          w->traj_stream));
+            DYPH_CUDA_TRY(cudaEventRecord(w->traj_copied[k], w->traj_stream));
+            w->traj_pending = true;
+            live[k] = true;
+            ++chunk;
+        }
+        done += r.n_frames;
+    }
+    return DYPH_OK;
+}
+
 // One frame; when probe_stage matches a stage (0 integrate, 1 broadphase,
 // 2 narrowphase, 3 solver) the events are recorded around it; probe_stage 4
 // records them around the solver's dataflow kernel alone.
@@ -181,39 +359,9 @@ dyph_status enqueue_frame(dyph_world* w, cudaStream_t s, int probe_stage = -1, v
     const dyph_world_desc& d = w->desc;
     dyph_status st;
     if (w->fused) {
-        // One launch per frame: every scene's integrate, pairs, narrowphase and solve.
-        DYPH_CUDA_TRY(cudaMemsetAsync(w->bp->counts, 0, 4 * sizeof(uint32_t), s));
-        DYPH_CUDA_TRY(cudaMemsetAsync(w->np->counts, 0, 4 * sizeof(uint32_t), s));
-        DYPH_CUDA_TRY(cudaMemsetAsync(w->sv->meta, 0, 16 * sizeof(uint32_t), s));
         if (probe_stage >= 0 && (st = probe_record(ev0, s)) != DYPH_OK) return st;
-        const dyph_integrator_params& ip = d.integrator;
-        const float sub_dt = ip.dt / static_cast<float>(ip.n_substeps);
-        SceneBufs S{w->bp->body_offset, w->bp->bvh.scene_of, w->sv->scene_order, nullptr, nullptr, 0,
-                    w->bp->n_scenes, w->frame_smem};
-        FrameBufs F{w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw,
-                    w->f_counts, w->f_words, w->f_words_stride, w->f_contact_slots};
-        FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
-                      w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(w->sv->mode), w->sv->n_iters,
-                      w->sv->meta, w->bp->counts, w->np->counts, w->stats + 4, w->f_phase};
-        switch (w->f_variant) {
-            case 1:
-                scene_frame_kernel<5><<<w->f_n_items, kSceneThreads, w->frame_smem, s>>>(S, F, P, w->f_items,
-                                                                                       w->f_n_items);
-                break;
-            case 2:
-                scene_frame_kernel<6><<<w->f_n_items, kSceneThreads, w->frame_smem, s>>>(S, F, P, w->f_items,
-                                                                                       w->f_n_items);
-                break;
-            default:
-                scene_frame_kernel<4><<<w->f_n_items, kSceneThreads, w->frame_smem, s>>>(S, F, P, w->f_items,
-                                                                                       w->f_n_items);
-        }
-        DYPH_CUDA_TRY(cudaGetLastError());
-        if (probe_stage >= 0 && (st = probe_record(ev1, s)) != DYPH_OK) return st;
-        frame_stats_kernel<<<1, 1, 0, s>>>(w->bp->counts, w->np->counts, w->bp->max_pairs, w->np->max_contacts,
-                                           w->stats);
-        DYPH_CUDA_TRY(cudaGetLastError());
-        return DYPH_OK;
+        if ((st = launch_run(w, FusedRun{1u}, s)) != DYPH_OK) return st;
+        return probe_stage >= 0 ? probe_record(ev1, s) : DYPH_OK;
     }
     w->sv->probe_flow[0] = probe_stage == 4 ? ev0 : nullptr;
     w->sv->probe_flow[1] = probe_stage == 4 ? ev1 : nullptr;
@@ -259,8 +407,8 @@ extern "C" void dyph_world_destroy(dyph_world* w) {
         if (w->traj_copied[k]) cudaEventDestroy(w->traj_copied[k]);
     }
     if (w->traj_stream) cudaStreamDestroy(w->traj_stream);
-    void* fb[] = {w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw, w->f_counts,
-                  w->f_words, w->f_pos, w->f_items, w->r_items, w->f_phase, w->a_g[0], w->a_g[1], w->a_seg[0],
+    void* fb[] = {w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw, w->f_counts, w->f_run,
+                  w->f_words, w->f_pos, w->f_items, w->r_items, w->f_phase, w->a_g, w->a_sets, w->a_seg[0],
                   w->a_seg[1], w->a_flag, w->a_pairs};
     for (void* p : fb)
         if (p) cudaFree(p);
@@ -307,46 +455,60 @@ extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_strea
     return DYPH_OK;
 }
 
-extern "C" dyph_status dyph_world_step(dyph_world* w, int32_t n_frames, dyph_stream s) {
-    if (!w || n_frames < 0) return DYPH_ERR_INVALID;
-    if (n_frames == 0) return DYPH_OK;
+namespace {
+// dyph_world_step; a fused batch also writes checkpoints (dyph_world_rollout).
+dyph_status world_step(dyph_world* w, int32_t n_frames, dyph_stream s, float* ckpt = nullptr, uint32_t ckpt_every = 1) {
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
     DYPH_CUDA_TRY(cudaEventRecord(w->ev_in, cs));
     DYPH_CUDA_TRY(cudaStreamWaitEvent(w->stream, w->ev_in, 0));
-    if (!w->graph) {
-        cudaGraph_t g = nullptr;
-        DYPH_CUDA_TRY(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
-        dyph_status st = enqueue_frame(w, w->stream);
-        cudaError_t ce = cudaStreamEndCapture(w->stream, &g);
-        if (st != DYPH_OK) {
-            if (g) cudaGraphDestroy(g);
-            return st;
+    uint64_t last = 0;
+    if (w->fused) {
+        const dyph_status st = enqueue_run(w, w->stream, w->traj_frame, static_cast<uint32_t>(n_frames), w->traj_chunk,
+                                           w->traj_live, ckpt, ckpt_every);
+        if (st != DYPH_OK) return st;
+        w->traj_frame += static_cast<uint64_t>(n_frames);
+        last = w->traj_chunk - 1;
+    } else {
+        if (!w->graph) {
+            cudaGraph_t g = nullptr;
+            DYPH_CUDA_TRY(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
+            dyph_status st = enqueue_frame(w, w->stream);
+            cudaError_t ce = cudaStreamEndCapture(w->stream, &g);
+            if (st != DYPH_OK) {
+                if (g) cudaGraphDestroy(g);
+                return st;
+            }
+            if (ce != cudaSuccess) return DYPH_ERR_CUDA;
+            ce = cudaGraphInstantiate(&w->graph, g, 0);
+            cudaGraphDestroy(g);
+            if (ce != cudaSuccess) {
+                w->graph = nullptr;
+                return DYPH_ERR_CUDA;
+            }
         }
-        if (ce != cudaSuccess) return DYPH_ERR_CUDA;
-        ce = cudaGraphInstantiate(&w->graph, g, 0);
-        cudaGraphDestroy(g);
-        if (ce != cudaSuccess) {
-            w->graph = nullptr;
-            return DYPH_ERR_CUDA;
+        for (int32_t f = 0; f < n_frames; ++f) {
+            DYPH_CUDA_TRY(cudaGraphLaunch(w->graph, w->stream));
+            if (trajectory_frame(w, w->traj_frame)) {
+                last = w->traj_frame / w->traj_every;
+                const int k = static_cast<int>(last & 1u);
+                dyph_status st = enqueue_trajectory_record(w, w->stream, last, w->traj_live[k]);
+                if (st != DYPH_OK) return st;
+                w->traj_live[k] = true;
+            }
+            ++w->traj_frame;
         }
     }
-    uint64_t last_rec = 0;
-    for (int32_t f = 0; f < n_frames; ++f) {
-        DYPH_CUDA_TRY(cudaGraphLaunch(w->graph, w->stream));
-        if (trajectory_frame(w, w->traj_frame)) {
-            last_rec = w->traj_frame / w->traj_every;
-            const int k = static_cast<int>(last_rec & 1u);
-            dyph_status st = enqueue_trajectory_record(w, w->stream, last_rec, w->traj_live[k]);
-            if (st != DYPH_OK) return st;
-            w->traj_live[k] = true;
-        }
-        ++w->traj_frame;
-    }
-    dyph_status jst = join_trajectory(w, w->stream, last_rec);
+    dyph_status jst = join_trajectory(w, w->stream, last);
     if (jst != DYPH_OK) return jst;
     DYPH_CUDA_TRY(cudaEventRecord(w->ev_out, w->stream));
     DYPH_CUDA_TRY(cudaStreamWaitEvent(cs, w->ev_out, 0));
     return DYPH_OK;
+}
+}  // namespace
+
+extern "C" dyph_status dyph_world_step(dyph_world* w, int32_t n_frames, dyph_stream s) {
+    if (!w || n_frames < 0) return DYPH_ERR_INVALID;
+    return n_frames == 0 ? DYPH_OK : world_step(w, n_frames, s);
 }
 
 extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frames, int32_t probe_stage,
@@ -360,16 +522,24 @@ extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frame
     cudaGraph_t g = nullptr;
     DYPH_CUDA_TRY(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
     dyph_status st = DYPH_OK;
-    uint64_t last_rec = 0;
-    for (int32_t f = 0; f < n_frames && st == DYPH_OK; ++f) {
-        st = enqueue_frame(w, w->stream, probe_stage, probe_stage >= 0 ? ev_start[f] : nullptr,
-                           probe_stage >= 0 ? ev_end[f] : nullptr);
-        if (st == DYPH_OK && trajectory_frame(w, static_cast<uint64_t>(f))) {
-            last_rec = static_cast<uint64_t>(f) / w->traj_every;
-            st = enqueue_trajectory_record(w, w->stream, last_rec, last_rec >= 2);
+    uint64_t last = 0;
+    if (w->fused && probe_stage < 0) {
+        uint64_t chunk = 0;
+        bool live[2] = {false, false};
+        st = enqueue_run(w, w->stream, 0, static_cast<uint32_t>(n_frames), chunk, live);
+        last = chunk - 1;
+    } else {
+        for (int32_t f = 0; f < n_frames && st == DYPH_OK; ++f) {
+            // a probed fused frame is a launch of its own between the events
+            st = enqueue_frame(w, w->stream, probe_stage, probe_stage >= 0 ? ev_start[f] : nullptr,
+                               probe_stage >= 0 ? ev_end[f] : nullptr);
+            if (st == DYPH_OK && trajectory_frame(w, static_cast<uint64_t>(f))) {
+                last = static_cast<uint64_t>(f) / w->traj_every;
+                st = enqueue_trajectory_record(w, w->stream, last, last >= 2);
+            }
         }
     }
-    if (st == DYPH_OK) st = join_trajectory(w, w->stream, last_rec);
+    if (st == DYPH_OK) st = join_trajectory(w, w->stream, last);
     w->traj_pending = false;
     cudaError_t ce = cudaStreamEndCapture(w->stream, &g);
     if (st != DYPH_OK) {
@@ -541,10 +711,12 @@ dyph_status fused_smem_prepare() {
     if (dev < 0 || dev >= kFusedMaxDevices) return DYPH_ERR_INVALID;
     std::lock_guard<std::mutex> lock(g_fused_smem_mu);
     if (g_fused_smem[dev]) return DYPH_OK;
-    for (const void* k : {reinterpret_cast<const void*>(scene_frame_kernel<4>),
-                          reinterpret_cast<const void*>(scene_frame_kernel<5>),
-                          reinterpret_cast<const void*>(scene_frame_kernel<6>),
-                          reinterpret_cast<const void*>(scene_frame_record_kernel),
+    for (const void* k : {reinterpret_cast<const void*>(scene_frame_kernel<4, kSceneThreads>),
+                          reinterpret_cast<const void*>(scene_frame_kernel<5, kSceneThreads>),
+                          reinterpret_cast<const void*>(scene_frame_kernel<6, kSceneThreads>),
+                          reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>),
+                          reinterpret_cast<const void*>(scene_frame_record_kernel<4, kSceneThreads>),
+                          reinterpret_cast<const void*>(scene_frame_record_kernel<2, kSceneWideThreads>),
                           reverse_kernel()})
         DYPH_CUDA_TRY(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kMaxSmem)));
     g_fused_smem[dev] = true;
@@ -555,7 +727,7 @@ dyph_status fused_smem_prepare() {
 // share an SM, as the occupancy calculator counts it (static shared memory
 // and the per-block reservation included): the SM's share for one block,
 // lowered in 128-byte steps until that many blocks fit.
-uint32_t smem_for_blocks(const void* kernel, int blocks) {
+uint32_t smem_for_blocks(const void* kernel, int threads, int blocks) {
     int dev = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) {
@@ -565,7 +737,7 @@ uint32_t smem_for_blocks(const void* kernel, int blocks) {
     uint32_t bytes = std::min(kMaxSmem, static_cast<uint32_t>(per_sm / blocks)) & ~127u;
     for (; bytes >= 128u; bytes -= 128u) {
         int fit = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, kSceneThreads, bytes) != cudaSuccess) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, bytes) != cudaSuccess) {
             cudaGetLastError();
             return 0u;
         }
@@ -623,6 +795,15 @@ dyph_status setup_reverse(dyph_world* w) {
     return DYPH_OK;
 }
 
+// The words of a launch's statistics.
+dyph_status run_words(dyph_world* w) {
+    if (w->f_run) return DYPH_OK;
+    const size_t bytes = (kAccWords + 4ull * kMaxRunFrames) * sizeof(uint32_t);
+    if (cudaMalloc(&w->f_run, bytes) != cudaSuccess) return DYPH_ERR_NOMEM;
+    DYPH_CUDA_TRY(cudaMemset(w->f_run, 0, bytes));
+    return DYPH_OK;
+}
+
 dyph_status setup_fused(dyph_world* w, uint32_t n_scenes, const uint32_t* body_offset) {
     w->fused = false;
     w->h_body_offset.assign(body_offset, body_offset + n_scenes + 1);
@@ -638,9 +819,6 @@ dyph_status setup_fused(dyph_world* w, uint32_t n_scenes, const uint32_t* body_o
     dyph_status prep = fused_smem_prepare();
     if (prep != DYPH_OK) return prep;
     uint32_t smem = fused_smem_need(max_nb);
-    const void* variant = w->f_variant == 1   ? reinterpret_cast<const void*>(scene_frame_kernel<5>)
-                          : w->f_variant == 2 ? reinterpret_cast<const void*>(scene_frame_kernel<6>)
-                                              : reinterpret_cast<const void*>(scene_frame_kernel<4>);
     if (w->f_smem_cap) {
         smem = std::max(fused_smem_floor(max_nb), std::min(smem, w->f_smem_cap & ~15u));
     } else {
@@ -649,7 +827,8 @@ dyph_status setup_fused(dyph_world* w, uint32_t n_scenes, const uint32_t* body_o
         int dev = 0, sms = 0;
         DYPH_CUDA_TRY(cudaGetDevice(&dev));
         DYPH_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        const uint32_t two = smem_for_blocks(variant, 2);
+        const uint32_t two = smem_for_blocks(reinterpret_cast<const void*>(scene_frame_kernel<4, kSceneThreads>),
+                                             kSceneThreads, 2);
         if (n_scenes > static_cast<uint32_t>(sms) && smem > two && two >= fused_smem_floor(max_nb)) smem = two;
     }
     uint32_t** bufs[] = {&w->f_pair_base, &w->f_contact_base, &w->f_pair_raw, &w->f_contact_raw, &w->f_color_raw,
@@ -680,7 +859,28 @@ dyph_status setup_fused(dyph_world* w, uint32_t n_scenes, const uint32_t* body_o
     DYPH_CUDA_TRY(cudaMemcpy(w->f_pair_base, pb.data(), pb.size() * 4, cudaMemcpyHostToDevice));
     DYPH_CUDA_TRY(cudaMemcpy(w->f_contact_base, cb.data(), cb.size() * 4, cudaMemcpyHostToDevice));
     DYPH_CUDA_TRY(cudaMemset(w->f_counts, 0, 4ull * n_scenes * sizeof(uint32_t)));
+    prep = run_words(w);
+    if (prep != DYPH_OK) return prep;
     w->frame_smem = smem;
+    {
+        int dev = 0, sms = 0, per_sm = 0;
+        DYPH_CUDA_TRY(cudaGetDevice(&dev));
+        DYPH_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        w->f_threads = kSceneThreads;
+        FusedForm form = fused_form(w);
+        DYPH_CUDA_TRY(
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form.kernel, static_cast<int>(form.threads), smem));
+        // Blocks of twice the threads where the chip would otherwise hold at most
+        // half the warps the registers allow: shared memory for two blocks an SM
+        // at most, or hardly more blocks than SMs.
+        if (w->f_variant == 0 && (per_sm <= 2 || w->f_n_items <= 2u * static_cast<uint32_t>(sms))) {
+            w->f_threads = kSceneWideThreads;
+            form = fused_form(w);
+            DYPH_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form.kernel,
+                                                                        static_cast<int>(form.threads), smem));
+        }
+        w->f_resident = w->f_n_items <= static_cast<uint32_t>(per_sm) * static_cast<uint32_t>(sms);
+    }
     w->f_warp_scenes = n_small;
     w->f_half_scenes = n_mid;
     w->f_block_scenes = n_scenes - n_small - n_mid;
@@ -701,10 +901,8 @@ void fused_report(const dyph_world* w, dyph_fused_config* out) {
     *out = dyph_fused_config{};
     if (!w->fused) return;
     int per_sm = 0;
-    const void* k = w->f_variant == 1   ? reinterpret_cast<const void*>(scene_frame_kernel<5>)
-                    : w->f_variant == 2 ? reinterpret_cast<const void*>(scene_frame_kernel<6>)
-                                        : reinterpret_cast<const void*>(scene_frame_kernel<4>);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kSceneThreads, w->frame_smem);
+    const FusedForm form = fused_form(w);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form.kernel, static_cast<int>(form.threads), w->frame_smem);
     out->smem_bytes = w->frame_smem;
     out->teams = w->f_teams;
     out->warp_scenes = w->f_warp_scenes;
@@ -880,11 +1078,12 @@ extern "C" dyph_status dyph_world_autotune(dyph_world* w, int32_t frames, dyph_s
                 w->f_variant = variant;
                 st = setup_fused(w, static_cast<uint32_t>(w->h_body_offset.size() - 1), w->h_body_offset.data());
                 if (st != DYPH_OK) break;
-                // one untimed frame, then the timed ones, each trial from the saved state
-                for (int f = 0; f <= frames && st == DYPH_OK; ++f) {
-                    if (f == 1 && cudaEventRecord(e0, w->stream) != cudaSuccess) st = DYPH_ERR_CUDA;
-                    if (st == DYPH_OK) st = enqueue_frame(w, w->stream);
-                }
+                // one untimed frame, then the timed ones as one run, each trial from the saved state
+                st = launch_run(w, FusedRun{1u}, w->stream);
+                if (st == DYPH_OK && cudaEventRecord(e0, w->stream) != cudaSuccess) st = DYPH_ERR_CUDA;
+                const uint32_t run = w->f_resident ? kMaxRunFrames : 1u;
+                for (uint32_t f = 0; f < static_cast<uint32_t>(frames) && st == DYPH_OK; f += run)
+                    st = launch_run(w, FusedRun{std::min(static_cast<uint32_t>(frames) - f, run)}, w->stream);
                 if (st == DYPH_OK && cudaEventRecord(e1, w->stream) != cudaSuccess) st = DYPH_ERR_CUDA;
                 if (st == DYPH_OK && (copy_rows(false) != cudaSuccess || cudaStreamSynchronize(w->stream) != cudaSuccess))
                     st = DYPH_ERR_CUDA;
@@ -981,6 +1180,7 @@ extern "C" dyph_status dyph_world_set_trajectory(dyph_world* w, float* host_dst,
     w->traj_every = every;
     w->traj_max = max_records;
     w->traj_frame = 0;
+    w->traj_chunk = 0;
     w->traj_pending = false;
     w->traj_live[0] = w->traj_live[1] = false;
     if (!host_dst) return DYPH_OK;
@@ -990,13 +1190,26 @@ extern "C" dyph_status dyph_world_set_trajectory(dyph_world* w, float* host_dst,
         w->traj_host = nullptr;
         return DYPH_ERR_INVALID;  // pageable memory: the copies could not run asynchronously or be captured
     }
+    // A single scene's frames are recorded one by one, a fused batch's a few to
+    // a launch: staging buffers of at most 64 MiB and 8 records.
     const size_t bytes = 7ull * w->desc.bodies.n * sizeof(float);
+    const uint32_t slots =
+        w->fused ? static_cast<uint32_t>(std::clamp<size_t>((size_t(64) << 20) / bytes, 1, 8)) : 1u;
     for (int k = 0; k < 2; ++k) {
-        if (!w->traj_stage[k] && cudaMalloc(&w->traj_stage[k], bytes) != cudaSuccess) return DYPH_ERR_NOMEM;
+        if (w->traj_stage[k] && slots > w->traj_slots) {
+            cudaFree(w->traj_stage[k]);
+            w->traj_stage[k] = nullptr;
+        }
+        if (!w->traj_stage[k] && cudaMalloc(&w->traj_stage[k], slots * bytes) != cudaSuccess) {
+            w->traj_host = nullptr;
+            w->traj_slots = 0;
+            return DYPH_ERR_NOMEM;
+        }
         if (!w->traj_packed[k]) DYPH_CUDA_TRY(cudaEventCreateWithFlags(&w->traj_packed[k], cudaEventDisableTiming));
         if (!w->traj_copied[k]) DYPH_CUDA_TRY(cudaEventCreateWithFlags(&w->traj_copied[k], cudaEventDisableTiming));
     }
     if (!w->traj_stream) DYPH_CUDA_TRY(cudaStreamCreateWithFlags(&w->traj_stream, cudaStreamNonBlocking));
+    w->traj_slots = std::max(w->traj_slots, slots);
     return DYPH_OK;
 }
 
@@ -1032,42 +1245,6 @@ extern "C" dyph_status dyph_world_download_phase_ns(dyph_world* w, dyph_stream s
 namespace dyph {
 namespace {
 
-// State rows (pos xyz, rot wxyz, vel xyz, ang xyz) of every body to / from a
-// [13][n] buffer.
-__global__ void pack_state_kernel(GlobalBodies B, float* __restrict__ out) {
-    const uint32_t n = B.v.n;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float v[13] = {B.px(i), B.py(i), B.pz(i), B.qw(i), B.qx(i), B.qy(i), B.qz(i),
-                             B.vx(i), B.vy(i), B.vz(i), B.wx(i), B.wy(i), B.wz(i)};
-        for (int r = 0; r < 13; ++r) out[static_cast<size_t>(r) * n + i] = v[r];
-    }
-}
-
-__global__ void unpack_state_kernel(const float* __restrict__ in, GlobalBodies B) {
-    const uint32_t n = B.v.n;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float* r = in + i;
-        B.px(i) = r[0]; B.py(i) = r[n]; B.pz(i) = r[2ull * n];
-        B.qw(i) = r[3ull * n]; B.qx(i) = r[4ull * n]; B.qy(i) = r[5ull * n]; B.qz(i) = r[6ull * n];
-        B.vx(i) = r[7ull * n]; B.vy(i) = r[8ull * n]; B.vz(i) = r[9ull * n];
-        B.wx(i) = r[10ull * n]; B.wy(i) = r[11ull * n]; B.wz(i) = r[12ull * n];
-    }
-}
-
-dyph_status pack_state(const dyph_world* w, float* out, cudaStream_t s) {
-    const uint32_t n = w->desc.bodies.n;
-    pack_state_kernel<<<(n + 255) / 256, 256, 0, s>>>(GlobalBodies{w->desc.bodies}, out);
-    DYPH_CUDA_TRY(cudaGetLastError());
-    return DYPH_OK;
-}
-
-dyph_status unpack_state(const dyph_world* w, const float* in, cudaStream_t s) {
-    const uint32_t n = w->desc.bodies.n;
-    unpack_state_kernel<<<(n + 255) / 256, 256, 0, s>>>(in, GlobalBodies{w->desc.bodies});
-    DYPH_CUDA_TRY(cudaGetLastError());
-    return DYPH_OK;
-}
-
 // A BodyView over a [13][n] state buffer, with the world's constant rows.
 dyph_bodies state_view(const dyph_world* w, float* st) {
     dyph_bodies v = w->desc.bodies;
@@ -1099,9 +1276,9 @@ size_t record_set_bytes(const dyph_world* w) {
 dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
     const size_t n = w->desc.bodies.n;
     const uint32_t n_sc = std::max(w->bp->n_scenes, 1u);
-    if (!w->a_g[0]) {
-        const bool ok = cudaMalloc(&w->a_g[0], 13 * n * 4) == cudaSuccess &&
-                        cudaMalloc(&w->a_g[1], 13 * n * 4) == cudaSuccess && cudaMalloc(&w->a_flag, 4) == cudaSuccess;
+    if (!w->a_g) {
+        const bool ok =
+            cudaMalloc(&w->a_g, 13 * n * 4) == cudaSuccess && cudaMalloc(&w->a_flag, 4) == cudaSuccess;
         if (!ok) return DYPH_ERR_NOMEM;
         DYPH_CUDA_TRY(cudaStreamCreateWithFlags(&w->a_stream, cudaStreamNonBlocking));
         for (cudaEvent_t* e : {&w->a_seg_ready, &w->a_rtail, &w->a_rev_done})
@@ -1119,6 +1296,8 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
         w->a_qs.clear();
         w->a_words.clear();
         w->a_mg.clear();
+        if (w->a_sets) cudaFree(w->a_sets);
+        w->a_sets = nullptr;
         if (w->a_pairs) cudaFree(w->a_pairs);
         w->a_pairs = nullptr;
         std::fill(w->a_sized, w->a_sized + 4, 0u);
@@ -1126,6 +1305,7 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
             return DYPH_ERR_NOMEM;
         std::copy(sized, sized + 4, w->a_sized);
     }
+    const bool grow = w->a_rec.size() < sets;
     while (w->a_rec.size() < sets) {
         float *rec = nullptr, *pose1 = nullptr, *qs = nullptr;
         uint32_t *words = nullptr, *mg = nullptr;
@@ -1146,6 +1326,15 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
         w->a_words.push_back(words);
         w->a_mg.push_back(mg);
     }
+    if (grow || !w->a_sets) {
+        std::vector<AdjSet> table(w->a_rec.size());
+        for (size_t k = 0; k < table.size(); ++k)
+            table[k] = AdjSet{w->a_rec[k], w->a_pose1[k], w->a_qs[k], w->a_words[k], w->a_mg[k]};
+        if (w->a_sets) cudaFree(w->a_sets);
+        w->a_sets = nullptr;
+        if (cudaMalloc(&w->a_sets, table.size() * sizeof(AdjSet)) != cudaSuccess) return DYPH_ERR_NOMEM;
+        DYPH_CUDA_TRY(cudaMemcpy(w->a_sets, table.data(), table.size() * sizeof(AdjSet), cudaMemcpyHostToDevice));
+    }
     if (seg_states > w->a_seg_frames) {
         for (float*& b : w->a_seg) {
             if (b) cudaFree(b);
@@ -1165,17 +1354,7 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
 extern "C" dyph_status dyph_world_rollout(dyph_world* w, int32_t n_frames, int32_t every, float* d_ckpt,
                                           dyph_stream s) {
     if (!w || !w->fused || n_frames <= 0 || every <= 0 || !d_ckpt) return DYPH_ERR_INVALID;
-    const size_t n = w->desc.bodies.n;
-    cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
-    for (int32_t f = 0; f < n_frames; ++f) {
-        if (f % every == 0) {
-            dyph_status st = pack_state(w, d_ckpt + static_cast<size_t>(f / every) * 13 * n, cs);
-            if (st != DYPH_OK) return st;
-        }
-        dyph_status st = dyph_world_step(w, 1, s);
-        if (st != DYPH_OK) return st;
-    }
-    return DYPH_OK;
+    return world_step(w, n_frames, s, d_ckpt, static_cast<uint32_t>(every));
 }
 
 extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_frames, int32_t every,
@@ -1184,7 +1363,8 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     if (!w || !w->fused || n_frames <= 0 || every <= 0 || !d_ckpt || !d_grad_final || !d_grad_init ||
         !d_grad_inv_mass)
         return DYPH_ERR_INVALID;
-    // Frames are recorded in segments on a_stream, one record set per frame;
+    // Frames are recorded in segments on a_stream, one launch a segment and one
+    // record set per frame;
     // sets alternate between two segments, so segment seg - 1 is recorded
     // while segment seg is reversed on the caller's stream, last frame first.
     // With checkpoints every `every` > 1 frames a segment is a checkpoint's
@@ -1211,7 +1391,7 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
     DYPH_CUDA_TRY(cudaMemsetAsync(w->a_flag, 0, 4, cs));
     DYPH_CUDA_TRY(cudaMemsetAsync(d_grad_inv_mass, 0, n * 4, cs));
-    DYPH_CUDA_TRY(cudaMemcpyAsync(w->a_g[0], d_grad_final, 13 * n * 4, cudaMemcpyDeviceToDevice, cs));
+    DYPH_CUDA_TRY(cudaMemcpyAsync(w->a_g, d_grad_final, 13 * n * 4, cudaMemcpyDeviceToDevice, cs));
     const dyph_world_desc& d = w->desc;
     const dyph_integrator_params& ip = d.integrator;
     const float sub_dt = ip.dt / static_cast<float>(ip.n_substeps);
@@ -1221,40 +1401,46 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     S_rev.smem_bytes = w->r_smem;
     auto seg_len = [&](int32_t seg) { return std::min(group, n_frames - seg * group); };
     auto ckpt = [&](int32_t c) { return d_ckpt + static_cast<size_t>(c) * 13 * n; };
-    // Frame f's start state: its segment's checkpoint, or the state its
-    // predecessor's recording stored. The record and reverse kernels only
-    // read it, so a checkpoint serves directly.
-    auto state = [&](int32_t f) {
-        const int32_t seg = f / every, j = f % every;
-        return j == 0 ? const_cast<float*>(ckpt(seg)) : w->a_seg[seg & 1] + static_cast<size_t>(j - 1) * 13 * n;
+    // Segment seg's frames. Frame f starts from its segment's checkpoint, or from
+    // the state its predecessor's recording stored (with a checkpoint at every
+    // frame, from its own checkpoint). The kernels only read a checkpoint.
+    auto segment = [&](int32_t seg) {
+        float* state1 = every > 1 ? w->a_seg[seg & 1] : const_cast<float*>(ckpt(seg * group)) + 13 * n;
+        const float* state0 = ckpt(every > 1 ? seg : seg * group);
+        return AdjSegment{w->a_sets + static_cast<size_t>(seg & 1) * seg_frames, w->f_contact_slots,
+                          static_cast<uint32_t>(n), w->a_flag, state0, state1, every > 1 ? 1u : 0u};
     };
-    auto set_of = [&](int32_t f) { return static_cast<size_t>(((f / group) & 1) * seg_frames + f % group); };
-    auto params = [&](int32_t f) {
-        return FrameParams{state_view(w, state(f)), d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt,
-                           0.5f * sub_dt, w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(w->sv->mode),
-                           w->sv->n_iters, w->sv->meta, w->bp->counts, w->np->counts, w->stats + 4, nullptr};
+    auto params = [&](int32_t seg) {
+        FrameParams p{};
+        p.gb = state_view(w, const_cast<float*>(segment(seg).state0));
+        p.gs = d.shapes;
+        p.gx = ip.gravity[0];
+        p.gy = ip.gravity[1];
+        p.gz = ip.gravity[2];
+        p.sub_dt = sub_dt;
+        p.half_dt = 0.5f * sub_dt;
+        p.mu = w->sv->friction;
+        p.dt = ip.dt;
+        p.n_substeps = ip.n_substeps;
+        p.mode = static_cast<int>(w->sv->mode);
+        p.n_iters = w->sv->n_iters;
+        p.status = w->stats + 4;
+        p.n_frames = static_cast<uint32_t>(seg_len(seg));
+        return p;
     };
-    auto adj = [&](int32_t f, float* store) {
-        const size_t k = set_of(f);
-        return AdjRun{w->a_rec[k], w->f_contact_slots, w->a_pose1[k], w->a_qs[k], static_cast<uint32_t>(n),
-                      w->a_flag, store};
-    };
-    auto keep = [&](int32_t f) { return AdjKeep{w->a_words[set_of(f)], w->a_mg[set_of(f)]}; };
-    auto frame_bufs = [&](int32_t f) {
-        return FrameBufs{w->f_pair_base, w->f_contact_base, w->a_pairs, w->f_contact_raw, w->f_color_raw,
-                         w->f_counts, w->a_words[set_of(f)], w->f_words_stride, w->f_contact_slots};
-    };
-    // The recordings spill into their own pair slots and keep their contact
-    // words; each but a segment's last stores the next frame's start state.
+    // The recordings spill into their own pair slots; the contact words are a set's.
+    FrameBufs fb{w->f_pair_base, w->f_contact_base, w->a_pairs, w->f_contact_raw, w->f_color_raw,
+                 w->f_counts, nullptr, w->f_words_stride, w->f_contact_slots};
     auto record_segment = [&](int32_t seg) -> dyph_status {
-        const int32_t f0 = seg * group, len = seg_len(seg);
-        for (int32_t j = 0; j < len; ++j) {
-            const int32_t f = f0 + j;
-            float* store = every > 1 && j + 1 < len ? state(f + 1) : nullptr;
-            scene_frame_record_kernel<<<w->f_n_items, kSceneThreads, w->frame_smem, w->a_stream>>>(
-                S, frame_bufs(f), params(f), adj(f, store), keep(f), w->f_items, w->f_n_items);
-            DYPH_CUDA_TRY(cudaGetLastError());
-        }
+        const bool wide = w->f_threads == static_cast<uint32_t>(kSceneWideThreads);
+        const void* kernel =
+            wide ? reinterpret_cast<const void*>(scene_frame_record_kernel<2, kSceneWideThreads>)
+                 : reinterpret_cast<const void*>(scene_frame_record_kernel<4, kSceneThreads>);
+        FrameParams p = params(seg);
+        AdjSegment ds = segment(seg);
+        void* args[] = {&S, &fb, &p, &ds, &w->f_items, &w->f_n_items};
+        DYPH_CUDA_TRY(cudaLaunchKernel(kernel, dim3(w->f_n_items), dim3(w->f_threads), args, w->frame_smem,
+                                       w->a_stream));
         DYPH_CUDA_TRY(cudaEventRecord(w->a_seg_ready, w->a_stream));
         return DYPH_OK;
     };
@@ -1262,7 +1448,6 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     DYPH_CUDA_TRY(cudaEventRecord(w->a_rtail, cs));
     DYPH_CUDA_TRY(cudaStreamWaitEvent(w->a_stream, w->a_rtail, 0));
     if ((st = record_segment(n_seg - 1)) != DYPH_OK) return st;
-    int cur = 0;
     for (int32_t seg = n_seg - 1; seg >= 0; --seg) {
         DYPH_CUDA_TRY(cudaStreamWaitEvent(cs, w->a_seg_ready, 0));
         if (seg > 0) {
@@ -1271,23 +1456,17 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
             if (seg + 1 < n_seg) DYPH_CUDA_TRY(cudaStreamWaitEvent(w->a_stream, w->a_rev_done, 0));
             if ((st = record_segment(seg - 1)) != DYPH_OK) return st;
         }
-        for (int32_t f = seg * group + seg_len(seg) - 1; f >= seg * group; --f) {
-            AdjFrame G{w->a_g[cur], w->a_g[cur ^ 1], d_grad_inv_mass};
-            FrameBufs fb = frame_bufs(f);
-            FrameParams pf = params(f);
-            AdjRun af = adj(f, nullptr);
-            AdjKeep kf = keep(f);
-            void* args[] = {&S_rev, &fb, &pf, &af, &kf, &G, &w->r_items, &w->r_n_items};
-            DYPH_CUDA_TRY(
-                cudaLaunchKernel(reverse_kernel(), dim3(w->r_n_items), dim3(kSceneThreads), args, w->r_smem, cs));
-            cur ^= 1;
-        }
+        AdjFrame G{w->a_g, d_grad_inv_mass};
+        FrameParams ps = params(seg);
+        AdjSegment ds = segment(seg);
+        void* args[] = {&S_rev, &fb, &ps, &ds, &G, &w->r_items, &w->r_n_items};
+        DYPH_CUDA_TRY(cudaLaunchKernel(reverse_kernel(), dim3(w->r_n_items), dim3(kSceneThreads), args, w->r_smem, cs));
         DYPH_CUDA_TRY(cudaEventRecord(w->a_rev_done, cs));
     }
     // the side stream ends before the caller's stream goes on
     DYPH_CUDA_TRY(cudaEventRecord(w->a_rtail, w->a_stream));
     DYPH_CUDA_TRY(cudaStreamWaitEvent(cs, w->a_rtail, 0));
-    DYPH_CUDA_TRY(cudaMemcpyAsync(d_grad_init, w->a_g[cur], 13 * n * 4, cudaMemcpyDeviceToDevice, cs));
+    DYPH_CUDA_TRY(cudaMemcpyAsync(d_grad_init, w->a_g, 13 * n * 4, cudaMemcpyDeviceToDevice, cs));
     uint32_t flag = 0;
     DYPH_CUDA_TRY(cudaMemcpyAsync(&flag, w->a_flag, 4, cudaMemcpyDeviceToHost, cs));
     DYPH_CUDA_TRY(cudaStreamSynchronize(cs));
