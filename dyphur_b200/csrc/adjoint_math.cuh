@@ -395,214 +395,199 @@ struct BodyBar {
     float im;
 };
 
-// solve_contact on the pair (L body 0 = a, body 1 = b) from its pre-solve
-// state, with the branch flags `fl` the forward solve recorded. G0 / G1 hold
-// the adjoint of the post-solve state on entry and of the pre-solve state on
-// return (im accumulates); pb, nb, db receive the contact geometry's adjoint.
+// The sum of a lane pair's values, body a's first.
+__device__ __forceinline__ float sum_sides(bool is_b, float mine) {
+    float a, b;
+    both_sides(is_b, mine, a, b);
+    return a + b;
+}
+__device__ __forceinline__ F3 sum_sides(bool is_b, F3 v) {
+    return f3(sum_sides(is_b, v.x), sum_sides(is_b, v.y), sum_sides(is_b, v.z));
+}
+// body a's vector minus body b's
+__device__ __forceinline__ F3 diff_sides(bool is_b, F3 v) {
+    F3 a, b;
+    both_sides(is_b, v.x, a.x, b.x);
+    both_sides(is_b, v.y, a.y, b.y);
+    both_sides(is_b, v.z, a.z, b.z);
+    return a - b;
+}
+
+// The adjoint of solve_contact from its pre-solve state, with the branch flags
+// `fl` the forward solve recorded, on a lane pair as solve_contact_side: each
+// lane holds one body (S, its adjoint G), the scalars of both cross by shuffles.
+// The two bodies' terms are alike up to the sign sg of the contact's action.
+// The whole warp calls it; pairs with fl == 0 do nothing. G is the adjoint of the
+// body's post-solve state on entry and of the pre-solve state on return (im
+// accumulates); pb, nb, db receive the contact geometry's adjoint (both lanes).
 // lc_in is lambda before the solve.
-__device__ __forceinline__ void solve_contact_adj(const LocalPair& L, const Contact& ct, float mu, float dt,
-                                                  float lc_in, uint32_t fl, BodyBar& G0, BodyBar& G1, F3& pb,
-                                                  F3& nb, float& db) {
-    if (!(fl & kSfActive)) return;
-    const float wa = L.m[0], wb = L.m[1];
-    const bool da = wa != 0.f, dbn = wb != 0.f;
-    const F3 n = f3(ct.nx, ct.ny, ct.nz), p = f3(ct.px, ct.py, ct.pz);
-    const F3 xa = f3(L.p[0][0], L.p[0][1], L.p[0][2]), xb = f3(L.p[1][0], L.p[1][1], L.p[1][2]);
-    const F3 va = f3(L.v[0][0], L.v[0][1], L.v[0][2]), vb = f3(L.v[1][0], L.v[1][1], L.v[1][2]);
-    const F3 oa = f3(L.w[0][0], L.w[0][1], L.w[0][2]), ob = f3(L.w[1][0], L.w[1][1], L.w[1][2]);
-    const float* qa = L.q[0];
-    const float* qbq = L.q[1];
-    const F3 ra = p - xa, rb = p - xb;
-    const F3 ca = cross(ra, n), cb = cross(rb, n);
-    const F3 ua = winv(qa, L.I[0], ca), ub = winv(qbq, L.I[1], cb);
-    const float w = wa + wb + dot(ca, ua) + dot(cb, ub);
+__device__ __forceinline__ void solve_contact_side_adj(bool is_b, const SideBody& S, const Contact& ct, float mu,
+                                                       float dt, float lc_in, uint32_t fl, BodyBar& G, F3& pb, F3& nb,
+                                                       float& db) {
+    constexpr unsigned kAll = 0xffffffffu;
+    const F3 zero = f3(0.f, 0.f, 0.f);
+    const bool act = fl & kSfActive, normal = fl & kSfNormal, fr = fl & kSfFriction, clamped = fl & kSfClamped;
+    const float m = S.m, sg = is_b ? -1.f : 1.f, sm = sg * m;
+    const bool dyn = m != 0.f;
+    const F3 n = f3(ct.nx, ct.ny, ct.nz), o = f3(S.wx, S.wy, S.wz), v = f3(S.vx, S.vy, S.vz);
+    const float q[4] = {S.qw, S.qx, S.qy, S.qz};
+    const float I[6] = {S.ixx, S.iyy, S.izz, S.ixy, S.ixz, S.iyz};
+    const F3 r = f3(ct.px - S.px, ct.py - S.py, ct.pz - S.pz);
+    const F3 c = cross(r, n);
+    const F3 u = winv(q, I, c);
+    float wa, wb, da, dbs;
+    both_sides(is_b, m, wa, wb);
+    both_sides(is_b, dot(c, u), da, dbs);
+    const float w = act ? wa + wb + da + dbs : 1.f;
     const float rem = ct.depth - lc_in;
     const float dl = rem / w;
     const float lc_out = lc_in + rem;
-    // rotations after the position correction
-    float qa1[4] = {qa[0], qa[1], qa[2], qa[3]}, qb1[4] = {qbq[0], qbq[1], qbq[2], qbq[3]};
-    const F3 aa = dl * ua, ab = (-dl) * ub;
-    if (da) {
-        qa1[0] += 0.5f * (-aa.x * qa[1] - aa.y * qa[2] - aa.z * qa[3]);
-        qa1[1] += 0.5f * (aa.x * qa[0] + aa.y * qa[3] - aa.z * qa[2]);
-        qa1[2] += 0.5f * (-aa.x * qa[3] + aa.y * qa[0] + aa.z * qa[1]);
-        qa1[3] += 0.5f * (aa.x * qa[2] - aa.y * qa[1] + aa.z * qa[0]);
-    }
-    if (dbn) {
-        qb1[0] += 0.5f * (-ab.x * qbq[1] - ab.y * qbq[2] - ab.z * qbq[3]);
-        qb1[1] += 0.5f * (ab.x * qbq[0] + ab.y * qbq[3] - ab.z * qbq[2]);
-        qb1[2] += 0.5f * (-ab.x * qbq[3] + ab.y * qbq[0] + ab.z * qbq[1]);
-        qb1[3] += 0.5f * (ab.x * qbq[2] - ab.y * qbq[1] + ab.z * qbq[0]);
+    // rotation after the position correction
+    float q1[4] = {q[0], q[1], q[2], q[3]};
+    const F3 a = (sg * dl) * u;
+    if (dyn) {
+        q1[0] += 0.5f * (-a.x * q[1] - a.y * q[2] - a.z * q[3]);
+        q1[1] += 0.5f * (a.x * q[0] + a.y * q[3] - a.z * q[2]);
+        q1[2] += 0.5f * (-a.x * q[3] + a.y * q[0] + a.z * q[1]);
+        q1[3] += 0.5f * (a.x * q[2] - a.y * q[1] + a.z * q[0]);
     }
     // normal velocity impulse
-    const F3 vrel = (va + cross(oa, ra)) - (vb + cross(ob, rb));
-    const float vreln = dot(vrel, n);
+    const F3 vrel = diff_sides(is_b, v + cross(o, r));
     float jn = 0.f;
-    F3 dA = f3(0.f, 0.f, 0.f), dB = f3(0.f, 0.f, 0.f);
-    F3 va1 = va, vb1 = vb, oa1 = oa, ob1 = ob;
-    if (fl & kSfNormal) {
-        jn = -vreln / w;
-        dA = winv(qa1, L.I[0], ca);
-        dB = winv(qb1, L.I[1], cb);
-        if (da) { va1 += (wa * jn) * n; oa1 += jn * dA; }
-        if (dbn) { vb1 -= (wb * jn) * n; ob1 -= jn * dB; }
+    F3 d = zero, v1 = v, o1 = o;
+    if (normal) {
+        jn = -dot(vrel, n) / w;
+        d = winv(q1, I, c);
+        if (dyn) {
+            v1 += (sm * jn) * n;
+            o1 += (sg * jn) * d;
+        }
     }
     // friction
-    F3 rv = f3(0.f, 0.f, 0.f), vt = rv, t = rv, ea = rv, eb = rv, fa = rv, fb = rv;
-    float rvn = 0.f, Lt = 0.f, wt = 0.f, jt = 0.f, jt_raw = 0.f, jns = 0.f;
-    const bool fr = fl & kSfFriction, clamped = fl & kSfClamped;
-    if (fr) {
-        rv = (va1 + cross(oa1, ra)) - (vb1 + cross(ob1, rb));
-        rvn = dot(rv, n);
-        vt = rv - rvn * n;
-        Lt = sqrtf(dot(vt, vt));
-        t = (1.f / Lt) * vt;
-        ea = cross(ra, t);
-        eb = cross(rb, t);
-        fa = winv(qa1, L.I[0], ea);
-        fb = winv(qb1, L.I[1], eb);
-        wt = wa + wb + dot(ea, fa) + dot(eb, fb);
-        jns = lc_out / (dt * w);
-        jt_raw = Lt / wt;
-        jt = clamped ? mu * jns : jt_raw;
+    const bool any_fr = __any_sync(kAll, fr);
+    F3 rv = zero, vt = zero, t = zero, e = zero, f = zero;
+    float rvn = 0.f, Lt = 1.f, wt = 1.f, jt = 0.f, jt_raw = 0.f;
+    if (any_fr) {
+        rv = diff_sides(is_b, v1 + cross(o1, r));
+        if (fr) {
+            rvn = dot(rv, n);
+            vt = rv - rvn * n;
+            Lt = sqrtf(dot(vt, vt));
+            t = (1.f / Lt) * vt;
+            e = cross(r, t);
+            f = winv(q1, I, e);
+        }
+        float ea, eb;
+        both_sides(is_b, dot(e, f), ea, eb);
+        if (fr) {
+            wt = wa + wb + ea + eb;
+            jt_raw = Lt / wt;
+            jt = clamped ? mu * (lc_out / (dt * w)) : jt_raw;
+        }
     }
-    // ── reverse ──
-    float wab = 0.f, wbb = 0.f, wbar = 0.f, remb = 0.f, dlb = 0.f;
-    F3 rab = f3(0.f, 0.f, 0.f), rbb = rab, cab = rab, cbb = rab, uab = rab, ubb = rab;
-    float qa1b[4] = {G0.q[0], G0.q[1], G0.q[2], G0.q[3]}, qb1b[4] = {G1.q[0], G1.q[1], G1.q[2], G1.q[3]};
-    F3 va1b = G0.v, oa1b = G0.w, vb1b = G1.v, ob1b = G1.w;
-    if (fr) {
-        float jtb = 0.f;
-        F3 tb = f3(0.f, 0.f, 0.f), fab = tb, fbb = tb;
-        if (da) {
-            jtb += -wa * dot(G0.v, t) - dot(G0.w, fa);
-            tb = fmav((-wa * jt), G0.v, tb);
-            fab = fmav((-jt), G0.w, fab);
-            wab += -jt * dot(G0.v, t);
+    // ── reverse ── (mb: this body's inverse mass; wbar, remb, dlb of both)
+    float mb = 0.f, wbar = 0.f, remb = 0.f;
+    F3 rb = zero, cb = zero, nb_own = zero, nb_both = zero;
+    float q1b[4] = {G.q[0], G.q[1], G.q[2], G.q[3]};
+    F3 v1b = G.v, o1b = G.w;
+    if (any_fr) {
+        float jt_part = 0.f;
+        F3 t_part = zero, fb = zero;
+        const float gt = dot(G.v, t);
+        if (fr && dyn) {
+            jt_part = -sm * gt - sg * dot(G.w, f);
+            t_part = (-sm * jt) * G.v;
+            fb = (-sg * jt) * G.w;
+            mb += -sg * jt * gt;
         }
-        if (dbn) {
-            jtb += wb * dot(G1.v, t) + dot(G1.w, fb);
-            tb = fmav((wb * jt), G1.v, tb);
-            fbb = fmav(jt, G1.w, fbb);
-            wbb += jt * dot(G1.v, t);
-        }
+        const float jtb = sum_sides(is_b, jt_part);
         float Ltb = 0.f, wtb = 0.f;
-        if (clamped) {
-            const float jnsb = mu * jtb;
-            remb += jnsb / (dt * w);
-            wbar += -jnsb * lc_out / (dt * w * w);
-        } else {
-            Ltb += jtb / wt;
-            wtb = -jtb * jt_raw / wt;
+        if (fr) {
+            if (clamped) {
+                const float jnsb = mu * jtb;
+                remb += jnsb / (dt * w);
+                wbar += -jnsb * lc_out / (dt * w * w);
+            } else {
+                Ltb = jtb / wt;
+                wtb = -jtb * jt_raw / wt;
+            }
+            mb += wtb;
+            F3 eb = wtb * f;
+            fb = fmav(wtb, e, fb);
+            winv_adj(q1, I, e, fb, eb, q1b);
+            rb += cross(t, eb);
+            t_part += cross(eb, r);
         }
-        wab += wtb;
-        wbb += wtb;
-        F3 eab = wtb * fa, ebb = wtb * fb;
-        fab = fmav(wtb, ea, fab);
-        fbb = fmav(wtb, eb, fbb);
-        winv_adj(qa1, L.I[0], ea, fab, eab, qa1b);
-        winv_adj(qb1, L.I[1], eb, fbb, ebb, qb1b);
-        rab += cross(t, eab);
-        tb += cross(eab, ra);
-        rbb += cross(t, ebb);
-        tb += cross(ebb, rb);
-        F3 vtb = (1.f / Lt) * tb;
-        Ltb += -dot(tb, vt) / (Lt * Lt);
-        vtb = fmav((Ltb / Lt), vt, vtb);
-        const F3 rvb0 = vtb;
-        const float rvnb = -dot(vtb, n);
-        nb = fmav((-rvn), vtb, nb);
-        const F3 rvb = rvb0 + rvnb * n;
-        nb = fmav(rvnb, rv, nb);
-        va1b += rvb;
-        oa1b += cross(ra, rvb);
-        rab += cross(rvb, oa1);
-        vb1b -= rvb;
-        ob1b -= cross(rb, rvb);
-        rbb -= cross(rvb, ob1);
+        const F3 tb = sum_sides(is_b, t_part);
+        if (fr) {
+            F3 vtb = (1.f / Lt) * tb;
+            Ltb += -dot(tb, vt) / (Lt * Lt);
+            vtb = fmav(Ltb / Lt, vt, vtb);
+            const float rvnb = -dot(vtb, n);
+            nb_both = fmav(rvnb, rv, fmav(-rvn, vtb, nb_both));
+            const F3 rvb = vtb + rvnb * n;
+            v1b += sg * rvb;
+            o1b += sg * cross(r, rvb);
+            rb += sg * cross(rvb, o1);
+        }
     }
-    F3 vab = va1b, oab = oa1b, vbb = vb1b, obb = ob1b;
-    if (fl & kSfNormal) {
-        float jnb = 0.f;
-        F3 dAb = f3(0.f, 0.f, 0.f), dBb = dAb;
-        if (da) {
-            jnb += wa * dot(va1b, n) + dot(oa1b, dA);
-            nb = fmav((wa * jn), va1b, nb);
-            wab += jn * dot(va1b, n);
-            dAb = fmav(jn, oa1b, dAb);
+    F3 vb = v1b, ob = o1b;
+    if (__any_sync(kAll, normal)) {
+        float jn_part = 0.f;
+        F3 dbar = zero;
+        const float vn = dot(v1b, n);
+        if (normal && dyn) {
+            jn_part = sm * vn + sg * dot(o1b, d);
+            nb_own = fmav(sm * jn, v1b, nb_own);
+            mb += sg * jn * vn;
+            dbar = (sg * jn) * o1b;
         }
-        if (dbn) {
-            jnb += -wb * dot(vb1b, n) - dot(ob1b, dB);
-            nb = fmav((-wb * jn), vb1b, nb);
-            wbb += -jn * dot(vb1b, n);
-            dBb = fmav((-jn), ob1b, dBb);
+        const float jnb = sum_sides(is_b, jn_part);
+        if (normal) {
+            winv_adj(q1, I, c, dbar, cb, q1b);
+            const float vrelnb = -jnb / w;
+            wbar += -jnb * jn / w;
+            const F3 vrelb = vrelnb * n;
+            nb_both = fmav(vrelnb, vrel, nb_both);
+            vb += sg * vrelb;
+            ob += sg * cross(r, vrelb);
+            rb += sg * cross(vrelb, o);
         }
-        winv_adj(qa1, L.I[0], ca, dAb, cab, qa1b);
-        winv_adj(qb1, L.I[1], cb, dBb, cbb, qb1b);
-        const float vrelnb = -jnb / w;
-        wbar += -jnb * jn / w;
-        const F3 vrelb = vrelnb * n;
-        nb = fmav(vrelnb, vrel, nb);
-        vab += vrelb;
-        oab += cross(ra, vrelb);
-        rab += cross(vrelb, oa);
-        vbb -= vrelb;
-        obb -= cross(rb, vrelb);
-        rbb -= cross(vrelb, ob);
     }
     // rotation and position corrections
-    float qab[4] = {qa1b[0], qa1b[1], qa1b[2], qa1b[3]}, qbb[4] = {qb1b[0], qb1b[1], qb1b[2], qb1b[3]};
-    if (da) {
-        F3 aab = f3(0.f, 0.f, 0.f);
+    float qb[4] = {q1b[0], q1b[1], q1b[2], q1b[3]};
+    float dl_part = 0.f;
+    F3 ub = zero;
+    if (dyn) {
+        F3 ab = zero;
         float qin[4] = {0.f, 0.f, 0.f, 0.f};
-        quat_delta_adj(qa, aa, 0.5f, qa1b, qin, aab);
-        for (int k = 0; k < 4; ++k) qab[k] = qin[k];
-        dlb += dot(aab, ua);
-        uab = fmav(dl, aab, uab);
-        dlb += wa * dot(G0.x, n);
-        wab += dl * dot(G0.x, n);
-        nb = fmav((wa * dl), G0.x, nb);
+        quat_delta_adj(q, a, 0.5f, q1b, qin, ab);
+        for (int k = 0; k < 4; ++k) qb[k] = qin[k];
+        const float gn = dot(G.x, n);
+        dl_part = sg * dot(ab, u) + sm * gn;
+        ub = (sg * dl) * ab;
+        mb += sg * dl * gn;
+        nb_own = fmav(sm * dl, G.x, nb_own);
     }
-    if (dbn) {
-        F3 abb = f3(0.f, 0.f, 0.f);
-        float qin[4] = {0.f, 0.f, 0.f, 0.f};
-        quat_delta_adj(qbq, ab, 0.5f, qb1b, qin, abb);
-        for (int k = 0; k < 4; ++k) qbb[k] = qin[k];
-        dlb += -dot(abb, ub);
-        ubb = fmav((-dl), abb, ubb);
-        dlb += -wb * dot(G1.x, n);
-        wbb += -dl * dot(G1.x, n);
-        nb = fmav((-wb * dl), G1.x, nb);
-    }
+    const float dlb = sum_sides(is_b, dl_part);
     remb += dlb / w;
     wbar += -dlb * dl / w;
-    wab += wbar;
-    wbb += wbar;
-    cab = fmav(wbar, ua, cab);
-    uab = fmav(wbar, ca, uab);
-    cbb = fmav(wbar, ub, cbb);
-    ubb = fmav(wbar, cb, ubb);
-    winv_adj(qa, L.I[0], ca, uab, cab, qab);
-    winv_adj(qbq, L.I[1], cb, ubb, cbb, qbb);
-    rab += cross(n, cab);
-    nb += cross(cab, ra);
-    rbb += cross(n, cbb);
-    nb += cross(cbb, rb);
-    pb += rab + rbb;
-    // outputs: adjoint of the pre-solve state
-    G0.x -= rab;
-    G1.x -= rbb;
-    for (int k = 0; k < 4; ++k) {
-        G0.q[k] = qab[k];
-        G1.q[k] = qbb[k];
-    }
-    G0.v = vab;
-    G0.w = oab;
-    G1.v = vbb;
-    G1.w = obb;
-    G0.im += wab;
-    G1.im += wbb;
-    db += remb;
+    mb += wbar;
+    cb = fmav(wbar, u, cb);
+    ub = fmav(wbar, c, ub);
+    winv_adj(q, I, c, ub, cb, qb);
+    rb += cross(n, cb);
+    nb_own += cross(cb, r);
+    pb = sum_sides(is_b, rb);
+    nb = nb_both + sum_sides(is_b, nb_own);
+    db = remb;
+    if (!act) return;
+    // the adjoint of the pre-solve state
+    G.x -= rb;
+    for (int k = 0; k < 4; ++k) G.q[k] = qb[k];
+    G.v = vb;
+    G.w = ob;
+    G.im += mb;
 }
 
 }  // namespace dyph

@@ -385,32 +385,6 @@ __device__ __forceinline__ int solve_contact(const Bodies& B, const Contact& ct,
 
 namespace dyph {
 
-// The two bodies of one contact held in registers (index 0 = body a, 1 = body
-// b), the reverse pass's pre-solve states.
-struct LocalPair {
-    float p[2][3], q[2][4], v[2][3], w[2][3], m[2], I[2][6];
-    __device__ __forceinline__ float& px(uint32_t i) { return p[i][0]; }
-    __device__ __forceinline__ float& py(uint32_t i) { return p[i][1]; }
-    __device__ __forceinline__ float& pz(uint32_t i) { return p[i][2]; }
-    __device__ __forceinline__ float& qw(uint32_t i) { return q[i][0]; }
-    __device__ __forceinline__ float& qx(uint32_t i) { return q[i][1]; }
-    __device__ __forceinline__ float& qy(uint32_t i) { return q[i][2]; }
-    __device__ __forceinline__ float& qz(uint32_t i) { return q[i][3]; }
-    __device__ __forceinline__ float& vx(uint32_t i) { return v[i][0]; }
-    __device__ __forceinline__ float& vy(uint32_t i) { return v[i][1]; }
-    __device__ __forceinline__ float& vz(uint32_t i) { return v[i][2]; }
-    __device__ __forceinline__ float& wx(uint32_t i) { return w[i][0]; }
-    __device__ __forceinline__ float& wy(uint32_t i) { return w[i][1]; }
-    __device__ __forceinline__ float& wz(uint32_t i) { return w[i][2]; }
-    __device__ __forceinline__ float im(uint32_t i) const { return m[i]; }
-    __device__ __forceinline__ float ixx(uint32_t i) const { return I[i][0]; }
-    __device__ __forceinline__ float iyy(uint32_t i) const { return I[i][1]; }
-    __device__ __forceinline__ float izz(uint32_t i) const { return I[i][2]; }
-    __device__ __forceinline__ float ixy(uint32_t i) const { return I[i][3]; }
-    __device__ __forceinline__ float ixz(uint32_t i) const { return I[i][4]; }
-    __device__ __forceinline__ float iyz(uint32_t i) const { return I[i][5]; }
-};
-
 // ── one contact on two lanes ────────────────────────────────────────────────
 // Contact solves wait for one another in long chains of few contacts each, so
 // a solve's latency counts and lanes are idle. solve_contact's work is the same

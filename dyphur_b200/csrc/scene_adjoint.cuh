@@ -13,7 +13,7 @@
 //            memory, and store the frame's end state when asked;
 //   reverse: reverse the renormalisations, then the contact solves group by
 //            group in descending order (a group's contacts share no dynamic
-//            body), each with solve_contact_adj on its recorded pre-solve
+//            body), each with solve_contact_side_adj on its recorded pre-solve
 //            state, then the narrowphase (contact geometry -> the two bodies'
 //            poses after integrate) and the integration.
 // The adjoint of the state at the frame's end comes in, the adjoint of the
@@ -194,58 +194,42 @@ __device__ void reverse_scene(Team& T, uint32_t s, bool first, const float* st0,
         }
         T.sync();
         // ── contact solves, last group first ──
+        // one contact per lane pair, one body each (solve_contact_side_adj)
+        const bool is_b = T.rank() & 1u;
         for (int g = static_cast<int>(n_groups) - 1; g >= 0; --g) {
             const uint32_t end = SC.pa(g + 1);
-            for (uint32_t idx = SC.pa(g) + T.rank(); idx < end; idx += T.size()) {
-                const uint32_t k = SC.ent(idx);
-                const float* r = recb + k;
-                if (r[35ull * rst] == 0.f) continue;  // did not act
+            for (uint32_t i0 = SC.pa(g) + ((T.rank() & ~31u) >> 1); i0 < end; i0 += T.size() >> 1) {  // warp-uniform
+                const uint32_t idx = i0 + ((T.rank() & 31u) >> 1);
+                const uint32_t k = SC.ent(idx < end ? idx : i0);
+                float* r = recb + k;
+                const uint32_t fl = idx < end ? __float_as_uint(r[35ull * rst]) : 0u;  // 0: did not act
+                if (!__any_sync(0xffffffffu, fl != 0u)) continue;
                 const Contact ct = SC.contact(k);
-                const uint32_t ia = ct.a, ib = ct.b;
-                LocalPair L;
-                for (int j = 0; j < 2; ++j) {
-                    const uint32_t bi = j ? ib : ia;
-                    const int o = j ? 13 : 0;
-                    for (int c = 0; c < 3; ++c) L.p[j][c] = r[static_cast<size_t>(o + c) * rst];
-                    for (int c = 0; c < 4; ++c) L.q[j][c] = r[static_cast<size_t>(o + 3 + c) * rst];
-                    for (int c = 0; c < 3; ++c) L.v[j][c] = r[static_cast<size_t>(o + 7 + c) * rst];
-                    for (int c = 0; c < 3; ++c) L.w[j][c] = r[static_cast<size_t>(o + 10 + c) * rst];
-                    L.m[j] = SB.im(bi);
-                    L.I[j][0] = SB.ixx(bi); L.I[j][1] = SB.iyy(bi); L.I[j][2] = SB.izz(bi);
-                    L.I[j][3] = SB.ixy(bi); L.I[j][4] = SB.ixz(bi); L.I[j][5] = SB.iyz(bi);
+                const uint32_t bi = is_b ? ct.b : ct.a, gi = b0 + bi;
+                const float* s13 = r + (is_b ? 13u : 0u) * rst;
+                auto rec = [&](uint32_t row) { return s13[row * rst]; };
+                const SideBody S{rec(0), rec(1), rec(2), rec(3), rec(4), rec(5), rec(6), rec(7), rec(8), rec(9),
+                                 rec(10), rec(11), rec(12), SB.im(bi), SB.ixx(bi), SB.iyy(bi), SB.izz(bi),
+                                 SB.ixy(bi), SB.ixz(bi), SB.iyz(bi)};
+                auto gr = [&](int row) -> float& { return grow(G.g, ns, row, gi); };
+                BodyBar Gb{f3(gr(0), gr(1), gr(2)), {gr(3), gr(4), gr(5), gr(6)}, f3(gr(7), gr(8), gr(9)),
+                           f3(gr(10), gr(11), gr(12)), 0.f};
+                F3 pb, nb3;
+                float db;
+                solve_contact_side_adj(is_b, S, ct, P_.mu, P_.dt, r[26ull * rst], fl, Gb, pb, nb3, db);
+                if (fl == 0u) continue;
+                if (S.m != 0.f) {  // a static body's state is not a variable
+                    gr(0) = Gb.x.x; gr(1) = Gb.x.y; gr(2) = Gb.x.z;
+                    for (int c = 0; c < 4; ++c) gr(3 + c) = Gb.q[c];
+                    gr(7) = Gb.v.x; gr(8) = Gb.v.y; gr(9) = Gb.v.z;
+                    gr(10) = Gb.w.x; gr(11) = Gb.w.y; gr(12) = Gb.w.z;
+                    G.gim[gi] += Gb.im;
                 }
-                BodyBar G0, G1;
-                BodyBar* Gs[2] = {&G0, &G1};
-                for (int j = 0; j < 2; ++j) {
-                    const uint32_t gi = b0 + (j ? ib : ia);
-                    BodyBar& Gj = *Gs[j];
-                    Gj.x = f3(grow(G.g, ns, 0, gi), grow(G.g, ns, 1, gi), grow(G.g, ns, 2, gi));
-                    for (int c = 0; c < 4; ++c) Gj.q[c] = grow(G.g, ns, 3 + c, gi);
-                    Gj.v = f3(grow(G.g, ns, 7, gi), grow(G.g, ns, 8, gi), grow(G.g, ns, 9, gi));
-                    Gj.w = f3(grow(G.g, ns, 10, gi), grow(G.g, ns, 11, gi), grow(G.g, ns, 12, gi));
-                    Gj.im = 0.f;
+                if (!is_b) {
+                    r[28ull * rst] = pb.x; r[29ull * rst] = pb.y; r[30ull * rst] = pb.z;
+                    r[31ull * rst] = nb3.x; r[32ull * rst] = nb3.y; r[33ull * rst] = nb3.z;
+                    r[34ull * rst] = db;
                 }
-                F3 pb = f3(0.f, 0.f, 0.f), nb3 = pb;
-                float db = 0.f;
-                solve_contact_adj(L, ct, P_.mu, P_.dt, r[26ull * rst], __float_as_uint(r[35ull * rst]), G0, G1, pb,
-                                  nb3, db);
-                for (int j = 0; j < 2; ++j) {
-                    if (L.m[j] == 0.f) continue;  // a static body's state is not a variable
-                    const uint32_t gi = b0 + (j ? ib : ia);
-                    const BodyBar& Gj = *Gs[j];
-                    grow(G.g, ns, 0, gi) = Gj.x.x; grow(G.g, ns, 1, gi) = Gj.x.y;
-                    grow(G.g, ns, 2, gi) = Gj.x.z;
-                    for (int c = 0; c < 4; ++c) grow(G.g, ns, 3 + c, gi) = Gj.q[c];
-                    grow(G.g, ns, 7, gi) = Gj.v.x; grow(G.g, ns, 8, gi) = Gj.v.y;
-                    grow(G.g, ns, 9, gi) = Gj.v.z;
-                    grow(G.g, ns, 10, gi) = Gj.w.x; grow(G.g, ns, 11, gi) = Gj.w.y;
-                    grow(G.g, ns, 12, gi) = Gj.w.z;
-                    G.gim[gi] += Gj.im;
-                }
-                float* w = recb + k;
-                w[28ull * rst] = pb.x; w[29ull * rst] = pb.y; w[30ull * rst] = pb.z;
-                w[31ull * rst] = nb3.x; w[32ull * rst] = nb3.y; w[33ull * rst] = nb3.z;
-                w[34ull * rst] = db;
             }
             T.sync();
         }
