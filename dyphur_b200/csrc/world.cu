@@ -5,8 +5,9 @@
 // Narrowphase::run, XpbdSolver::solve. Every count stays on the device, so a
 // frame has no host round trip. A single scene's first step captures one frame
 // into a CUDA graph and every later frame replays it; a batch whose scenes fit
-// a block's shared memory runs on fused kernels. A small kernel at the end folds
-// the pair / contact counts into peak and overflow words.
+// a block's shared memory runs on fused kernels, and so do the frames of a
+// small single scene but a call's last. A small kernel at the end folds the
+// pair / contact counts into peak and overflow words.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -60,6 +61,13 @@ struct dyph_world {
     uint32_t* f_items = nullptr;         // [4 f_n_items] work items of the fused kernel
     uint32_t f_n_items = 0;
     unsigned long long* f_phase = nullptr;  // [kFramePhases] phase timing of fused frames (null = off)
+    // A small single scene's frames but a call's last (solo_prepare): one block of
+    // the fused kernel on one scene. Device words: body, pair and contact ranges,
+    // the work item and counts; then the pair slots and the contact words.
+    uint32_t* s_buf = nullptr;
+    uint32_t s_smem = 0, s_pairs = 0, s_contacts = 0;
+    bool s_off = false;                   // its buffers could not be had
+    dyph_solver_mode graph_mode = DYPH_SOLVER_REFERENCE;  // the solver mode that the captured frame holds
     // Adjoint of fused frames (dyph_world_rollout_backward), allocated on first use.
     // Record sets, one per frame of two checkpoint segments: contact records,
     // poses after integrate, quaternions before renormalisation, contact
@@ -267,23 +275,39 @@ FusedForm fused_form(const dyph_world* w) {
     }
 }
 
-// n_frames frames of every scene in one launch, and their statistics.
+constexpr uint32_t kSoloHead = 16;  // words before a solo scene's pair slots
+
+// n_frames frames of every scene (of the one scene, for a world that is not a
+// batch) in one launch, and their statistics.
 dyph_status launch_run(dyph_world* w, const FusedRun& r, cudaStream_t s) {
     const dyph_world_desc& d = w->desc;
     const dyph_integrator_params& ip = d.integrator;
     const float sub_dt = ip.dt / static_cast<float>(ip.n_substeps);
+    const bool solo = !w->fused;
     SceneBufs S{w->bp->body_offset, w->bp->bvh.scene_of, w->sv->scene_order, nullptr, nullptr, 0, w->bp->n_scenes,
                 w->frame_smem};
     FrameBufs F{w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw,
                 w->f_counts, w->f_words, w->f_words_stride, w->f_contact_slots};
-    const FusedForm form = fused_form(w);
+    FusedForm form = fused_form(w);
+    const uint32_t* items = w->f_items;
+    uint32_t n_items = w->f_n_items, smem = w->frame_smem;
+    if (solo) {
+        uint32_t* h = w->s_buf;
+        S = SceneBufs{h, nullptr, nullptr, nullptr, nullptr, 0, 1u, w->s_smem};
+        F = FrameBufs{h + 2, h + 4, h + kSoloHead, nullptr, nullptr, h + 12, h + kSoloHead + w->s_pairs,
+                      w->s_contacts + 1u, w->s_contacts};
+        items = h + 8;
+        n_items = 1u;
+        smem = w->s_smem;
+        form = {reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>), kSceneWideThreads};
+    }
     FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
-                  w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(w->sv->mode),
+                  w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(solo ? w->graph_mode : w->sv->mode),
                   w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->stats + 4, w->f_phase, r.n_frames,
                   r.keep ? 1u : 0u, r.traj, r.traj_first, std::max(w->traj_every, 1u), r.traj_count, r.ckpt,
                   r.ckpt_first, r.ckpt_every};
-    void* args[] = {&S, &F, &P, &w->f_items, &w->f_n_items};
-    DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(w->f_n_items), dim3(form.threads), args, w->frame_smem, s));
+    void* args[] = {&S, &F, &P, &items, &n_items};
+    DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(n_items), dim3(form.threads), args, smem, s));
     frame_run_stats_kernel<<<1, kMaxRunFrames, 0, s>>>(w->f_run, r.n_frames, w->bp->counts, w->np->counts, w->sv->meta,
                                                       w->bp->max_pairs, w->np->max_contacts, w->stats);
     DYPH_CUDA_TRY(cudaGetLastError());
@@ -407,7 +431,7 @@ extern "C" void dyph_world_destroy(dyph_world* w) {
         if (w->traj_copied[k]) cudaEventDestroy(w->traj_copied[k]);
     }
     if (w->traj_stream) cudaStreamDestroy(w->traj_stream);
-    void* fb[] = {w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw, w->f_counts, w->f_run,
+    void* fb[] = {w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw, w->f_counts, w->f_run, w->s_buf,
                   w->f_words, w->f_pos, w->f_items, w->r_items, w->f_phase, w->a_g, w->a_sets, w->a_seg[0],
                   w->a_seg[1], w->a_flag, w->a_pairs};
     for (void* p : fb)
@@ -456,6 +480,56 @@ extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_strea
 }
 
 namespace {
+dyph_status run_words(dyph_world* w);
+uint32_t fused_smem_need(uint32_t max_nb);
+uint32_t fused_smem_floor(uint32_t max_nb);
+dyph_status fused_smem_prepare();
+
+// A single scene of at most this many bodies steps the frames of a call but the
+// last on one block of the fused kernel, in one launch: a frame is then one
+// block's work instead of a dozen launches that a scene of this size cannot
+// fill. The last frame runs the stage kernels, so the tree, the lists, the
+// colours and the statistics that a program reads after a call are theirs.
+// A frame, one block against the stage kernels: 17 and 66 us on 9 stacked boxes,
+// 113 and 177 on 201, 156 and 181 on 289, 273 and 208 on 433; in the sequential
+// order, whose chains leave a chip idle, 322 and 725 us on 433; 27 and 82 us on a
+// loose pile of 400.
+constexpr uint32_t kSoloBodies = 256, kSoloSequentialBodies = 512;
+
+bool solo_prepare(dyph_world* w) {
+    const uint32_t n = w->desc.bodies.n;
+    const uint32_t most = w->sv->mode == DYPH_SOLVER_SEQUENTIAL ? kSoloSequentialBodies : kSoloBodies;
+    if (w->fused || w->bp->n_scenes != 0u || n > most || w->s_off || w->traj_host) return false;
+    if (w->s_buf) return true;
+    // no more pairs than there are, so that the slots stay small whatever the capacities
+    const uint32_t pairs = std::min(w->bp->max_pairs, n * (n - 1u) / 2u), contacts = std::min(w->np->max_contacts, pairs);
+    const size_t words = kSoloHead + pairs + static_cast<size_t>(kSceneWords) * (contacts + 1u);
+    const uint32_t head[kSoloHead] = {0u, n, 0u, pairs, 0u, contacts, 0u, 0u, 0u, kItemBlock, kItemEmpty, kItemEmpty};
+    w->s_off = true;
+    if (fused_smem_prepare() != DYPH_OK || run_words(w) != DYPH_OK ||
+        cudaMalloc(&w->s_buf, words * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    w->s_off = false;
+    w->s_pairs = pairs;
+    w->s_contacts = contacts;
+    w->s_smem = fused_smem_need(n);
+    return true;
+}
+
+// The frames of a solo scene before a call's last one.
+dyph_status enqueue_solo(dyph_world* w, cudaStream_t s, uint32_t n_frames) {
+    for (uint32_t done = 0; done < n_frames; done += kMaxRunFrames) {
+        FusedRun r{std::min(n_frames - done, kMaxRunFrames)};
+        r.keep = false;
+        const dyph_status st = launch_run(w, r, s);
+        if (st != DYPH_OK) return st;
+    }
+    return DYPH_OK;
+}
+
 // dyph_world_step; a fused batch also writes checkpoints (dyph_world_rollout).
 dyph_status world_step(dyph_world* w, int32_t n_frames, dyph_stream s, float* ckpt = nullptr, uint32_t ckpt_every = 1) {
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
@@ -485,8 +559,16 @@ dyph_status world_step(dyph_world* w, int32_t n_frames, dyph_stream s, float* ck
                 w->graph = nullptr;
                 return DYPH_ERR_CUDA;
             }
+            w->graph_mode = w->sv->mode;
         }
-        for (int32_t f = 0; f < n_frames; ++f) {
+        int32_t f = 0;
+        if (n_frames > 1 && solo_prepare(w)) {
+            const dyph_status st = enqueue_solo(w, w->stream, static_cast<uint32_t>(n_frames - 1));
+            if (st != DYPH_OK) return st;
+            f = n_frames - 1;
+            w->traj_frame += static_cast<uint64_t>(f);
+        }
+        for (; f < n_frames; ++f) {
             DYPH_CUDA_TRY(cudaGraphLaunch(w->graph, w->stream));
             if (trajectory_frame(w, w->traj_frame)) {
                 last = w->traj_frame / w->traj_every;
@@ -519,6 +601,7 @@ extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frame
         cudaGraphExecDestroy(w->episode);
         w->episode = nullptr;
     }
+    const bool solo = probe_stage < 0 && n_frames > 1 && solo_prepare(w);
     cudaGraph_t g = nullptr;
     DYPH_CUDA_TRY(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
     dyph_status st = DYPH_OK;
@@ -529,7 +612,15 @@ extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frame
         st = enqueue_run(w, w->stream, 0, static_cast<uint32_t>(n_frames), chunk, live);
         last = chunk - 1;
     } else {
-        for (int32_t f = 0; f < n_frames && st == DYPH_OK; ++f) {
+        int32_t f0 = 0;
+        if (solo) {
+            const dyph_solver_mode mode = w->graph_mode;
+            w->graph_mode = w->sv->mode;
+            st = enqueue_solo(w, w->stream, static_cast<uint32_t>(n_frames - 1));
+            w->graph_mode = mode;
+            f0 = n_frames - 1;
+        }
+        for (int32_t f = f0; f < n_frames && st == DYPH_OK; ++f) {
             // a probed fused frame is a launch of its own between the events
             st = enqueue_frame(w, w->stream, probe_stage, probe_stage >= 0 ? ev_start[f] : nullptr,
                                probe_stage >= 0 ? ev_end[f] : nullptr);
