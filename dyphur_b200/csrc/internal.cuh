@@ -71,6 +71,8 @@ struct dyph_narrowphase {
     uint32_t* status = nullptr;   // look-back status per 256-pair tile
     uint32_t status_words = 0;    // words cleared before a run
     uint32_t max_pairs_seen = 0;  // status capacity in tiles * 256
+    float4* packed = nullptr;     // [3 packed_n] bodies as the pair test reads them (see pack_bodies_kernel)
+    uint32_t packed_n = 0;
 };
 
 struct dyph_xpbd {
@@ -126,6 +128,8 @@ dyph_status narrowphase_create(uint32_t max_contacts, dyph_narrowphase** out);
 void narrowphase_destroy(dyph_narrowphase* np);
 // Size the tile-status buffer for up to max_pairs pairs (allocates; call outside graph capture).
 dyph_status narrowphase_reserve(dyph_narrowphase* np, uint32_t max_pairs);
+// Room for the packed bodies of scenes that use them (allocates; call outside graph capture).
+dyph_status narrowphase_reserve_bodies(dyph_narrowphase* np, uint32_t n);
 dyph_status narrowphase_run(dyph_narrowphase* np, const dyph_pair* pairs, const uint32_t* d_n_pairs,
                             uint32_t max_pairs, const dyph_bodies* bodies, const dyph_shapes* shapes,
                             cudaStream_t s);

@@ -461,6 +461,7 @@ extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_strea
     dyph_status st = broadphase_create(desc->bodies.n, desc->max_pairs, &w->bp);
     if (st == DYPH_OK) st = narrowphase_create(desc->max_contacts, &w->np);
     if (st == DYPH_OK) st = narrowphase_reserve(w->np, desc->max_pairs);
+    if (st == DYPH_OK) st = narrowphase_reserve_bodies(w->np, desc->bodies.n);
     if (st == DYPH_OK) st = xpbd_create(desc->n_iters, desc->max_contacts, desc->bodies.n, desc->friction, &w->sv);
     if (st == DYPH_OK) {
         w->sv->mode = desc->mode;
