@@ -89,8 +89,7 @@ struct dyph_xpbd {
     uint64_t* bmask = nullptr;      // [max_bodies] JP used-colour masks
     uint32_t* blast = nullptr;      // [max_bodies] last contact seen per body (sequential path)
     uint32_t* meta = nullptr;       // solver control words (see solver.cu)
-    uint64_t* body_list = nullptr;  // [64 max_bodies] dataflow path: (key, entry) lists of each body
-    uint32_t* slot = nullptr;       // [2 max_contacts] dataflow path: list slot of each entry
+    uint32_t* body_list = nullptr;  // [2][64 max_bodies] dataflow path: each body's entries, and by colour
     uint32_t* link = nullptr;       // [2 max_contacts] dataflow path: list predecessor of each entry
     uint64_t* cmask = nullptr;      // [2 max_contacts] dataflow path: published colour masks
     uint64_t* hand = nullptr;       // [2 max_contacts][16] dataflow path: tagged body-state records

@@ -200,8 +200,7 @@ dyph_status xpbd_create(int32_t n_iters, uint32_t max_contacts, uint32_t max_bod
               cudaMalloc(&sv->done, mc * 4) == cudaSuccess && cudaMalloc(&sv->bpri, 3 * mb * 8) == cudaSuccess &&
               cudaMalloc(&sv->bmask, mb * 8) == cudaSuccess && cudaMalloc(&sv->blast, 2 * (mb + 1) * 4) == cudaSuccess &&
               cudaMalloc(&sv->meta, kMetaWords * 4) == cudaSuccess &&
-              cudaMalloc(&sv->body_list, mb * kBodySlots * 8) == cudaSuccess &&
-              cudaMalloc(&sv->slot, 2 * mc * 4) == cudaSuccess &&
+              cudaMalloc(&sv->body_list, 2 * mb * kBodySlots * 4) == cudaSuccess &&
               cudaMalloc(&sv->link, 2 * mc * 4) == cudaSuccess && cudaMalloc(&sv->cmask, 2 * mc * 8) == cudaSuccess &&
               cudaMalloc(&sv->hand, 2 * mc * kHandWords * 8) == cudaSuccess &&
               cudaMemset(sv->hand, 0, 2 * mc * kHandWords * 8) == cudaSuccess &&
@@ -223,7 +222,7 @@ dyph_status xpbd_create(int32_t n_iters, uint32_t max_contacts, uint32_t max_bod
 void xpbd_destroy(dyph_xpbd* sv) {
     if (!sv) return;
     void* ptrs[] = {sv->lambda, sv->color, sv->order, sv->pred, sv->done, sv->bpri, sv->bmask, sv->blast, sv->meta,
-                    sv->body_list, sv->slot, sv->link, sv->cmask, sv->hand, sv->tail, sv->sweep_tag,
+                    sv->body_list, sv->link, sv->cmask, sv->hand, sv->tail, sv->sweep_tag,
                     sv->csr_off, sv->csr_cur, sv->csr, sv->partial, sv->scene_range, sv->scene_order,
                     sv->scene_scratch};
     for (void* p : ptrs)
@@ -278,7 +277,7 @@ dyph_status xpbd_set_scenes(dyph_xpbd* sv, uint32_t n_scenes, const uint32_t* h_
     void** unused[] = {reinterpret_cast<void**>(&sv->order), reinterpret_cast<void**>(&sv->pred),
                        reinterpret_cast<void**>(&sv->done), reinterpret_cast<void**>(&sv->bpri),
                        reinterpret_cast<void**>(&sv->bmask), reinterpret_cast<void**>(&sv->blast),
-                       reinterpret_cast<void**>(&sv->body_list), reinterpret_cast<void**>(&sv->slot),
+                       reinterpret_cast<void**>(&sv->body_list),
                        reinterpret_cast<void**>(&sv->link), reinterpret_cast<void**>(&sv->cmask),
                        reinterpret_cast<void**>(&sv->hand), reinterpret_cast<void**>(&sv->tail),
                        reinterpret_cast<void**>(&sv->csr_off), reinterpret_cast<void**>(&sv->csr_cur),
@@ -320,7 +319,8 @@ dyph_status xpbd_solve(dyph_xpbd* sv, const dyph_contacts* contacts, const dyph_
     }
     // Per-body contact counts live in `blast`, JP rounds in `order`: the
     // kernels that also use them run only after this one declined the frame.
-    FlowBufs F{sv->blast, reinterpret_cast<unsigned long long*>(sv->body_list), sv->slot, sv->link,
+    FlowBufs F{sv->blast, sv->body_list, sv->body_list + static_cast<size_t>(sv->max_bodies) * kBodySlots,
+               reinterpret_cast<unsigned long long*>(sv->bmask), sv->link,
                reinterpret_cast<unsigned long long*>(sv->cmask), sv->order,
                reinterpret_cast<unsigned long long*>(sv->hand), 2u * sv->max_contacts, sv->tail, sv->sweep_tag,
                sv->csr_off, sv->csr_cur, sv->csr, sv->partial};
