@@ -97,27 +97,21 @@ __global__ void __launch_bounds__(kBuildThreads) build_kernel(GlobalBodies B, Gl
     s_delta[threadIdx.x + 1] = boundary_delta(codes, codes64, si, k, n);
     if (threadIdx.x == 0) s_delta[0] = boundary_delta(codes, codes64, si, k0 - 1, n);
     uint4 box = make_uint4(0u, 0u, 0u, 0u);
-    uint32_t big = 0u;
+    uint32_t big = 0u, body = 0u;
     int l = k, r = k;
     bool open = k < n;  // this thread carries a subtree [l, r] that has no parent yet
     if (open) {
-        const uint32_t body = si[k];
-        T.sorted_keys[k] = key64(codes, codes64, si, k);
-        T.inv_sorted[body] = static_cast<uint32_t>(k);
+        body = si[k];
         const uint32_t sh = B.shape(body);
         box = leaf_box(S.type(sh), B.px(body), B.py(body), B.pz(body), B.qw(body), B.qx(body), B.qy(body),
                        B.qz(body), S.hx(sh), S.hy(sh), S.hz(sh));
-        T.aabb[n - 1 + k] = box;
         // Static bodies (grounds, walls) are "large" to the tree walks: pairs with
         // them are found from the other body's side, so no thread walks the whole tree.
         big = B.im(body) == 0.f ? 1u : 0u;
-        T.big[n - 1 + k] = big;
-        if (k == 0) {
-            T.parent[0] = -1;
-            T.root[0] = 0;
-        }
         if (n == 1) open = false;
     }
+    const uint4 own_box = box;
+    const uint32_t own_big = big;
     __syncthreads();
     auto delta = [&](int i) {
         return i >= k0 - 1 && i < k1 ? s_delta[i - k0 + 1] : boundary_delta(codes, codes64, si, i, n);
@@ -165,6 +159,17 @@ __global__ void __launch_bounds__(kBuildThreads) build_kernel(GlobalBodies B, Gl
             make_uint4(static_cast<uint32_t>(r), static_cast<uint32_t>(node_index(l, r)), 0u, 0u);
     }
     __syncthreads();
+    // (global writes wait until here: a fence above would wait for them)
+    if (k < n) {
+        T.sorted_keys[k] = key64(codes, codes64, si, k);
+        T.inv_sorted[body] = static_cast<uint32_t>(k);
+        T.aabb[n - 1 + k] = own_box;
+        T.big[n - 1 + k] = own_big;
+        if (k == 0) {
+            T.parent[0] = -1;
+            T.root[0] = 0;
+        }
+    }
     if (s_flag[threadIdx.x] == 2u) {
         const uint4 a = s_child[0][threadIdx.x], b = s_child[1][threadIdx.x];
         write_node(k, static_cast<int>(a.w & 0x7FFFFFFFu), static_cast<int>(b.x), static_cast<int>(b.y),
@@ -508,24 +513,23 @@ __global__ void __launch_bounds__(kBpThreads) pair_subtree_kernel(uint32_t n_u, 
 }
 
 // Pass 1 for a single scene of at most kTiledBodies bodies, one warp per tile of
-// 32 leaves in Morton order and part of the tiles before it: tile boxes are
-// tested 32 at a time, and of two tiles that meet the leaves that meet the other's
-// box, a lane holding one and meeting the other tile's as broadcasts (see
-// pair_overlap). Wide leaves are kept out of the tiles and meet every leaf. Every
+// 32 leaves in Morton order and part of the tiles before it: a lane holds a leaf
+// and meets 32 tile boxes as broadcasts (see pair_overlap), then the leaves of
+// each tile that some lane's leaf met. Wide leaves are kept out of the tiles and meet every leaf. Every
 // overlapping pair is found once, from its later leaf (or from the leaf that is
 // not wide), and goes to the bucket of its smaller body index. The tests are
 // dense and independent, where a walk of the tree per leaf waits for a node per
 // step in divergent lanes; but tiles that straddle distant parts of the Morton
 // order meet more tiles the more there are. Whole broadphase, tiles against tree
-// walks: 83 and 116 us at 2,000 bodies of a pile, 146 and 198 at 10,000, 197 and
-// 275 at 32,000, 352 and 326 at 48,000.
+// walks: 52 and 67 us at 500 bodies of a pile, 89 and 122 at 2,000, 142 and 198 at
+// 10,000, 209 and 274 at 32,000, 343 and 320 at 48,000.
 // A NaN bound overlaps everything it is compared with, and a tree walk meets it
 // only below ancestors that overlap: with one in the scene every leaf walks.
 constexpr uint32_t kTiledBodies = 32768;
 constexpr int kTileWarps = kBpThreads / 32;
 __global__ void __launch_bounds__(kBpThreads) pair_tiles_kernel(uint32_t n_u, BvhBuffers T, uint32_t parts,
                                                                 const uint32_t* __restrict__ counts) {
-    __shared__ uint4 s_box[kTileWarps][32];
+    __shared__ uint4 s_box[kTileWarps][32], s_tile[kTileWarps][32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t tiles = (n_u + 31u) >> 5;
     const uint32_t item = blockIdx.x * kTileWarps + warp;
@@ -558,27 +562,54 @@ __global__ void __launch_bounds__(kBpThreads) pair_tiles_kernel(uint32_t n_u, Bv
         for (; w; w &= w - 1u) bucket_pair(T, me, other[__ffs(static_cast<int>(w)) - 1].w & ~kWideBit);
     };
     const uint3 tq = facing_box(__ldg(&T.tile_box[tile]));
+    uint4* const boxes = s_tile[warp];
     for (uint32_t t0 = part; t0 <= tile; t0 += 32u * parts) {  // every parts-th tile, 32 at a time
+        // which of the 32 tiles' boxes this lane's leaf meets; a tile of leaves that
+        // lie apart has a box that meets many tiles its leaves do not
         const uint32_t t = t0 + lane * parts;
-        const bool meets = t <= tile && pair_overlap(__ldg(&T.tile_box[min(t, tile)]), tq);
-        for (unsigned hits = __ballot_sync(0xffffffffu, meets); hits; hits &= hits - 1u) {
-            const uint32_t u = t0 + (static_cast<uint32_t>(__ffs(static_cast<int>(hits))) - 1u) * parts;
-            // the leaves of each that meet the other's box: a tile whose leaves lie
-            // apart has a box that meets many tiles its leaves do not
-            const uint4 ub = __ldg(&T.tile_box[u]), o = __ldg(&T.leaf_box[32u * u + lane]);
-            const bool near = i_am && !wide && pair_overlap(ub, q);
-            if (!__any_sync(0xffffffffu, near)) continue;
-            unsigned others = __ballot_sync(0xffffffffu, (o.w & kWideBit) == 0u && pair_overlap(o, tq));
+        __syncwarp();
+        boxes[lane] = t <= tile ? __ldg(&T.tile_box[t]) : make_uint4(0x7C007C00u, 0x7C007C00u, 0x7C007C00u, 0u);
+        __syncwarp();
+        uint32_t near = 0;
+#pragma unroll 8
+        for (uint32_t j = 0; j < 32u; ++j) near |= pair_overlap(boxes[j], q) ? 1u << j : 0u;
+        const uint32_t there = (tile - t0) / parts;  // tiles of the 32 past the first
+        if (there < 31u) near &= (2u << there) - 1u;
+        if (!i_am || wide) near = 0u;
+        uint32_t hits = __reduce_or_sync(0xffffffffu, near);
+        uint4 o = make_uint4(0u, 0u, 0u, 0u);
+        if (hits) o = __ldg(&T.leaf_box[32u * (t0 + (__ffs(static_cast<int>(hits)) - 1) * parts) + lane]);
+        while (hits) {
+            const uint32_t bit = static_cast<uint32_t>(__ffs(static_cast<int>(hits))) - 1u, u = t0 + bit * parts;
+            hits &= hits - 1u;
+            const uint4 cur = o;
+            if (hits)  // the next tile's leaves, while this one's are tested
+                o = __ldg(&T.leaf_box[32u * (t0 + (__ffs(static_cast<int>(hits)) - 1) * parts) + lane]);
+            const bool mine_near = (near >> bit) & 1u, theirs = (cur.w & kWideBit) == 0u;
+            unsigned others = __ballot_sync(0xffffffffu, theirs && pair_overlap(cur, tq));
+            const unsigned nears = __ballot_sync(0xffffffffu, mine_near);
             if (!others) continue;
             __syncwarp();
-            other[lane] = o;
-            __syncwarp();
+            other[lane] = cur;
             uint32_t w = 0;
-            for (; others; others &= others - 1u) {
-                const uint32_t j = static_cast<uint32_t>(__ffs(static_cast<int>(others))) - 1u;
-                w |= pair_overlap(other[j], q) ? 1u << j : 0u;
+            if (__popc(nears) < __popc(others)) {
+                // few leaves here: each met by the 32 there at once
+                for (unsigned m = nears; m; m &= m - 1u) {
+                    const int src = __ffs(static_cast<int>(m)) - 1;
+                    const uint3 sq = make_uint3(__shfl_sync(0xffffffffu, q.x, src), __shfl_sync(0xffffffffu, q.y, src),
+                                                __shfl_sync(0xffffffffu, q.z, src));
+                    const unsigned met = __ballot_sync(0xffffffffu, theirs && pair_overlap(cur, sq));
+                    if (static_cast<int>(lane) == src) w = met;
+                }
+                __syncwarp();
+            } else {
+                __syncwarp();
+                for (; others; others &= others - 1u) {
+                    const uint32_t j = static_cast<uint32_t>(__ffs(static_cast<int>(others))) - 1u;
+                    w |= pair_overlap(other[j], q) ? 1u << j : 0u;
+                }
+                if (!mine_near) w = 0u;
             }
-            if (!near) w = 0u;
             if (u == tile) w &= (1u << lane) - 1u;  // earlier leaves only
             emit(w);
         }

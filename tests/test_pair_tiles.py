@@ -76,3 +76,14 @@ def test_non_finite_bodies(oracle_mod, value):
     s = _cloud(200, "plain", 9)
     s.pos[[5, 77], [0, 2]] = value
     _compare(oracle_mod, s, tree=False)
+
+
+@pytest.mark.parametrize("n", [20, 70, 300])
+def test_unbounded_bodies(oracle_mod, n):
+    """Half extents past fp16: boxes without bounds overlap every other one."""
+    s = _cloud(n, "plain", 4)
+    s.shape_half = np.concatenate([s.shape_half, np.full((1, 3), 1e6, np.float32)])
+    s.shape_type = np.append(s.shape_type, np.uint32(0))
+    s.shape_offset = np.array([0, len(s.shape_type)], np.uint32)
+    s.shape[[0, n // 2]] = len(s.shape_type) - 1
+    _compare(oracle_mod, s, tree=False)
