@@ -12,11 +12,14 @@
 //
 // The ray walk keeps the reference's visiting order (a 64-entry stack, right
 // child pushed before left, node box tested when popped) and its float
-// expressions, so hits and tie-breaks are identical, not just close.
+// expressions, so hits and tie-breaks are identical, not just close. In trees of
+// some size it finds a bound on the hit first and then follows that order only
+// among the leaves that can matter (ray_walk_kernel).
 #include <algorithm>
+#include <mutex>
 #include <new>
 
-#include "common.cuh"
+#include "physics.cuh"
 
 namespace dyph {
 namespace {
@@ -24,14 +27,15 @@ namespace {
 constexpr int kRayThreads = 128;
 constexpr int kRayStack = 64;  // ray_query.cpp:173
 
-// Slab test against a node box (ray_query.cpp:14-33).
+// Slab test against a node box (ray_query.cpp:14-33); tmin is where the ray
+// enters it.
 __device__ __forceinline__ bool ray_node_hit(float ox, float oy, float oz, float ix, float iy, float iz,
                                              float mnx, float mny, float mnz, float mxx, float mxy, float mxz,
-                                             float best_t) {
+                                             float best_t, float& tmin) {
     const float t1x = (mnx - ox) * ix, t2x = (mxx - ox) * ix;
     const float t1y = (mny - oy) * iy, t2y = (mxy - oy) * iy;
     const float t1z = (mnz - oz) * iz, t2z = (mxz - oz) * iz;
-    float tmin = t1x < t2x ? t1x : t2x;
+    tmin = t1x < t2x ? t1x : t2x;
     float tmax = t1x < t2x ? t2x : t1x;
     const float ylo = t1y < t2y ? t1y : t2y, yhi = t1y < t2y ? t2y : t1y;
     tmin = tmin > ylo ? tmin : ylo;
@@ -118,6 +122,14 @@ __device__ __forceinline__ void ray_leaf(const RayScene& S, uint32_t bi, const d
     }
 }
 
+// The slab test against the six fp16 bounds of a NodeBox.
+__device__ __forceinline__ bool ray_box_hit(const dyph_ray& r, float ix, float iy, float iz, const uint4& nb,
+                                            float best_t, float& tmin) {
+    return ray_node_hit(r.ox, r.oy, r.oz, ix, iy, iz, h2f_bits(nb.x & 0xFFFFu), h2f_bits(nb.x >> 16),
+                        h2f_bits(nb.y & 0xFFFFu), h2f_bits(nb.y >> 16), h2f_bits(nb.z & 0xFFFFu),
+                        h2f_bits(nb.z >> 16), best_t, tmin);
+}
+
 __global__ void __launch_bounds__(kRayThreads) ray_query_kernel(dyph_bvh_view bvh, RayScene S,
                                                                 const dyph_ray* __restrict__ rays,
                                                                 dyph_ray_hit* __restrict__ hits, uint32_t n_rays) {
@@ -138,11 +150,8 @@ __global__ void __launch_bounds__(kRayThreads) ray_query_kernel(dyph_bvh_view bv
         const uint4* boxes = reinterpret_cast<const uint4*>(bvh.aabb);
         while (top > 0) {
             const int32_t node = stack[--top];
-            const uint4 nb = __ldg(&boxes[node]);
-            if (!ray_node_hit(r.ox, r.oy, r.oz, ix, iy, iz, h2f_bits(nb.x & 0xFFFFu), h2f_bits(nb.x >> 16),
-                              h2f_bits(nb.y & 0xFFFFu), h2f_bits(nb.y >> 16), h2f_bits(nb.z & 0xFFFFu),
-                              h2f_bits(nb.z >> 16), best_t))
-                continue;
+            float tmin;
+            if (!ray_box_hit(r, ix, iy, iz, __ldg(&boxes[node]), best_t, tmin)) continue;
             if (node >= n_int) {
                 ray_leaf(S, __ldg(&bvh.sorted_idx[node - n_int]), r, best_t, best_body);
             } else if (top + 1 < kRayStack) {
@@ -152,6 +161,378 @@ __global__ void __launch_bounds__(kRayThreads) ray_query_kernel(dyph_bvh_view bv
         }
     }
     hits[idx] = dyph_ray_hit{best_t, best_body};
+}
+
+// ── the closest hit first ────────────────────────────────────────────────────
+// The reference's walk visits the tree in leaf order and so passes most of a
+// long ray's leaves before the near ones. Its result is a fold over the leaves
+// in that order, best = t_max at first: leaf k is taken when its box test passes
+// with an entry point m_k < best (its ancestors' tests then pass too: their boxes
+// contain its box exactly and every operation of the slab test is monotone), and
+// then best = t_k if t_k < best. For any leaf best ends at or below
+// max(t_k, m_k), so a walk that goes to the nearer child first finds a bound U on
+// the result quickly. With W >= U such that t_k <= W implies m_k <= W, leaves
+// with t_k > W do not change the result: while best > W a leaf with t_k <= W is
+// always taken, and afterwards t_k > W >= best is not. A second walk, in leaf
+// order, therefore folds only the leaves with t_k <= W; it starts at W = U and
+// begins again with W = m_k in the rare case that it meets one past W (the boxes
+// are rounded to fp16 and may cut a body).
+// The second walk needs a lower bound on t_k <= W at every node: the entry point
+// into the node's box widened so far that it holds every point o + t_k d that the
+// leaf tests can return. Such a point is at most L = W |d| from the origin o. The
+// box test's lies within 5e-5 (L + size) of the body's box (rounding of rotation
+// and slabs, quaternions within 1e-5 of unit length), the sphere test's within
+// min(sqrt(20 eps) (L + 2 r), 10 eps (L + 2 r)^2 / r) of the sphere (the quadratic's
+// cancellation). A leaf box holds its body's to within fp16 rounding, 2^-11 of
+// each bound, and within the body's movement since the tree was built (a solve
+// moves bodies). So each bound is widened by 5e-4 of itself and by the largest
+// movement, with the terms in the bodies' sizes, over all leaves, found with the
+// records, + 1e-4 L + min(2.5e-3 L, 1.5e-6 L^2 / the smallest sphere's radius).
+// A body beyond fp16's range, as a pile that bursts throws out, has a leaf box
+// that starts at +infinity or ends at -infinity on some axis: its entry point is
+// infinite or behind the ray, so no ray with a finite t_max ever tests it.
+// Rays with a zero or non-finite component, trees or bodies outside these
+// assumptions, folds of more than kRayFoldSteps nodes (margins far beyond the
+// leaves' sizes) and walks that reach the reference's stack limit take the
+// reference's walk as it is (in_order).
+//
+// Records of the tree and its bodies, 16-byte words:
+//   nodes  two per internal node, one sector: the left child's box and index,
+//          the right child's box and index;
+//   leaves four per leaf, in leaf order: position and body, rotation, half
+//          extents and shape type, leaf box.
+struct RayRecords {
+    uint4* nodes;
+    uint4* leaves;
+    // [0] largest excess (float bits), [1] 1 when the tree or a body is outside the
+    // assumptions, [2] complement of the smallest sphere radius's bits (0: no sphere),
+    // [3] leaf boxes out of every finite ray's reach
+    uint32_t* words;
+};
+
+// A tree of fewer bodies is walked as it is. The walk in leaf order and this one:
+// 900 and 252 us for 64 rays at random into a pile of 65,537 bodies, 1,478 and 526
+// for 131,072, 6,364 and 2,676 for a million; 2,790 and 2,730 for a million at
+// 16,385 bodies, 1,852 and 2,474 at 8,193. A million camera rays: 715 and 621 us
+// at 65,537, 464 and 439 at 16,385.
+constexpr uint32_t kRayRecordsBodies = 16384;
+// Nodes that a ray visits in leaf order before it looks for a bound first. Leaf
+// order is Morton order, which ascends in every coordinate: the more a ray does,
+// the nearer it comes to meeting the near leaves first anyway.
+__device__ __forceinline__ uint32_t ray_steps(const dyph_ray& r) {
+    const float s = (r.dx + r.dy + r.dz) / (fabsf(r.dx) + fabsf(r.dy) + fabsf(r.dz));
+    return s > 0.25f ? 384u : (s > -0.25f ? 96u : 24u);
+}
+
+// The node index and the height of the reference's stack share a stack word.
+constexpr uint32_t kRayNodeBits = 26;
+constexpr uint32_t kRayMaxBodies = 1u << (kRayNodeBits - 1);  // nodes 0 .. 2 n - 2
+constexpr uint32_t kRayNone = 0xFFFFFFFFu, kRayNodeMask = (1u << kRayNodeBits) - 1u;
+
+// A ray past far bodies has a margin that grows with its length. A million rays
+// into a pile that has thrown 10 % of its bodies 100 to 1e10 away: 8.6 ms with
+// 128 steps, 7.8 with 512, 9.4 with 4096 (8.5 in leaf order alone).
+constexpr uint32_t kRayFoldSteps = 512;
+
+// A bound v moved by c of its magnitude (an infinite one stays). The margins are
+// taken with fp16's 2^-11 and a little more, the fold's boxes with more still,
+// which covers the rounding of far bodies' bounds.
+constexpr float kRayHalf = 4.95e-4f, kRayWide = 5e-4f;
+__device__ __forceinline__ float widen(float v, float c) { return v + c * fminf(fabsf(v), 1e5f); }
+// Whether the box test never passes for a finite t_max, whatever the direction.
+__device__ __forceinline__ bool out_of_reach(const BoxF& f) {
+    return fmaxf(fmaxf(f.mnx, f.mny), f.mnz) == INFINITY || fminf(fminf(f.mxx, f.mxy), f.mxz) == -INFINITY;
+}
+
+__device__ __forceinline__ bool box_holds(const BoxF& a, const BoxF& b) {
+    return a.mnx <= b.mnx && a.mny <= b.mny && a.mnz <= b.mnz && a.mxx >= b.mxx && a.mxy >= b.mxy && a.mxz >= b.mxz;
+}
+
+__global__ void __launch_bounds__(256) ray_records_kernel(dyph_bvh_view bvh, RayScene S, RayRecords R) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint4* boxes = reinterpret_cast<const uint4*>(bvh.aabb);
+    float excess = 0.f;
+    uint32_t small = 0u;
+    bool odd = false, away = false;
+    if (i < bvh.n) {
+        if (i + 1u < bvh.n) {
+            const int32_t l = bvh.left[i], r = bvh.right[i];
+            uint4 lb = boxes[l], rb = boxes[r];
+            const BoxF own = unpack_box(boxes[i]);
+            odd = !box_holds(own, unpack_box(lb)) || !box_holds(own, unpack_box(rb));
+            lb.w = static_cast<uint32_t>(l);
+            rb.w = static_cast<uint32_t>(r);
+            R.nodes[2ull * i] = lb;
+            R.nodes[2ull * i + 1] = rb;
+        }
+        const uint32_t b = bvh.sorted_idx[i], sh = S.b.shape[b], type = S.sh.type[sh];
+        const uint4 box = boxes[bvh.n - 1u + i];
+        auto bits = [](float x) { return __float_as_uint(x); };
+        const float px = S.b.pos_x[b], py = S.b.pos_y[b], pz = S.b.pos_z[b];
+        const float qw = S.b.rot_w[b], qx = S.b.rot_x[b], qy = S.b.rot_y[b], qz = S.b.rot_z[b];
+        const float hx = S.sh.half_x[sh], hy = S.sh.half_y[sh], hz = S.sh.half_z[sh];
+        R.leaves[4ull * i] = make_uint4(bits(px), bits(py), bits(pz), b);
+        R.leaves[4ull * i + 1] = make_uint4(bits(qw), bits(qx), bits(qy), bits(qz));
+        R.leaves[4ull * i + 2] = make_uint4(bits(hx), bits(hy), bits(hz), type);
+        R.leaves[4ull * i + 3] = box;
+        const BoxF f = unpack_box(box);
+        odd = odd || isnan(f.mnx) || isnan(f.mny) || isnan(f.mnz) || isnan(f.mxx) || isnan(f.mxy) || isnan(f.mxz);
+        away = !odd && out_of_reach(f);
+        if (!away) {
+            // how far the body's present box leaves its leaf box
+            float ex = hx, ey = hx, ez = hx;
+            if (type != kShapeSphere) {
+                ex = fabsf(1.f - 2.f * (qy * qy + qz * qz)) * hx + fabsf(2.f * (qx * qy - qz * qw)) * hy +
+                     fabsf(2.f * (qx * qz + qy * qw)) * hz;
+                ey = fabsf(2.f * (qx * qy + qz * qw)) * hx + fabsf(1.f - 2.f * (qx * qx + qz * qz)) * hy +
+                     fabsf(2.f * (qy * qz - qx * qw)) * hz;
+                ez = fabsf(2.f * (qx * qz - qy * qw)) * hx + fabsf(2.f * (qy * qz + qx * qw)) * hy +
+                     fabsf(1.f - 2.f * (qx * qx + qy * qy)) * hz;
+                const float q2 = qw * qw + qx * qx + qy * qy + qz * qz;
+                odd = odd || !(fabsf(q2 - 1.f) <= 1e-5f) || !(hy >= 0.f) || !(hz >= 0.f);
+            }
+            const float over = fmaxf(
+                fmaxf(fmaxf(widen(f.mnx, -kRayHalf) - (px - ex), (px + ex) - widen(f.mxx, kRayHalf)),
+                      fmaxf(widen(f.mny, -kRayHalf) - (py - ey), (py + ey) - widen(f.mxy, kRayHalf))),
+                fmaxf(widen(f.mnz, -kRayHalf) - (pz - ez), (pz + ez) - widen(f.mxz, kRayHalf)));
+            // the sums above round: 1e-5 of the extents and of the excess, and of the
+            // bounds what kRayWide leaves; and the leaf tests' terms in the size
+            const float size = type == kShapeSphere ? 5e-3f * hx : 1e-4f * (hx + hy + hz);
+            excess = 1.00001f * fmaxf(over, 0.f) + 1e-5f * (ex + ey + ez) + size + 1e-6f;
+            if (type == kShapeSphere) small = ~bits(fabsf(hx));
+            odd = odd || !(hx >= 0.f) || !isfinite(fabsf(px) + fabsf(py) + fabsf(pz) + ex + ey + ez) ||
+                  !(excess < 1e6f);
+        }
+    }
+    const uint32_t e = __reduce_max_sync(0xffffffffu, odd ? 0u : __float_as_uint(excess));
+    const bool any_odd = __any_sync(0xffffffffu, odd);
+    const uint32_t n_away = __popc(__ballot_sync(0xffffffffu, away));
+    small = __reduce_max_sync(0xffffffffu, small);
+    if ((threadIdx.x & 31u) == 0u) {
+        if (small) atomicMax(&R.words[2], small);
+        if (e) atomicMax(&R.words[0], e);
+        if (any_odd) R.words[1] = 1u;
+        if (n_away) atomicAdd(&R.words[3], n_away);
+    }
+}
+
+// One ray's walks over the records.
+struct RayWalk {
+    const dyph_bvh_view& bvh;
+    const RayRecords& R;
+    const dyph_ray& r;
+    float ix, iy, iz;
+    uint2* stack;  // [kRayStack] node | height << kRayNodeBits (of the reference's stack under the node), entry point
+    float best_t;
+    uint32_t best_body;
+    bool deep;  // met the reference's stack limit, or the fold's own
+
+    __device__ __forceinline__ bool box(const uint4& b, float best, float& tmin) const {
+        return ray_box_hit(r, ix, iy, iz, b, best, tmin);
+    }
+    // t of a leaf if it is below `best`, else negative
+    __device__ __forceinline__ float leaf(const uint4* l, float best, uint32_t& body) const {
+        const uint4 p = __ldg(l), q = __ldg(l + 1), h = __ldg(l + 2);
+        auto f = [](uint32_t x) { return __uint_as_float(x); };
+        body = p.w;
+        return h.w == kShapeSphere
+                   ? ray_sphere(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, f(p.x), f(p.y), f(p.z), f(h.x), best)
+                   : ray_box(r.ox, r.oy, r.oz, r.dx, r.dy, r.dz, f(p.x), f(p.y), f(p.z), f(q.x), f(q.y), f(q.z),
+                             f(q.w), f(h.x), f(h.y), f(h.z), best);
+    }
+    // Whether the ray meets box b, widened by m (lo = o + m, hi = o - m), at or
+    // before `most`; tlow: where it enters.
+    __device__ __forceinline__ bool wide_box(const uint4& b, const float lo[3], const float hi[3], float most,
+                                             float& tlow) const {
+        const BoxF f = unpack_box(b);
+        const float t1x = (widen(f.mnx, -kRayWide) - lo[0]) * ix, t2x = (widen(f.mxx, kRayWide) - hi[0]) * ix;
+        const float t1y = (widen(f.mny, -kRayWide) - lo[1]) * iy, t2y = (widen(f.mxy, kRayWide) - hi[1]) * iy;
+        const float t1z = (widen(f.mnz, -kRayWide) - lo[2]) * iz, t2z = (widen(f.mxz, kRayWide) - hi[2]) * iz;
+        tlow = fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fminf(t1z, t2z));
+        const float thigh = fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fmaxf(t1z, t2z));
+        return thigh >= 0.f && thigh >= tlow && tlow <= most;
+    }
+    // A walk from `root`, of two children to the nearer or to the left one first:
+    // test(box, entry) says whether a child is gone into, leaf_fn(leaf, entry) ends
+    // the walk with true, keep(entry) whether a waiting node still is when its turn
+    // comes. False when `steps` nodes did not end it.
+    template <bool kNearFirst, class Test, class Leaf, class Keep>
+    __device__ __forceinline__ bool walk(uint32_t root, float entry, uint32_t steps, Test&& test, Leaf&& leaf_fn,
+                                         Keep&& keep) {
+        const uint32_t n_int = bvh.n - 1u;
+        uint32_t height = 0, node = root;
+        int top = 0;
+        while (true) {
+            if (steps-- == 0u) return false;
+            bool next = true;
+            if (node < n_int) {
+                const uint4 lb = __ldg(&R.nodes[2ull * node]), rb = __ldg(&R.nodes[2ull * node + 1]);
+                float lt, rt;
+                const bool room = height + 1u < static_cast<uint32_t>(kRayStack);
+                deep = deep || !room;
+                const bool lh = test(lb, lt) && room, rh = test(rb, rt) && room;
+                if (lh || rh) {
+                    const bool left = lh && (!kNearFirst || !rh || lt <= rt);
+                    if (lh && rh)
+                        stack[top++] = left ? make_uint2(rb.w | (height << kRayNodeBits), __float_as_uint(rt))
+                                            : make_uint2(lb.w | ((height + 1u) << kRayNodeBits), __float_as_uint(lt));
+                    node = left ? lb.w : rb.w;
+                    entry = left ? lt : rt;
+                    height += left ? 1u : 0u;
+                    next = false;
+                }
+            } else if (leaf_fn(R.leaves + 4ull * (node - n_int), entry)) {
+                return true;
+            }
+            while (next) {
+                if (top == 0) return true;
+                const uint2 e = stack[--top];
+                entry = __uint_as_float(e.y);
+                node = e.x & kRayNodeMask;
+                height = e.x >> kRayNodeBits;
+                next = !keep(entry);
+            }
+        }
+    }
+
+    // The reference's walk (ray_query_kernel), both children tested in one step:
+    // a box test depends on the closest hit so far only through "enters before
+    // it", which is tested again when the node's turn comes. False when it is not
+    // done after `steps` nodes; best_t bounds the result from above then too.
+    __device__ __forceinline__ bool in_order(uint32_t root, uint32_t steps) {
+        best_t = r.t_max;
+        best_body = kRayNone;
+        float tmin;
+        if (!box(__ldg(reinterpret_cast<const uint4*>(bvh.aabb) + root), best_t, tmin)) return true;
+        return walk<false>(
+            root, tmin, steps, [&](const uint4& b, float& t) { return box(b, best_t, t); },
+            [&](const uint4* l, float) {
+                uint32_t body;
+                const float t = leaf(l, best_t, body);
+                if (t >= 0.f) {
+                    best_t = t;
+                    best_body = body;
+                }
+                return false;
+            },
+            [&](float entry) { return entry < best_t; });
+    }
+
+    // A bound on the result that is at most U, nearer children first; U when
+    // nothing below it is hit.
+    __device__ __forceinline__ float bound(uint32_t root, float U) {
+        float tmin;
+        if (!box(__ldg(reinterpret_cast<const uint4*>(bvh.aabb) + root), U, tmin)) return U;
+        walk<true>(
+            root, tmin, ~0u, [&](const uint4& b, float& t) { return box(b, U, t); },
+            [&](const uint4* l, float entry) {
+                uint32_t body;
+                const float t = leaf(l, U, body);
+                if (t >= 0.f) U = fminf(U, fmaxf(t, entry));
+                return false;
+            },
+            [&](float entry) { return entry < U; });
+        return U;
+    }
+
+    // The fold over the leaves with t <= W in leaf order; returns W, or a larger
+    // bound with which to begin again.
+    __device__ __forceinline__ float fold(uint32_t root, float W, float slack, float inv_radius, float length) {
+        const float past = nextafterf(W, INFINITY);  // t < past: t <= W
+        const float L = W * length;
+        const float m = slack + 1e-4f * L + fminf(2.5e-3f * L, 1.5e-6f * L * L * inv_radius);
+        const float lo[3] = {r.ox + m, r.oy + m, r.oz + m}, hi[3] = {r.ox - m, r.oy - m, r.oz - m};
+        float again = W;
+        best_t = r.t_max;
+        best_body = kRayNone;
+        const bool ended = walk<false>(
+            root, 0.f, kRayFoldSteps, [&](const uint4& b, float& t) { return wide_box(b, lo, hi, fminf(W, best_t), t); },
+            [&](const uint4* l, float) {
+                float tmin;
+                if (!box(__ldg(l + 3), INFINITY, tmin)) return false;
+                uint32_t body;
+                const float t = leaf(l, fminf(past, best_t), body);
+                if (!(t >= 0.f)) return false;
+                if (tmin > W && best_t > W) {
+                    again = tmin;
+                    return true;
+                }
+                if (tmin < best_t) {
+                    best_t = t;
+                    best_body = body;
+                }
+                return false;
+            },
+            [&](float entry) { return entry <= fminf(W, best_t); });
+        deep = deep || !ended;
+        return again;
+    }
+};
+
+// One thread per ray: ray_steps nodes of the reference's walk, which end most
+// rays whose leaf order happens to be near first, then the bound and the fold.
+// Bound by the latency of dependent loads in divergent lanes.
+__global__ void __launch_bounds__(kRayThreads) ray_walk_kernel(dyph_bvh_view bvh, RayRecords R,
+                                                               const dyph_ray* __restrict__ rays,
+                                                               dyph_ray_hit* __restrict__ hits, uint32_t n_rays) {
+    const uint32_t idx = blockIdx.x * kRayThreads + threadIdx.x;
+    if (idx >= n_rays) return;
+    const dyph_ray r = rays[idx];
+    const uint32_t root = static_cast<uint32_t>(__ldg(bvh.root));
+    uint2 stack[kRayStack];
+    RayWalk w{bvh, R, r, 1.f / r.dx, 1.f / r.dy, 1.f / r.dz, stack};
+    w.deep = false;
+    const float d2 = r.dx * r.dx + r.dy * r.dy + r.dz * r.dz;
+    const bool plain = R.words[1] != 0u || !isfinite(fabsf(r.ox) + fabsf(r.oy) + fabsf(r.oz)) ||
+                       !isfinite(fabsf(w.ix) + fabsf(w.iy) + fabsf(w.iz)) || !(d2 > 1e-20f && d2 < 1e20f) ||
+                       !(r.t_max > 0.f) || (R.words[3] != 0u && !isfinite(r.t_max));
+    if (!w.in_order(root, plain ? ~0u : ray_steps(r))) {
+        float W = w.bound(root, w.best_t);
+        bool done = !w.deep && W == r.t_max;  // nothing is entered and hit before t_max
+        if (done) {
+            w.best_t = r.t_max;
+            w.best_body = kRayNone;
+        }
+        const float slack = __uint_as_float(R.words[0]), length = __fsqrt_rn(d2);
+        const uint32_t small = R.words[2];
+        const float inv_radius = small ? 1.f / __uint_as_float(~small) : 0.f;
+        for (int k = 0; k < 8 && !done && !w.deep; ++k) {
+            const float W1 = w.fold(root, W, slack, inv_radius, length);
+            done = W1 == W;
+            W = W1;
+        }
+        if (!done || w.deep) w.in_order(root, ~0u);
+    }
+    hits[idx] = dyph_ray_hit{w.best_t, w.best_body};
+}
+
+// Stream-ordered scratch of the queries: a pool of its own per device that
+// keeps at most kRayPoolKeep bytes between calls. Calls on any streams and
+// threads take and return blocks through it.
+constexpr int kRayMaxDevices = 64;
+constexpr uint64_t kRayPoolKeep = 64ull << 20;
+std::mutex g_ray_pool_mu;
+cudaMemPool_t g_ray_pool[kRayMaxDevices] = {};
+
+cudaMemPool_t ray_pool() {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kRayMaxDevices) return nullptr;
+    std::lock_guard<std::mutex> lock(g_ray_pool_mu);
+    if (!g_ray_pool[dev]) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        uint64_t keep = kRayPoolKeep;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+        if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaMemPoolDestroy(pool);
+            return nullptr;
+        }
+        g_ray_pool[dev] = pool;
+    }
+    return g_ray_pool[dev];
 }
 
 // ── contact sensor ──────────────────────────────────────────────────────────
@@ -248,6 +629,28 @@ extern "C" dyph_status dyph_ray_query(const dyph_bvh_view* bvh, const dyph_bodie
         return DYPH_ERR_INVALID;
     if (bvh->n > bodies->n) return DYPH_ERR_INVALID;
     const uint32_t grid = (n_rays + kRayThreads - 1) / kRayThreads;
+    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies) {
+        cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
+        const size_t node_bytes = 32ull * bvh->n, leaf_bytes = 64ull * bvh->n;
+        void* ws = nullptr;
+        cudaMemPool_t pool = ray_pool();
+        if (pool && cudaMallocFromPoolAsync(&ws, node_bytes + leaf_bytes + 16, pool, cs) == cudaSuccess) {
+            char* base = static_cast<char*>(ws);
+            const RayRecords R{reinterpret_cast<uint4*>(base), reinterpret_cast<uint4*>(base + node_bytes),
+                               reinterpret_cast<uint32_t*>(base + node_bytes + leaf_bytes)};
+            cudaError_t e = cudaMemsetAsync(R.words, 0, 16, cs);
+            if (e == cudaSuccess) {
+                ray_records_kernel<<<(bvh->n + 255) / 256, 256, 0, cs>>>(*bvh, RayScene{*bodies, *shapes}, R);
+                ray_walk_kernel<<<grid, kRayThreads, 0, cs>>>(*bvh, R, d_rays, d_hits, n_rays);
+                e = cudaGetLastError();
+            }
+            const cudaError_t fe = cudaFreeAsync(ws, cs);
+            DYPH_CUDA_TRY(e);
+            DYPH_CUDA_TRY(fe);
+            return DYPH_OK;
+        }
+        cudaGetLastError();  // no scratch: the rays walk the view's own arrays
+    }
     ray_query_kernel<<<grid, kRayThreads, 0, reinterpret_cast<cudaStream_t>(s)>>>(*bvh, RayScene{*bodies, *shapes},
                                                                                    d_rays, d_hits, n_rays);
     DYPH_CUDA_TRY(cudaGetLastError());
