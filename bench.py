@@ -323,21 +323,27 @@ def flow_kernel_active(contacts: np.ndarray, mode: int) -> np.ndarray:
     round-synchronous kernel."""
     c = contacts.astype(np.int64)
     seq = (mode == 1) | ((mode == 0) & (c <= 256))
-    return (c > 0) & ~(seq & (c <= 2048)) & (c <= 16 * FLOW_THREADS)
+    return (c > 0) & ~(seq & (c <= 128)) & (c <= 16 * FLOW_THREADS)
 
 
-def kernels_per_frame(n: int, n_scenes: int = 1, fused: bool = False) -> int:
-    """Library kernels one frame launches (matches the ncu launch lists in profiles/)."""
-    if fused:  # the fused frame kernel and the frame's statistics
-        return 2
+def fused_launches(cfg: dict, frames: int, sms: int) -> int:
+    """Library kernels that an episode of fused batched frames launches: the fused kernel and its
+    statistics, once for up to 256 frames when every block is resident at once, else every frame."""
+    resident = cfg["blocks"] <= cfg["blocks_per_sm"] * sms
+    return 2 * (-(-frames // 256) if resident else frames)
+
+
+def kernels_per_frame(n: int, n_scenes: int = 1) -> int:
+    """Library kernels one frame of the stage kernels launches (matches the ncu launch lists in profiles/)."""
     if n_scenes > 1:  # (scene << 30 | code) keys: histogram + one pass per 8 key bits, + scene ranges
         key_bits = 30 + max(1, (n_scenes - 1).bit_length())
         sort = (1 if n <= 4096 else 1 + (key_bits + 7) // 8) + 1
     else:
         sort = 1 if n <= 4096 else 5  # one-block sort, or histogram + 4 onesweep passes
-    # integrate, morton, sort, build, finalize, pair find (two passes), pair write, narrowphase,
-    # solver (dataflow, round-synchronous, sequential: two of them return at once), stats
-    return 1 + 1 + sort + 1 + 1 + 2 + 1 + 1 + 3 + 1
+    # integrate, morton, sort, build, finalize, pair search (tiles, or tree walks in two passes), pair
+    # write, narrowphase, solver (dataflow, round-synchronous, sequential: two of them return at once), stats
+    find = 1 if n_scenes == 1 and n <= 32768 else 2
+    return 1 + 1 + sort + 1 + 1 + find + 1 + 1 + 3 + 1
 
 
 def peaks() -> tuple[float, str]:
@@ -861,8 +867,9 @@ def run_b200(args) -> None:
             "frame_roofline": {"bound": "hbm", "achieved": frame_ach, "peak": peak, "unit": "GB/s",
                                "frac": frame_ach / peak, "peak_source": f"{peak_kind} hbm_gbs",
                                "bytes_rule": "424 B per body + 32 B per candidate pair + 72 B per contact, per frame"},
-            "gpu_launches": int(args.steps * frames * kernels_per_frame(n, scene.n_scenes,
-                                                                       fused=r["fused_config"] is not None)),
+            "gpu_launches": int(args.steps * (
+                fused_launches(r["fused_config"], frames, torch.cuda.get_device_properties(0).multi_processor_count)
+                if r["fused_config"] is not None else frames * kernels_per_frame(n, scene.n_scenes))),
             "fused_config": r["fused_config"], "colored_fused_config": rc["fused_config"],
             "clocks": r["clocks"], "overflow_status": r["status"],
         }

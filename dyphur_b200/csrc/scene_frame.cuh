@@ -452,7 +452,7 @@ __device__ __forceinline__ ItemTeam item_team(const uint32_t* item, uint32_t sme
 // (128 registers a thread), 5 (96) or 6 (80, a few bytes spilled), or 2 of
 // kSceneWideThreads (128). Which one runs best depends on the batch
 // (dyph_world_autotune picks the budget with the shared memory cap; the wide
-// form's rule is in fused_threads); all compute the same frames.
+// form's rule is in setup_fused); all compute the same frames.
 template <int kMinBlocks, int kThreads>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) scene_frame_kernel(SceneBufs S, FrameBufs F, FrameParams P_,
                                                                            const uint32_t* __restrict__ items,

@@ -90,14 +90,14 @@ struct dyph_world {
     // Knobs of the fused kernel (dyph_world_set_fused_config / dyph_world_autotune).
     std::vector<uint32_t> h_body_offset;  // host copy of the scenes' body ranges
     uint32_t f_smem_cap = 0;              // shared memory cap per block (0 = what the largest scene needs)
-    uint32_t f_teams = 2;                 // 0 blocks only, 1 + small scenes one per warp, 2 + mid-size two warps
-    uint32_t f_threads = kSceneThreads;   // threads of a block (fused_threads)
+    uint32_t f_teams = 2;                 // 0 blocks only, 1 + small scenes a quarter, 2 + mid-size half a block
+    uint32_t f_threads = kSceneThreads;   // threads of a block (rule in setup_fused)
     bool f_resident = false;              // all blocks of the batch fit the device at once
     uint32_t f_variant = 0;               // register budget: 4 (0), 5 (1) or 6 (2) blocks per SM
     uint32_t f_warp_scenes = 0, f_half_scenes = 0, f_block_scenes = 0;
     // Work items of the adjoint's reverse kernel, laid out on their own: its
     // levels are long dependent chains with a barrier each, which favours
-    // one-warp teams over the forward frame's choice.
+    // smaller teams than the forward frame's choice.
     uint32_t* r_items = nullptr;
     uint32_t r_n_items = 0, r_smem = 0;
     uint32_t r_smem_cap = 0;              // 0: a third of an SM's shared memory
@@ -759,9 +759,9 @@ uint32_t fused_smem_need(uint32_t max_nb) {
 uint32_t fused_smem_floor(uint32_t max_nb) { return frame_body_bytes(max_nb) + 56u * 64u; }
 
 // Work items, largest scenes first: a scene whose estimated shared-memory
-// need fits a quarter of the block's (`share`) runs on one warp, four such
-// scenes to a block (teams >= 1); one that fits half of it on two warps, two
-// to a block (teams == 2); larger scenes take the whole block.
+// need fits a quarter of the block's (`share`) runs on a quarter of the block,
+// four such scenes to a block (teams >= 1); one that fits half of it on half the
+// block (teams == 2); larger scenes take the whole block.
 template <class Est>
 void build_items(const uint32_t* body_offset, uint32_t n_scenes, uint32_t share, uint32_t teams, Est est,
                  std::vector<uint32_t>& items, uint32_t& n_small, uint32_t& n_mid) {
@@ -964,7 +964,9 @@ dyph_status setup_fused(dyph_world* w, uint32_t n_scenes, const uint32_t* body_o
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, form.kernel, static_cast<int>(form.threads), smem));
         // Blocks of twice the threads where the chip would otherwise hold at most
         // half the warps the registers allow: shared memory for two blocks an SM
-        // at most, or hardly more blocks than SMs.
+        // at most, or at most two blocks per SM in all. A frame with 256 against
+        // 128 threads: 220 and 297 us on 1024 mixed scenes (115 KB a block), 64
+        // and 67 on 256 push scenes, 46 and 50 on 64 stacks.
         if (w->f_variant == 0 && (per_sm <= 2 || w->f_n_items <= 2u * static_cast<uint32_t>(sms))) {
             w->f_threads = kSceneWideThreads;
             form = fused_form(w);

@@ -544,7 +544,7 @@ class World:
         return {k: getattr(c, k) for k, _ in capi.FusedConfig._fields_}
 
     def set_fused_config(self, smem_cap: int, teams: int = 2, register_blocks: int = 0) -> None:
-        """teams: 0 every scene a block, 1 small scenes one per warp, 2 also mid-size scenes on two warps."""
+        """teams: 0 every scene a block, 1 small scenes a quarter of one, 2 also mid-size scenes half of one."""
         check(capi.lib().dyph_world_set_fused_config(self.h, int(smem_cap), int(teams), int(register_blocks)),
               "dyph_world_set_fused_config")
 

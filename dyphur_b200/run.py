@@ -21,9 +21,9 @@ kernel that runs once per frame.
 --adjoint EVERY runs one differentiable rollout of n_frames (checkpoints every
 EVERY frames) and its backward pass instead, loss = squared distance of the
 boxes to the scenes' targets (the push workload), and prints both times; the
-backward pass runs one record and one reverse launch per frame, last frame
-first, so `ncu -k regex:scene_frame_reverse -s F -c 1` captures frame
-n_frames - 1 - F's reverse launch.
+backward pass runs one record and one reverse launch per checkpoint segment,
+last segment first, so `ncu -k regex:scene_frame_reverse -s S -c 1` captures
+the reverse launch of the S-th segment from the end.
 """
 from __future__ import annotations
 
@@ -54,7 +54,7 @@ def parse(argv=None):
     ap.add_argument("--smem-cap", type=int, default=None,
                     help="batch: shared memory cap per block of the fused frame (bytes; 0 = what it needs)")
     ap.add_argument("--teams", type=int, default=None, choices=[0, 1, 2],
-                    help="batch: 0 every scene a block, 1 small scenes one per warp, 2 also mid-size on two warps")
+                    help="batch: 0 every scene a block, 1 small scenes a quarter of one, 2 also mid-size half of one")
     ap.add_argument("--register-blocks", type=int, default=0, choices=[0, 4, 5, 6],
                     help="batch: register budget of the fused frame kernel (resident blocks per SM)")
     ap.add_argument("--autotune", type=int, default=0, metavar="FRAMES",

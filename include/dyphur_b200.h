@@ -385,9 +385,10 @@ dyph_status dyph_world_step(dyph_world* w, int32_t n_frames, dyph_stream s);
  * graphs. */
 dyph_status dyph_world_set_scenes(dyph_world* w, uint32_t n_scenes, const uint32_t* body_offset,
                                   const dyph_aabb* scene_bounds);
-/* Batched worlds whose frame runs fused (one kernel launch per frame, one
- * thread block per scene: integrate, pair search, narrowphase and solve in
- * shared memory, see dyph_world_set_scenes) keep each scene's pairs and
+/* Batched worlds whose frame runs fused (a team of threads per scene:
+ * integrate, pair search, narrowphase and solve in shared memory, see
+ * dyph_world_set_scenes; one launch for all frames of a call when every block
+ * is resident at once, else one per frame) keep each scene's pairs and
  * contacts in per-scene slots. This call compacts the last frame's lists, in
  * the order the per-frame stages produce them, into the broadphase's pair
  * list, the narrowphase's ContactView and the solver's colours (queued on s;
@@ -402,10 +403,13 @@ dyph_status dyph_world_sync_lists(dyph_world* w, dyph_stream s);
  *                  contacts' words; with no cap and more scenes than SMs, at
  *                  most what lets two blocks share an SM;
  *   teams          0: every scene takes a block; 1: scenes whose frame fits
- *                  a quarter of that run one per warp, four to a block; 2: also
- *                  scenes that fit half of it on two warps, two to a block;
+ *                  a quarter of that run on a quarter of a block, four to a
+ *                  block; 2: also scenes that fit half of it on half a block;
  *   register_blocks the kernel's register budget: 4, 5 or 6 resident blocks
- *                  per SM (128, 96 or 80 registers a thread; 0 = 4).
+ *                  of 128 threads per SM (128, 96 or 80 registers a thread;
+ *                  0 = 4). With 4, blocks have 256 threads (two per SM) when
+ *                  shared memory leaves room for two blocks an SM at most or
+ *                  there are at most two per SM.
  * dyph_world_autotune times `frames` frames of each candidate (smem caps
  * 96/72/56/48/44/40/32 KB below the need and the floor itself, each team
  * policy, each register budget) from the
@@ -417,8 +421,8 @@ dyph_status dyph_world_sync_lists(dyph_world* w, dyph_stream s);
 typedef struct dyph_fused_config {
     uint32_t smem_bytes;    /* dynamic shared memory per block */
     uint32_t teams;         /* team policy (0, 1, 2) */
-    uint32_t warp_scenes;   /* scenes run by one warp */
-    uint32_t half_scenes;   /* scenes run by two warps */
+    uint32_t warp_scenes;   /* scenes run by a quarter of a block */
+    uint32_t half_scenes;   /* scenes run by half a block */
     uint32_t block_scenes;  /* scenes run by a whole block */
     uint32_t blocks;        /* thread blocks per frame */
     uint32_t blocks_per_sm; /* resident blocks per SM at smem_bytes and the register budget */
@@ -465,15 +469,15 @@ dyph_status dyph_world_download_phase_ns(dyph_world* w, dyph_stream s, uint64_t*
  * state at frame 0 ([13][n]), and d_grad_inv_mass, the adjoint of every
  * body's inverse mass ([n], overwritten; the inverse inertia is held fixed).
  * Each checkpoint segment is recomputed forward once, from its checkpoint, by
- * a recording kernel (one launch per frame) that keeps every frame's contact
+ * a recording kernel (one launch per segment) that keeps every frame's contact
  * set, narrowphase branches and pre-solve states and stores the next frame's
- * start state; every frame is then reversed by one launch of the reverse
- * kernel, which applies the hand-written adjoints of the renormalisations,
+ * start state; the segment's frames are then reversed by one launch of the
+ * reverse kernel, which applies the hand-written adjoints of the renormalisations,
  * the contact solves (in reverse level order), the narrowphase and the
  * integration. Segment seg - 1 is recorded on a side stream while segment
- * seg is reversed on s (with every = 1, a segment is up to 4 frames, each
- * recorded from its own checkpoint, as many as keep two segments' record
- * sets within 2 GiB; 1 frame when they do not fit the device). The contact set and every branch are those of the
+ * seg is reversed on s (with every = 1, a segment is up to 4 frames, as many
+ * as keep two segments' record sets within 2 GiB; 1 frame when they do not fit
+ * the device). The contact set and every branch are those of the
  * forward frames. Static bodies get zero adjoints. Returns
  * DYPH_ERR_UNSUPPORTED (the gradients are then incomplete) when a frame took
  * a path the adjoint does not differentiate: a contact that first acted after
