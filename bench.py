@@ -310,16 +310,18 @@ def flow_kernel_bytes(n: int, contacts: np.ndarray) -> np.ndarray:
 def frame_kernel_bytes(n: int, pairs: np.ndarray, contacts: np.ndarray) -> np.ndarray:
     """Compulsory bytes of one fused batched-frame launch (scene_frame_kernel):
     per body the state it reads (80 B), its shape index, flags, shape type and
-    half extents (24 B) and the state it writes (52 B); per stored pair its
-    4-byte record; per contact its 36-byte row and 4-byte colour. Pairs and
-    contacts otherwise live in shared memory."""
-    return 156.0 * n + 4.0 * pairs.astype(np.float64) + 40.0 * contacts.astype(np.float64)
+    half extents (24 B) and the state it writes (52 B). Pairs and contacts live
+    in shared memory; the last frame of a call also stores them: 4 B per pair,
+    36-byte row and 4-byte colour per contact."""
+    b = np.full(len(pairs), 156.0 * n)
+    b[-1] += 4.0 * float(pairs[-1]) + 40.0 * float(contacts[-1])
+    return b
 
 
 def flow_kernel_active(contacts: np.ndarray, mode: int) -> np.ndarray:
     """Frames on which the dataflow kernel does the solve: the sequential order
-    at <= 2048 contacts and the reference order at <= 256 run the one-block
-    kernel, empty frames nothing, more than 16 contacts per resident thread the
+    and the reference order's at <= 256 run the one-block kernel up to 128
+    contacts, empty frames nothing, more than 16 contacts per resident thread the
     round-synchronous kernel."""
     c = contacts.astype(np.int64)
     seq = (mode == 1) | ((mode == 0) & (c <= 256))
@@ -467,8 +469,8 @@ def probe_flow_kernel(w, frames, mode, torch, fused=False):
         kernel = "scene_frame_kernel"
         act = np.ones(frames, bool)
         b = frame_kernel_bytes(n, pairs, contacts)
-        rule = ("156 B per body (read state 80 + shape and flags 24, write state 52) + 4 B per stored pair + "
-                "40 B per contact (row 36 + colour 4)")
+        rule = ("156 B per body (read state 80 + shape and flags 24, write state 52); the last frame + 4 B per "
+                "stored pair + 40 B per contact (row 36 + colour 4)")
     else:
         kernel = "flow_solve_kernel"
         act = flow_kernel_active(contacts, mode)
