@@ -515,9 +515,10 @@ __global__ void __launch_bounds__(kBpThreads) pair_subtree_kernel(uint32_t n_u, 
 // Pass 1 for a single scene of at most kTiledBodies bodies, one warp per tile of
 // 32 leaves in Morton order and part of the tiles before it: a lane holds a leaf
 // and meets 32 tile boxes as broadcasts (see pair_overlap), then the leaves of
-// each tile that some lane's leaf met. Wide leaves are kept out of the tiles and meet every leaf. Every
-// overlapping pair is found once, from its later leaf (or from the leaf that is
-// not wide), and goes to the bucket of its smaller body index. The tests are
+// each tile that some lane's leaf met. Wide leaves are kept out of the tiles and
+// meet every leaf. Every overlapping pair is found once, from its later leaf (or
+// from the leaf that is not wide), and goes to the bucket of its smaller body
+// index. The tests are
 // dense and independent, where a walk of the tree per leaf waits for a node per
 // step in divergent lanes; but tiles that straddle distant parts of the Morton
 // order meet more tiles the more there are. Whole broadphase, tiles against tree

@@ -3,6 +3,8 @@
 
 #include <cuda_runtime.h>
 
+#include <vector>
+
 #include "contact_math.cuh"
 #include "sort.cuh"
 
@@ -73,6 +75,7 @@ struct dyph_narrowphase {
     uint32_t max_pairs_seen = 0;  // status capacity in tiles * 256
     float4* packed = nullptr;     // [3 packed_n] bodies as the pair test reads them (see pack_bodies_kernel)
     uint32_t packed_n = 0;
+    std::vector<float4*> outgrown;  // smaller packed buffers (see narrowphase_reserve_bodies)
 };
 
 struct dyph_xpbd {

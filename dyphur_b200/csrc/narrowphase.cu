@@ -173,6 +173,7 @@ void narrowphase_destroy(dyph_narrowphase* np) {
                     np->view.norm_x, np->view.norm_y, np->view.norm_z, np->view.depth, np->counts, np->status, np->packed};
     for (void* p : ptrs)
         if (p) cudaFree(p);
+    for (float4* p : np->outgrown) cudaFree(p);
     delete np;
 }
 
@@ -194,11 +195,14 @@ constexpr uint32_t kPackedBodies = 8192;
 
 dyph_status narrowphase_reserve_bodies(dyph_narrowphase* np, uint32_t n) {
     if (n < kPackedBodies || n <= np->packed_n) return DYPH_OK;
-    if (np->packed) cudaFree(np->packed);
-    np->packed = nullptr;
-    np->packed_n = 0;
-    if (cudaMalloc(&np->packed, 48ull * n) != cudaSuccess) return DYPH_ERR_NOMEM;
-    np->packed_n = n;
+    // A smaller buffer stays until the handle goes: graphs recorded with it still
+    // write there. Each is at least twice the one before.
+    const uint32_t room = std::max(n, np->packed_n > 0x7FFFFFFFu ? n : 2u * np->packed_n);
+    float4* fresh = nullptr;
+    if (cudaMalloc(&fresh, 48ull * room) != cudaSuccess) return DYPH_ERR_NOMEM;
+    if (np->packed) np->outgrown.push_back(np->packed);
+    np->packed = fresh;
+    np->packed_n = room;
     return DYPH_OK;
 }
 
