@@ -822,6 +822,11 @@ dyph_status broadphase_build(dyph_broadphase* bp, const dyph_bodies* bodies, con
     return DYPH_OK;
 }
 
+dyph_status setup_done() {
+    DYPH_CUDA_TRY(cudaStreamSynchronize(cudaStreamLegacy));
+    return DYPH_OK;
+}
+
 dyph_status broadphase_create(uint32_t max_bodies, uint32_t max_pairs, dyph_broadphase** out) {
     if (!out || max_bodies == 0 || max_pairs == 0 || max_bodies >= (1u << 30)) return DYPH_ERR_INVALID;
     auto* bp = new (std::nothrow) dyph_broadphase();
@@ -852,7 +857,7 @@ dyph_status broadphase_create(uint32_t max_bodies, uint32_t max_pairs, dyph_broa
     // Arrival counters start even; every build adds none or two at a split.
     if (ok) ok = cudaMemset(bp->bvh.flags, 0, ni * sizeof(uint32_t)) == cudaSuccess;
     if (ok) ok = cudaMemset(bp->counts, 0, 8 * sizeof(uint32_t)) == cudaSuccess;
-    if (ok) ok = sort_prepare() == DYPH_OK;
+    if (ok) ok = sort_prepare() == DYPH_OK && setup_done() == DYPH_OK;
     if (!ok) {
         broadphase_destroy(bp);
         return DYPH_ERR_NOMEM;
@@ -906,7 +911,7 @@ dyph_status broadphase_set_scenes(dyph_broadphase* bp, uint32_t n_scenes, const 
     }
     bp->n_scenes = n_scenes;
     bp->scene_bits = bits;
-    return DYPH_OK;
+    return setup_done();
 }
 
 void broadphase_destroy(dyph_broadphase* bp) {

@@ -148,6 +148,12 @@ dyph_status xpbd_solve(dyph_xpbd* sv, const dyph_contacts* contacts, const dyph_
 dyph_status xpbd_set_scenes(dyph_xpbd* sv, uint32_t n_scenes, const uint32_t* h_body_offset,
                             const uint32_t* d_body_offset, const uint32_t* d_scene_of);
 
+// Set-up copies and fills go through the default stream and may still be on
+// their way when the call returns, and the streams that read them do not wait
+// for the default stream (a world's own never do): whatever makes or fills
+// buffers that way ends with this.
+dyph_status setup_done();
+
 // Pre-set kernel attributes of the sort (call once, outside graph capture).
 dyph_status sort_prepare();
 

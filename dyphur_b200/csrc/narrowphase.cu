@@ -155,7 +155,7 @@ dyph_status narrowphase_create(uint32_t max_contacts, dyph_narrowphase** out) {
     bool ok = true;
     for (void** b : bufs) ok = ok && cudaMalloc(b, static_cast<size_t>(max_contacts) * 4) == cudaSuccess;
     if (ok) ok = cudaMalloc(&np->counts, 4 * sizeof(uint32_t)) == cudaSuccess;
-    if (ok) ok = cudaMemset(np->counts, 0, 4 * sizeof(uint32_t)) == cudaSuccess;
+    if (ok) ok = cudaMemset(np->counts, 0, 4 * sizeof(uint32_t)) == cudaSuccess && setup_done() == DYPH_OK;
     if (!ok) {
         narrowphase_destroy(np);
         return DYPH_ERR_NOMEM;

@@ -208,7 +208,7 @@ dyph_status xpbd_create(int32_t n_iters, uint32_t max_contacts, uint32_t max_bod
               cudaMalloc(&sv->csr_off, (mb + 1) * 4) == cudaSuccess && cudaMalloc(&sv->csr_cur, mb * 4) == cudaSuccess &&
               cudaMalloc(&sv->csr, 2 * mc * 4) == cudaSuccess &&
               cudaMalloc(&sv->partial, kFlowMaxBlocks * 4) == cudaSuccess &&
-              cudaMemset(sv->sweep_tag, 0, 4) == cudaSuccess;
+              cudaMemset(sv->sweep_tag, 0, 4) == cudaSuccess && setup_done() == DYPH_OK;
     if (!ok) {
         xpbd_destroy(sv);
         return DYPH_ERR_NOMEM;

@@ -466,7 +466,7 @@ extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_strea
     if (st == DYPH_OK) {
         w->sv->mode = desc->mode;
         if (cudaMalloc(&w->stats, kStatsWords * sizeof(uint32_t)) != cudaSuccess ||
-            cudaMemset(w->stats, 0, kStatsWords * sizeof(uint32_t)) != cudaSuccess ||
+            cudaMemset(w->stats, 0, kStatsWords * sizeof(uint32_t)) != cudaSuccess || setup_done() != DYPH_OK ||
             cudaStreamCreateWithFlags(&w->stream, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&w->ev_in, cudaEventDisableTiming) != cudaSuccess ||
             cudaEventCreateWithFlags(&w->ev_out, cudaEventDisableTiming) != cudaSuccess)
@@ -509,7 +509,7 @@ bool solo_prepare(dyph_world* w) {
     w->s_off = true;
     if (fused_smem_prepare() != DYPH_OK || run_words(w) != DYPH_OK ||
         cudaMalloc(&w->s_buf, words * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess) {
+        cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess || setup_done() != DYPH_OK) {
         cudaGetLastError();
         return false;
     }
@@ -884,7 +884,7 @@ dyph_status setup_reverse(dyph_world* w) {
     w->r_warp_scenes = n_small;
     w->r_half_scenes = n_mid;
     w->r_block_scenes = n_scenes - n_small - n_mid;
-    return DYPH_OK;
+    return setup_done();
 }
 
 // The words of a launch's statistics.
@@ -1324,7 +1324,7 @@ extern "C" dyph_status dyph_world_set_phase_timing(dyph_world* w, int on) {
     if (!w->f_phase && cudaMalloc(&w->f_phase, kFramePhases * sizeof(unsigned long long)) != cudaSuccess)
         return DYPH_ERR_NOMEM;
     DYPH_CUDA_TRY(cudaMemset(w->f_phase, 0, kFramePhases * sizeof(unsigned long long)));
-    return DYPH_OK;
+    return setup_done();
 }
 
 extern "C" dyph_status dyph_world_download_phase_ns(dyph_world* w, dyph_stream s, uint64_t* out, uint32_t cap) {
@@ -1427,7 +1427,9 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
         if (w->a_sets) cudaFree(w->a_sets);
         w->a_sets = nullptr;
         if (cudaMalloc(&w->a_sets, table.size() * sizeof(AdjSet)) != cudaSuccess) return DYPH_ERR_NOMEM;
-        DYPH_CUDA_TRY(cudaMemcpy(w->a_sets, table.data(), table.size() * sizeof(AdjSet), cudaMemcpyHostToDevice));
+        // read by the recordings on a_stream and by the reversals that wait for them
+        DYPH_CUDA_TRY(cudaMemcpyAsync(w->a_sets, table.data(), table.size() * sizeof(AdjSet), cudaMemcpyHostToDevice,
+                                      w->a_stream));
     }
     if (seg_states > w->a_seg_frames) {
         for (float*& b : w->a_seg) {
