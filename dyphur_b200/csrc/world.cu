@@ -61,12 +61,12 @@ struct dyph_world {
     uint32_t* f_items = nullptr;         // [4 f_n_items] work items of the fused kernel
     uint32_t f_n_items = 0;
     unsigned long long* f_phase = nullptr;  // [kFramePhases] phase timing of fused frames (null = off)
-    // A small single scene's frames but a call's last (solo_prepare): one block of
+    // A small single scene's frames but a call's last (solo_frames): one block of
     // the fused kernel on one scene. Device words: body, pair and contact ranges,
-    // the work item and counts; then the pair slots and the contact words.
+    // the work item and counts; then the pair slots and the contact words. Null
+    // when the scene is not small.
     uint32_t* s_buf = nullptr;
     uint32_t s_smem = 0, s_pairs = 0, s_contacts = 0;
-    bool s_off = false;                   // its buffers could not be had
     dyph_solver_mode graph_mode = DYPH_SOLVER_REFERENCE;  // the solver mode that the captured frame holds
     // Adjoint of fused frames (dyph_world_rollout_backward), allocated on first use.
     // Record sets, one per frame of two checkpoint segments: contact records,
@@ -451,6 +451,55 @@ extern "C" void dyph_world_destroy(dyph_world* w) {
     delete w;
 }
 
+namespace {
+dyph_status run_words(dyph_world* w);
+uint32_t fused_smem_need(uint32_t max_nb);
+uint32_t fused_smem_floor(uint32_t max_nb);
+dyph_status fused_smem_prepare();
+
+// A single scene of at most this many bodies steps the frames of a call but the
+// last on one block of the fused kernel, in one launch: a frame is then one
+// block's work instead of a dozen launches that a scene of this size cannot
+// fill. The last frame runs the stage kernels, so the tree, the lists, the
+// colours and the statistics that a program reads after a call are theirs.
+// A frame, one block against the stage kernels: 17 and 66 us on 9 stacked boxes,
+// 113 and 177 on 201, 156 and 181 on 289, 273 and 208 on 433; in the sequential
+// order, whose chains leave a chip idle, 322 and 725 us on 433; 27 and 82 us on a
+// loose pile of 400.
+constexpr uint32_t kSoloBodies = 256, kSoloSequentialBodies = 512;
+bool solo_size(const dyph_world* w) {
+    return w->desc.bodies.n <= (w->sv->mode == DYPH_SOLVER_SEQUENTIAL ? kSoloSequentialBodies : kSoloBodies);
+}
+
+// The one block's buffers, made with the world: a step allocates nothing, since
+// it may run inside a stream capture or beside one. Without them the world steps
+// every frame on the stage kernels.
+void solo_reserve(dyph_world* w) {
+    if (!solo_size(w)) return;
+    const uint32_t n = w->desc.bodies.n;
+    // no more pairs than there are, so that the slots stay small whatever the capacities
+    const uint32_t pairs = std::min(w->bp->max_pairs, n * (n - 1u) / 2u), contacts = std::min(w->np->max_contacts, pairs);
+    const size_t words = kSoloHead + pairs + static_cast<size_t>(kSceneWords) * (contacts + 1u);
+    const uint32_t head[kSoloHead] = {0u, n, 0u, pairs, 0u, contacts, 0u, 0u, 0u, kItemBlock, kItemEmpty, kItemEmpty};
+    if (fused_smem_prepare() != DYPH_OK || run_words(w) != DYPH_OK ||
+        cudaMalloc(&w->s_buf, words * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess || setup_done() != DYPH_OK) {
+        cudaGetLastError();
+        if (w->s_buf) cudaFree(w->s_buf);
+        w->s_buf = nullptr;
+        return;
+    }
+    w->s_pairs = pairs;
+    w->s_contacts = contacts;
+    w->s_smem = fused_smem_need(n);
+}
+
+// Whether the frames of a call but the last run on one block.
+bool solo_frames(const dyph_world* w) {
+    return w->s_buf && !w->fused && w->bp->n_scenes == 0u && !w->traj_host && solo_size(w);
+}
+}  // namespace
+
 extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_stream, dyph_world** out) {
     if (!desc || !out || desc->bodies.n == 0 || desc->integrator.n_substeps <= 0) return DYPH_ERR_INVALID;
     dyph_status dc = dyph_device_check();
@@ -476,50 +525,12 @@ extern "C" dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_strea
         dyph_world_destroy(w);
         return st;
     }
+    solo_reserve(w);
     *out = w;
     return DYPH_OK;
 }
 
 namespace {
-dyph_status run_words(dyph_world* w);
-uint32_t fused_smem_need(uint32_t max_nb);
-uint32_t fused_smem_floor(uint32_t max_nb);
-dyph_status fused_smem_prepare();
-
-// A single scene of at most this many bodies steps the frames of a call but the
-// last on one block of the fused kernel, in one launch: a frame is then one
-// block's work instead of a dozen launches that a scene of this size cannot
-// fill. The last frame runs the stage kernels, so the tree, the lists, the
-// colours and the statistics that a program reads after a call are theirs.
-// A frame, one block against the stage kernels: 17 and 66 us on 9 stacked boxes,
-// 113 and 177 on 201, 156 and 181 on 289, 273 and 208 on 433; in the sequential
-// order, whose chains leave a chip idle, 322 and 725 us on 433; 27 and 82 us on a
-// loose pile of 400.
-constexpr uint32_t kSoloBodies = 256, kSoloSequentialBodies = 512;
-
-bool solo_prepare(dyph_world* w) {
-    const uint32_t n = w->desc.bodies.n;
-    const uint32_t most = w->sv->mode == DYPH_SOLVER_SEQUENTIAL ? kSoloSequentialBodies : kSoloBodies;
-    if (w->fused || w->bp->n_scenes != 0u || n > most || w->s_off || w->traj_host) return false;
-    if (w->s_buf) return true;
-    // no more pairs than there are, so that the slots stay small whatever the capacities
-    const uint32_t pairs = std::min(w->bp->max_pairs, n * (n - 1u) / 2u), contacts = std::min(w->np->max_contacts, pairs);
-    const size_t words = kSoloHead + pairs + static_cast<size_t>(kSceneWords) * (contacts + 1u);
-    const uint32_t head[kSoloHead] = {0u, n, 0u, pairs, 0u, contacts, 0u, 0u, 0u, kItemBlock, kItemEmpty, kItemEmpty};
-    w->s_off = true;
-    if (fused_smem_prepare() != DYPH_OK || run_words(w) != DYPH_OK ||
-        cudaMalloc(&w->s_buf, words * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess || setup_done() != DYPH_OK) {
-        cudaGetLastError();
-        return false;
-    }
-    w->s_off = false;
-    w->s_pairs = pairs;
-    w->s_contacts = contacts;
-    w->s_smem = fused_smem_need(n);
-    return true;
-}
-
 // The frames of a solo scene before a call's last one.
 dyph_status enqueue_solo(dyph_world* w, cudaStream_t s, uint32_t n_frames) {
     for (uint32_t done = 0; done < n_frames; done += kMaxRunFrames) {
@@ -563,7 +574,7 @@ dyph_status world_step(dyph_world* w, int32_t n_frames, dyph_stream s, float* ck
             w->graph_mode = w->sv->mode;
         }
         int32_t f = 0;
-        if (n_frames > 1 && solo_prepare(w)) {
+        if (n_frames > 1 && solo_frames(w)) {
             const dyph_status st = enqueue_solo(w, w->stream, static_cast<uint32_t>(n_frames - 1));
             if (st != DYPH_OK) return st;
             f = n_frames - 1;
@@ -602,7 +613,7 @@ extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frame
         cudaGraphExecDestroy(w->episode);
         w->episode = nullptr;
     }
-    const bool solo = probe_stage < 0 && n_frames > 1 && solo_prepare(w);
+    const bool solo = probe_stage < 0 && n_frames > 1 && solo_frames(w);
     cudaGraph_t g = nullptr;
     DYPH_CUDA_TRY(cudaStreamBeginCapture(w->stream, cudaStreamCaptureModeThreadLocal));
     dyph_status st = DYPH_OK;
@@ -1234,6 +1245,8 @@ extern "C" dyph_status dyph_world_set_scenes(dyph_world* w, uint32_t n_scenes, c
         st = setup_fused(w, n_scenes, body_offset);
         if (st != DYPH_OK && st != DYPH_ERR_TOO_LARGE) return st;
     }
+    if (w->s_buf) cudaFree(w->s_buf);  // a batch has no use for it
+    w->s_buf = nullptr;
     // Captured frames launch the single-scene form: record them again.
     if (w->graph) cudaGraphExecDestroy(w->graph);
     if (w->episode) cudaGraphExecDestroy(w->episode);
