@@ -525,7 +525,8 @@ __global__ void __launch_bounds__(kBpThreads) pair_subtree_kernel(uint32_t n_u, 
 // walks: 52 and 67 us at 500 bodies of a pile, 89 and 122 at 2,000, 142 and 198 at
 // 10,000, 209 and 274 at 32,000, 343 and 320 at 48,000.
 // A NaN bound overlaps everything it is compared with, and a tree walk meets it
-// only below ancestors that overlap: with one in the scene every leaf walks.
+// only below ancestors that overlap: with one in the scene every leaf walks to the
+// earlier leaves, as the reference's do (core/src/broadphase.cpp:290-345).
 constexpr uint32_t kTiledBodies = 32768;
 constexpr int kTileWarps = kBpThreads / 32;
 __global__ void __launch_bounds__(kBpThreads) pair_tiles_kernel(uint32_t n_u, BvhBuffers T, uint32_t parts,
@@ -541,10 +542,7 @@ __global__ void __launch_bounds__(kBpThreads) pair_tiles_kernel(uint32_t n_u, Bv
         if (part != 0u || k >= n_u) return;
         const int n = static_cast<int>(n_u), node = n - 1 + static_cast<int>(k);
         const uint4 r0 = __ldg(&T.trav[2 * node]);
-        const bool me_big = __ldg(&T.trav[2 * node + 1]).w != 0u;
-        walk_pairs(
-            T, n, unpack_box(r0), static_cast<int>(k), me_big, 0, 0, n,
-            [&](uint32_t other) { bucket_pair(T, r0.w, other); }, [](int) { return false; });
+        walk(T, n, unpack_box(r0), 0, static_cast<int>(k), [&](uint32_t other) { bucket_pair(T, r0.w, other); });
         return;
     }
     const uint4 mine = __ldg(&T.leaf_box[k]);
@@ -634,13 +632,22 @@ __global__ void __launch_bounds__(kBpThreads) pair_tiles_kernel(uint32_t n_u, Bv
     }
 }
 
+// Whether a walk with query q reaches leaf k: its box and those above it overlap.
+__device__ __forceinline__ bool reaches(const BvhBuffers& T, int n, int k, const BoxF& q) {
+    int budget = n;
+    for (int node = n - 1 + k; node >= 0 && budget-- > 0; node = T.parent[node])
+        if (!box_overlap(unpack_box(T.aabb[node]), q)) return false;
+    return true;
+}
+
 // Pass 2, one block per kWriteBodies bodies: place each body's pairs with a
 // block scan + decoupled look-back (the counts are final after pass 1, so every
 // tile publishes its aggregate at once), then write them sorted by b. Each warp
 // ranks four buckets at a time, an element's place being the number of smaller
 // partners (the partners are distinct): bound by the latency of a bucket's load,
 // so a warp has four in flight and few in turn. A bucket that overflowed is
-// rebuilt by a full traversal from the body's own leaf.
+// rebuilt by a full traversal from the body's own leaf; with a NaN in the scene
+// (counts[4], tiled search only), body by body, from the later leaf of each two.
 constexpr int kWriteBodies = 64;
 __global__ void __launch_bounds__(kBpThreads) pair_write_kernel(uint32_t n_u, BvhBuffers T, uint2* __restrict__ pairs,
                                                                 uint32_t max_pairs, uint32_t* __restrict__ counts,
@@ -680,9 +687,18 @@ __global__ void __launch_bounds__(kBpThreads) pair_write_kernel(uint32_t n_u, Bv
         const BoxF q = unpack_box(__ldg(&T.trav[2 * (n - 1 + static_cast<int>(leaf))]));
         int sb, se;
         scene_leaves(T, n, static_cast<int>(leaf), sb, se);
-        traverse(T, n, q, a, a, P, sb, se + 1);
         uint32_t written = 0;
-        while (true) {
+        const bool nan = counts[4] != 0u;
+        for (uint32_t b = a + 1u; nan && b < n_u; ++b) {
+            const uint32_t other = __ldg(&T.inv_sorted[b]);
+            const bool met = other < leaf ? reaches(T, n, static_cast<int>(other), q)
+                                          : reaches(T, n, static_cast<int>(leaf), unpack_box(T.aabb[n_u - 1u + other]));
+            if (!met) continue;
+            if (off + written < max_pairs) pairs[off + written] = make_uint2(a, b);
+            ++written;
+        }
+        if (!nan) traverse(T, n, q, a, a, P, sb, se + 1);
+        while (!nan) {
             for (int i = 0; i < P.m; ++i) {
                 const uint32_t pos = off + written + static_cast<uint32_t>(i);
                 if (pos < max_pairs) pairs[pos] = make_uint2(a, P.v[i]);

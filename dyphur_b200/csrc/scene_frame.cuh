@@ -12,12 +12,15 @@
 //     inclusive test (:322-325), because internal nodes merge the leaf boxes
 //     exactly. So every (a, b) with a < b is tested directly and the pairs
 //     come out in ascending (a << 32 | b) order, as Broadphase::sort_pairs
-//     leaves them; a scene keeps the first max_pairs of them, as it does alone;
+//     leaves them; a scene keeps the first max_pairs of them, as it does alone.
+//     A NaN bound overlaps every other, where a tree walk meets it only below
+//     ancestors that overlap: a single scene's frames follow the walk there
+//     (reach_box), those of a batch take every such pair;
 //   * narrowphase: process_pair (core/src/narrowphase.cpp:920-1001) per pair,
 //     contacts compacted in pair order, the first max_contacts kept;
 //   * solve: scene_solve (solver_scene.cuh).
 // A scene's frame is therefore bit-identical to the frame of the scene
-// stepped alone. The frame's pair and contact lists stay in per-scene slots
+// stepped alone (of a batch, as long as no leaf box holds a NaN). The frame's pair and contact lists stay in per-scene slots
 // and are compacted into the broadphase's / narrowphase's lists on request
 // (scene_gather_*).
 #pragma once
@@ -96,6 +99,7 @@ struct FrameParams {
     // State before frame ckpt_first + j ckpt_every: rows [13][n] at j of ckpt.
     float* ckpt;
     uint32_t ckpt_first, ckpt_every;
+    dyph_aabb bounds;  // of a single scene (Morton codes of bodies with NaN boxes about)
 };
 
 // Phases of a scene's fused frame, timed per scene by its team leader when
@@ -159,6 +163,40 @@ struct FrameOut {
     uint32_t m, groups;
 };
 
+__device__ __forceinline__ bool pair_box_nan(uint4 b) {
+    const __half2 x = half2_bits(b.x), y = half2_bits(b.y), z = half2_bits(b.z);
+    return (__heq2_mask(x, x) & __heq2_mask(y, y) & __heq2_mask(z, z)) != 0xFFFFFFFFu;
+}
+
+// The pair box of leaf i as a walk of the tree meets it. The walk reaches a leaf
+// below nodes that all overlap the query, and a node's box leaves out the NaN
+// bounds among its leaves: a NaN bound of the leaf is held to the tightest bound of
+// the nodes above it, the least (pair boxes negate the upper bounds) among the bodies
+// whose keys share the longest prefix with the leaf's and whose bound is a number.
+// The leaf's other bounds lie inside its ancestors'. code: Morton codes in the w
+// words of `reach`.
+__device__ __noinline__ uint4 reach_box(const uint4* box, const uint4* reach, uint32_t nb, uint32_t i) {
+    uint32_t out[3] = {box[i].x, box[i].y, box[i].z};
+    const uint64_t key = (static_cast<uint64_t>(reach[i].w) << 32) | i;
+#pragma unroll
+    for (int h = 0; h < 6; ++h) {
+        const int sh = 16 * (h & 1);
+        if (!__hisnan(__ushort_as_half(static_cast<unsigned short>(out[h >> 1] >> sh)))) continue;
+        int prefix = -1;
+        float least = 0.f;
+        for (uint32_t x = 0; x < nb; ++x) {
+            const uint32_t w = h < 2 ? box[x].x : (h < 4 ? box[x].y : box[x].z);
+            const float v = h2f_bits(static_cast<uint16_t>(w >> sh));
+            if (isnan(v)) continue;
+            const int c = __clzll(static_cast<long long>(key ^ ((static_cast<uint64_t>(reach[x].w) << 32) | x)));
+            least = c > prefix ? v : (c == prefix ? fminf(least, v) : least);
+            prefix = max(prefix, c);
+        }
+        if (prefix >= 0) out[h >> 1] = (out[h >> 1] & (0xFFFF0000u >> sh)) | (static_cast<uint32_t>(f2h_bits(least)) << sh);
+    }
+    return make_uint4(out[0], out[1], out[2], reach[i].w);
+}
+
 // Frame f of P_.n_frames of scene s by team T with `smem_bytes` of shared
 // memory at smem. The first frame loads the scene's bodies, the next ones find
 // them in shared memory as the frame before left them, and the last one writes
@@ -166,7 +204,8 @@ struct FrameOut {
 // of a call's last frame, so the frames before it do not write them.
 // Returns false after raising an error. kRecord compiles the adjoint's
 // recording in (`adj_in`, `out`); the forward frame is built without it.
-template <bool kRecord, bool kAhead>
+// kSingle: the scene is a world's only one (see reach_box).
+template <bool kRecord, bool kAhead, bool kSingle = false>
 __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem, uint32_t smem_bytes,
                             SceneShared& sh, const SceneBufs& S, const FrameBufs& F, const FrameParams& P_,
                             const AdjRun* adj_in = nullptr, FrameOut* out = nullptr) {
@@ -219,10 +258,21 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
         }
         box[i] = pair_box(leaf_box(SS.type(i), SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
                                    SS.hx(i), SS.hy(i), SS.hz(i)));
+        if (kSingle && pair_box_nan(box[i])) sh.nan = 1u;
         R.cnt[i] = 0u;
     }
     T.sync();
     phase_mark(T, P_, 0, t0);
+    const bool nan = kSingle && sh.nan != 0u;
+    uint4* reach = reinterpret_cast<uint4*>(R.mask);  // [ldb], over the masks and priorities of the solve
+    if (nan) {
+        for (uint32_t i = T.rank(); i < nb; i += T.size())
+            reach[i] = make_uint4(box[i].x, box[i].y, box[i].z, morton_code(SB.px(i), SB.py(i), SB.pz(i), P_.bounds));
+        T.sync();
+        for (uint32_t i = T.rank(); i < nb; i += T.size())
+            if (pair_box_nan(box[i])) reach[i] = reach_box(box, reach, nb, i);
+        T.sync();
+    }
     // ── candidate pairs: per body a, the partners b > a in ascending order ──
     // Every (a, b) is tested: a lane holds one body a and meets 32 partners one
     // after another, whose boxes the warp reads as broadcasts; the answers are
@@ -241,7 +291,16 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
     auto overlap_word = [&](uint32_t c, uint32_t a, const uint3& q) -> uint32_t {
         const uint32_t n_b = min(32u, nb - 32u * c);
         uint32_t w = 0;
-        if (n_b == 32u) {
+        if (nan) {
+            // the later leaf in Morton order walks to the earlier one
+            const uint32_t me = min(a, nb - 1u);
+            const uint4 mine = reach[me];
+            for (uint32_t j = 0; j < n_b; ++j) {
+                const uint32_t b = 32u * c + j;
+                const bool ov = mine.w > reach[b].w ? pair_overlap(reach[b], q) : pair_overlap(mine, facing_box(box[b]));
+                w |= ov ? 1u << j : 0u;
+            }
+        } else if (n_b == 32u) {
 #pragma unroll 8
             for (uint32_t j = 0; j < 32u; ++j) w |= pair_overlap(box[32u * c + j], q) ? 1u << j : 0u;
         } else {
@@ -311,6 +370,7 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
     phase_mark(T, P_, 1, t0);
     // ── narrowphase: contacts in pair order ──
     for (uint32_t i = T.rank(); i < nb; i += T.size()) R.cnt[i] = 0u;
+    if (kSingle && T.leader()) sh.nan = 0u;
     T.sync();
     uint32_t m_true = 0;
     const uint32_t cbase = F.contact_base[s];
@@ -414,12 +474,12 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
 
 // All frames of the launch of scene s: scenes do not depend on one another, so
 // a team takes its scene from frame to frame without waiting for the others.
-template <bool kAhead>
+template <bool kAhead, bool kSingle>
 __device__ __forceinline__ void run_scene(Team T, uint32_t s, unsigned char* smem, uint32_t smem_bytes,
                                           SceneShared& sh, const SceneBufs& S, const FrameBufs& F,
                                           const FrameParams& P_) {
     for (uint32_t f = 0; f < P_.n_frames; ++f)
-        if (!frame_scene<false, kAhead>(T, s, f, smem, smem_bytes, sh, S, F, P_)) return;
+        if (!frame_scene<false, kAhead, kSingle>(T, s, f, smem, smem_bytes, sh, S, F, P_)) return;
 }
 
 // Work item i: items[4 i] a large scene solved by the whole block when
@@ -452,17 +512,22 @@ __device__ __forceinline__ ItemTeam item_team(const uint32_t* item, uint32_t sme
 // (128 registers a thread), 5 (96) or 6 (80, a few bytes spilled), or 2 of
 // kSceneWideThreads (128). Which one runs best depends on the batch
 // (dyph_world_autotune picks the budget with the shared memory cap; the wide
-// form's rule is in setup_fused); all compute the same frames.
-template <int kMinBlocks, int kThreads>
+// form's rule is in setup_fused); all compute the same frames. kSingle: one work
+// item, a world's only scene.
+template <int kMinBlocks, int kThreads, bool kSingle = false>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) scene_frame_kernel(SceneBufs S, FrameBufs F, FrameParams P_,
                                                                            const uint32_t* __restrict__ items,
                                                                            uint32_t n_items) {
     extern __shared__ __align__(16) unsigned char scene_smem[];
     __shared__ SceneShared sh[4];
+    if (kSingle) {
+        if (threadIdx.x == 0) sh[0].nan = 0u;
+        __syncthreads();
+    }
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
         const ItemTeam t = item_team(items + 4 * it, S.smem_bytes);
         if (t.scene != kItemEmpty)
-            run_scene<kThreads == kSceneWideThreads>(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared], S, F, P_);
+            run_scene<kThreads == kSceneWideThreads, kSingle>(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared], S, F, P_);
         __syncthreads();
     }
 }

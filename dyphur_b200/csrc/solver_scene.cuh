@@ -389,6 +389,7 @@ __device__ void scene_sweep(const Team& T, uint32_t groups, uint32_t passes, con
 struct SceneShared {
     uint32_t scan[2 * (kSceneWideThreads / 32)];
     uint32_t rem, over, maxcol, passes;
+    uint32_t nan;  // a leaf box of a single scene's frame holds a NaN (frame_scene)
     int flag;
 };
 

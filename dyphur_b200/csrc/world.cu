@@ -299,13 +299,13 @@ dyph_status launch_run(dyph_world* w, const FusedRun& r, cudaStream_t s) {
         items = h + 8;
         n_items = 1u;
         smem = w->s_smem;
-        form = {reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>), kSceneWideThreads};
+        form = {reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads, true>), kSceneWideThreads};
     }
     FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
                   w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(solo ? w->graph_mode : w->sv->mode),
                   w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->stats + 4, w->f_phase, r.n_frames,
                   r.keep ? 1u : 0u, r.traj, r.traj_first, std::max(w->traj_every, 1u), r.traj_count, r.ckpt,
-                  r.ckpt_first, r.ckpt_every};
+                  r.ckpt_first, r.ckpt_every, d.scene_bounds};
     void* args[] = {&S, &F, &P, &items, &n_items};
     DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(n_items), dim3(form.threads), args, smem, s));
     frame_run_stats_kernel<<<1, kMaxRunFrames, 0, s>>>(w->f_run, r.n_frames, w->bp->counts, w->np->counts, w->sv->meta,
@@ -818,6 +818,7 @@ dyph_status fused_smem_prepare() {
                           reinterpret_cast<const void*>(scene_frame_kernel<5, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_kernel<6, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>),
+                          reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads, true>),
                           reinterpret_cast<const void*>(scene_frame_record_kernel<4, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_record_kernel<2, kSceneWideThreads>),
                           reverse_kernel()})

@@ -87,3 +87,15 @@ def test_unbounded_bodies(oracle_mod, n):
     s.shape_offset = np.array([0, len(s.shape_type)], np.uint32)
     s.shape[[0, n // 2]] = len(s.shape_type) - 1
     _compare(oracle_mod, s, tree=False)
+
+
+def test_nan_bodies_and_long_buckets(oracle_mod):
+    """A body with more partners than its bucket holds, next to NaN bodies and
+    static ones: the later leaf of each two looks for the other."""
+    for seed in range(6):
+        s = _cloud(400, "heap", seed)
+        rng = np.random.default_rng(seed)
+        s.mass[rng.integers(0, 400, 40)] = 0
+        s.pos[rng.integers(0, 400, 3), rng.integers(0, 3, 3)] = np.nan
+        s.rot[rng.integers(0, 400), 1] = np.nan
+        _compare(oracle_mod, s, tree=False)

@@ -97,3 +97,37 @@ def test_trajectory_records_every_frame():
     for f in range(20):
         a.step(1)
         assert np.array_equal(bits(a.state()[:7].T), bits(out[f].numpy()))
+
+
+def _alike(a, b):
+    """Equal bits, or both a NaN (whose payload is not part of the contract)."""
+    a, b = np.asarray(a, np.float32), np.asarray(b, np.float32)
+    return np.array_equal(np.isnan(a), np.isnan(b)) and np.array_equal(bits(a)[~np.isnan(a)], bits(b)[~np.isnan(b)])
+
+
+@pytest.mark.parametrize("rows,bodies", [([0], [50]), ([0], [-2]), ([1], [-1]), ([2, 0], [7, 8]), ([3], [-2]), ([6, 1], [20, -1]),
+                                         ([0, 1, 2], [9, 9, 9])])
+@pytest.mark.parametrize("n,start", [(8, 20), (99, 200), (127, 60), (200, 120)])
+def test_nan_bodies_meet_what_the_tree_lets_them(oracle_mod, n, start, rows, bodies):
+    """A NaN bound overlaps every other one that a walk of the tree brings it to: the
+    oracle's pairs, from one call of frames as from a call per frame."""
+    from dyphur_b200 import device
+    s = scenes.random_pile(n, seed=5)
+    o = oracle_mod.World(s)
+    assert o.step(start) == 0
+    st = o.state()
+    st[rows, [b % s.n_bodies for b in bodies]] = np.nan
+    a, b = device.World(s), device.World(s)
+    for w in (a, b):
+        w.bodies.set_state(st)
+    o.set_state(st)
+    o.step(1)
+    a.step(1)
+    assert np.array_equal(a.pairs(), o.pairs()[0]) and a.history()[0].tolist() == [o.pairs()[1]]
+    for _ in range(3):
+        a.step(1)
+    b.step(4)
+    for x, y in zip(a.history(), b.history()):
+        assert np.array_equal(x, y)
+    assert np.array_equal(a.pairs(), b.pairs()) and _alike(a.state(), b.state())
+    assert device.device_error() == 0
