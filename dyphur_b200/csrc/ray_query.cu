@@ -535,6 +535,26 @@ cudaMemPool_t ray_pool() {
     return g_ray_pool[dev];
 }
 
+// Another stream may be in a capture that forbids calls which could allocate on the
+// way: those of a query that is itself not captured are no part of it, so the thread
+// may make them while this lives.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// A captured query takes no scratch: it would put an allocation into the caller's
+// graph, which could then be instantiated only once at a time and not become part of
+// another graph. A million random rays into the settled 65,537-body pile take 6.4 ms
+// so instead of 2.7.
+bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+
 // ── contact sensor ──────────────────────────────────────────────────────────
 
 constexpr int kSensorThreads = 256;
@@ -629,8 +649,9 @@ extern "C" dyph_status dyph_ray_query(const dyph_bvh_view* bvh, const dyph_bodie
         return DYPH_ERR_INVALID;
     if (bvh->n > bodies->n) return DYPH_ERR_INVALID;
     const uint32_t grid = (n_rays + kRayThreads - 1) / kRayThreads;
-    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies) {
-        cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
+    cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
+    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies && !capturing(cs)) {
+        const RelaxedCapture relaxed;
         const size_t node_bytes = 32ull * bvh->n, leaf_bytes = 64ull * bvh->n;
         void* ws = nullptr;
         cudaMemPool_t pool = ray_pool();
@@ -651,8 +672,7 @@ extern "C" dyph_status dyph_ray_query(const dyph_bvh_view* bvh, const dyph_bodie
         }
         cudaGetLastError();  // no scratch: the rays walk the view's own arrays
     }
-    ray_query_kernel<<<grid, kRayThreads, 0, reinterpret_cast<cudaStream_t>(s)>>>(*bvh, RayScene{*bodies, *shapes},
-                                                                                   d_rays, d_hits, n_rays);
+    ray_query_kernel<<<grid, kRayThreads, 0, cs>>>(*bvh, RayScene{*bodies, *shapes}, d_rays, d_hits, n_rays);
     DYPH_CUDA_TRY(cudaGetLastError());
     return DYPH_OK;
 }
