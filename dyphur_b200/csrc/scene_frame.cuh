@@ -78,8 +78,8 @@ struct SceneBodiesShaped : SceneBodies {
 // rounds, some scene coloured, some scene solved.
 constexpr int kAccMaxColor = 0, kAccRounds = 1, kAccColored = 2, kAccSolved = 3, kAccWords = 4;
 
-// Frames of one launch at most (the per-frame count words).
-constexpr uint32_t kMaxRunFrames = 256;
+// Frames of one launch at most (the per-frame count words), and words of each.
+constexpr uint32_t kMaxRunFrames = 256, kRunRows = 5;
 
 // Parameters of the fused kernels, one launch.
 struct FrameParams {
@@ -88,8 +88,9 @@ struct FrameParams {
     float gx, gy, gz, sub_dt, half_dt, mu, dt;
     int n_substeps, mode, n_iters;
     uint32_t* acc;     // [kAccWords]
-    uint32_t* counts;  // [4][n_frames] stored / true pairs, stored / true contacts of every frame, over all scenes
-    uint32_t* status;
+    // [5][n_frames] stored / true pairs, stored / true contacts of every frame, over
+    // all scenes; bit 0: a scene past its pair capacity, bit 1: past its contact capacity
+    uint32_t* counts;
     unsigned long long* phase_ns;  // null, or [kFramePhases] device-clock ns summed over scenes
     uint32_t n_frames;             // frames of this launch
     uint32_t keep;                 // 1: the last frame's lists and statistics are kept (a call's last launch)
@@ -424,8 +425,8 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
         atomicAdd(&P_.counts[2u * P_.n_frames + f], m);
         atomicAdd(&P_.counts[3u * P_.n_frames + f], m_true);
         // a scene past its own capacity keeps its ordered prefix, as it does alone
-        if (p_true > pcap) atomicCAS(P_.status, 0u, static_cast<uint32_t>(DYPH_ERR_PAIR_OVERFLOW));
-        if (m_true > ccap) atomicCAS(P_.status, 0u, static_cast<uint32_t>(DYPH_ERR_CONTACT_OVERFLOW));
+        const uint32_t over = (p_true > pcap ? 1u : 0u) | (m_true > ccap ? 2u : 0u);
+        if (over) atomicOr(&P_.counts[4u * P_.n_frames + f], over);
     }
     phase_mark(T, P_, 2, t0);
     // ── contact solve (none without contacts, as the reference's solve returns) ──

@@ -55,7 +55,7 @@ struct dyph_world {
     uint32_t* f_contact_raw = nullptr;
     uint32_t* f_color_raw = nullptr;
     uint32_t* f_counts = nullptr;        // [4 n_scenes]
-    uint32_t* f_run = nullptr;           // [kAccWords] + [4 kMaxRunFrames] a launch's statistics (zero between launches)
+    uint32_t* f_run = nullptr;           // [kAccWords] + [kRunRows kMaxRunFrames] a launch's statistics (zero between launches)
     uint32_t* f_words = nullptr;
     uint32_t* f_pos = nullptr;           // [2 n_scenes] gather positions
     uint32_t* f_items = nullptr;         // [4 f_n_items] work items of the fused kernel
@@ -177,15 +177,18 @@ __global__ void __launch_bounds__(kMaxRunFrames) frame_run_stats_kernel(uint32_t
             np_counts[1] = c;
         }
     }
-    // the earliest frame past a capacity sets the status, its pairs before its contacts
+    // the earliest frame past a capacity sets the status: a scene's capacity before
+    // the world's, pairs before contacts
     __shared__ uint32_t s_first;
     if (f == 0) s_first = kMaxRunFrames;
+    const uint32_t over = f < n_frames ? counts[4u * n_frames + f] : 0u;
     __syncthreads();
-    if (f < n_frames && (p > max_pairs || c > max_contacts)) atomicMin(&s_first, f);
+    if (over || p > max_pairs || c > max_contacts) atomicMin(&s_first, f);
     __syncthreads();
-    if (f == s_first)
-        atomicCAS(&stats[4], 0u,
-                  static_cast<uint32_t>(p > max_pairs ? DYPH_ERR_PAIR_OVERFLOW : DYPH_ERR_CONTACT_OVERFLOW));
+    if (f == s_first) {
+        const bool pairs = over ? (over & 1u) != 0u : p > max_pairs;
+        atomicCAS(&stats[4], 0u, static_cast<uint32_t>(pairs ? DYPH_ERR_PAIR_OVERFLOW : DYPH_ERR_CONTACT_OVERFLOW));
+    }
     if (f < 16u) {
         uint32_t v = 0u;
         if (f == kMetaMaxColor && run[kAccMaxColor]) v = run[kAccMaxColor] - 1u;
@@ -197,7 +200,7 @@ __global__ void __launch_bounds__(kMaxRunFrames) frame_run_stats_kernel(uint32_t
     __syncthreads();
     if (f == 0) stats[5] = total + n_frames;
     if (f < static_cast<uint32_t>(kAccWords)) run[f] = 0u;
-    for (uint32_t i = f; i < 4u * n_frames; i += kMaxRunFrames) counts[i] = 0u;
+    for (uint32_t i = f; i < kRunRows * n_frames; i += kMaxRunFrames) counts[i] = 0u;
 }
 
 // Pose rows of every body, interleaved per body as the .trajectory row
@@ -303,7 +306,7 @@ dyph_status launch_run(dyph_world* w, const FusedRun& r, cudaStream_t s) {
     }
     FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
                   w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(solo ? w->graph_mode : w->sv->mode),
-                  w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->stats + 4, w->f_phase, r.n_frames,
+                  w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->f_phase, r.n_frames,
                   r.keep ? 1u : 0u, r.traj, r.traj_first, std::max(w->traj_every, 1u), r.traj_count, r.ckpt,
                   r.ckpt_first, r.ckpt_every, d.scene_bounds};
     void* args[] = {&S, &F, &P, &items, &n_items};
@@ -902,7 +905,7 @@ dyph_status setup_reverse(dyph_world* w) {
 // The words of a launch's statistics.
 dyph_status run_words(dyph_world* w) {
     if (w->f_run) return DYPH_OK;
-    const size_t bytes = (kAccWords + 4ull * kMaxRunFrames) * sizeof(uint32_t);
+    const size_t bytes = (kAccWords + static_cast<size_t>(kRunRows) * kMaxRunFrames) * sizeof(uint32_t);
     if (cudaMalloc(&w->f_run, bytes) != cudaSuccess) return DYPH_ERR_NOMEM;
     DYPH_CUDA_TRY(cudaMemset(w->f_run, 0, bytes));
     return DYPH_OK;
@@ -1534,7 +1537,6 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
         p.n_substeps = ip.n_substeps;
         p.mode = static_cast<int>(w->sv->mode);
         p.n_iters = w->sv->n_iters;
-        p.status = w->stats + 4;
         p.n_frames = static_cast<uint32_t>(seg_len(seg));
         return p;
     };

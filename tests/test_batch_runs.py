@@ -77,3 +77,36 @@ def test_rollout_checkpoints_of_a_run(frames, every):
     torch.cuda.synchronize()
     assert np.array_equal(bits(ckpt.cpu().numpy()), bits(np.stack(want)))
     assert np.array_equal(bits(a.state()), bits(b.state()))
+
+
+def _crowds():
+    """Scene 0: 30 fixed spheres in one place, 435 pairs and contacts in every frame.
+    Scene 1: 37 of them, and two that arrive after some frames, past its 688 contacts."""
+    from test_batch import concat_scenes
+    from test_oracle_pins import _single_scene
+    parts = []
+    for fixed, moving in ((30, 0), (37, 2)):
+        n = fixed + moving
+        pos = np.zeros((n, 3), np.float32)
+        pos[fixed:, 0] = [1.4, -1.4][:moving]
+        mass = np.r_[np.zeros(fixed), np.ones(moving)]
+        s = _single_scene([0] * n, pos.tolist(), [(1, 0.5, 0.5, 0.5)], mass.tolist(), (mass == 0).astype(int).tolist())
+        s.vel[fixed:, 0] = [-9.0, 9.0][:moving]
+        s.bounds = np.array([[-9, -9, -9, 9, 9, 9]], np.float32)
+        parts.append(s)
+    return concat_scenes(parts)
+
+
+@pytest.mark.parametrize("pairs,contacts", [(1000, 10**5), (10**5, 1000), (10**5, 10**5)])
+def test_status_is_the_first_frames_to_overflow(pairs, contacts):
+    """A run's status is that of its earliest frame past a capacity, the world's or a scene's."""
+    from dyphur_b200 import device
+    s = _crowds()
+    a, b = (device.World(s, max_pairs=pairs, max_contacts=contacts) for _ in range(2))
+    seen = []
+    for _ in range(8):
+        a.step(1)
+        seen.append(a.stats()["status"])
+    b.step(8)
+    assert (seen[0] != 0) == (min(pairs, contacts) == 1000) and seen[-1] != 0
+    assert a.stats() == b.stats()
