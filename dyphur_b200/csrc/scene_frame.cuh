@@ -176,7 +176,7 @@ __device__ __forceinline__ bool pair_box_nan(uint4 b) {
 // whose keys share the longest prefix with the leaf's and whose bound is a number.
 // The leaf's other bounds lie inside its ancestors'. code: Morton codes in the w
 // words of `reach`.
-__device__ __noinline__ uint4 reach_box(const uint4* box, const uint4* reach, uint32_t nb, uint32_t i) {
+__device__ __forceinline__ uint4 reach_box(const uint4* box, const uint4* reach, uint32_t nb, uint32_t i) {
     uint32_t out[3] = {box[i].x, box[i].y, box[i].z};
     const uint64_t key = (static_cast<uint64_t>(reach[i].w) << 32) | i;
 #pragma unroll
@@ -205,8 +205,11 @@ __device__ __noinline__ uint4 reach_box(const uint4* box, const uint4* reach, ui
 // of a call's last frame, so the frames before it do not write them.
 // Returns false after raising an error. kRecord compiles the adjoint's
 // recording in (`adj_in`, `out`); the forward frame is built without it.
-// kSingle: the scene is a world's only one (see reach_box).
-template <bool kRecord, bool kAhead, bool kSingle = false>
+// kPart: kFrameScene a frame of a batch's scene; kFrameSingle of a world's only
+// scene, which returns false with sh.nan set when a leaf box holds a NaN; kFrameNan
+// the rest of such a frame (see reach_box).
+constexpr int kFrameScene = 0, kFrameSingle = 1, kFrameNan = 2;
+template <bool kRecord, bool kAhead, int kPart = kFrameScene>
 __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem, uint32_t smem_bytes,
                             SceneShared& sh, const SceneBufs& S, const FrameBufs& F, const FrameParams& P_,
                             const AdjRun* adj_in = nullptr, FrameOut* out = nullptr) {
@@ -227,7 +230,7 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
     const uint32_t pcap = F.pair_base[s + 1] - F.pair_base[s];
     const uint32_t ccap = F.contact_base[s + 1] - F.contact_base[s];
     // ── stage and integrate ──
-    if (f == 0u) {
+    if (kPart != kFrameNan && f == 0u) {
         scene_load_bodies(T, B, b0, nb, fb, ldb);
         for (uint32_t i = T.rank(); i < nb; i += T.size()) {
             const uint32_t g = b0 + i, sh_i = P_.gb.shape[g];
@@ -237,11 +240,11 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
             half[2 * ldb + i] = P_.gs.half_z[sh_i];
         }
     }
-    if (!adj && P_.ckpt && f >= P_.ckpt_first && (f - P_.ckpt_first) % P_.ckpt_every == 0u) {
+    if (kPart != kFrameNan && !adj && P_.ckpt && f >= P_.ckpt_first && (f - P_.ckpt_first) % P_.ckpt_every == 0u) {
         const uint32_t j = (f - P_.ckpt_first) / P_.ckpt_every;
         scene_store_state(T, P_.ckpt + static_cast<size_t>(j) * 13u * P_.gb.n, P_.gb.n, b0, nb, SB);
     }
-    for (uint32_t i = T.rank(); i < nb; i += T.size()) {
+    for (uint32_t i = T.rank(); kPart != kFrameNan && i < nb; i += T.size()) {
         if (SB.im(i) != 0.f && !((info[i] >> 8) & kFlagSleeping)) {
             Pose p{SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
                    SB.vx(i), SB.vy(i), SB.vz(i)};
@@ -259,14 +262,14 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
         }
         box[i] = pair_box(leaf_box(SS.type(i), SB.px(i), SB.py(i), SB.pz(i), SB.qw(i), SB.qx(i), SB.qy(i), SB.qz(i),
                                    SS.hx(i), SS.hy(i), SS.hz(i)));
-        if (kSingle && pair_box_nan(box[i])) sh.nan = 1u;
+        if (kPart == kFrameSingle && pair_box_nan(box[i])) sh.nan = 1u;
         R.cnt[i] = 0u;
     }
     T.sync();
     phase_mark(T, P_, 0, t0);
-    const bool nan = kSingle && sh.nan != 0u;
+    if (kPart == kFrameSingle && sh.nan != 0u) return false;
     uint4* reach = reinterpret_cast<uint4*>(R.mask);  // [ldb], over the masks and priorities of the solve
-    if (nan) {
+    if (kPart == kFrameNan) {
         for (uint32_t i = T.rank(); i < nb; i += T.size())
             reach[i] = make_uint4(box[i].x, box[i].y, box[i].z, morton_code(SB.px(i), SB.py(i), SB.pz(i), P_.bounds));
         T.sync();
@@ -292,8 +295,8 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
     auto overlap_word = [&](uint32_t c, uint32_t a, const uint3& q) -> uint32_t {
         const uint32_t n_b = min(32u, nb - 32u * c);
         uint32_t w = 0;
-        if (nan) {
-            // the later leaf in Morton order walks to the earlier one
+        if (kPart == kFrameNan) {
+            // the later leaf in Morton order (of equal codes the larger index) walks to the earlier one
             const uint32_t me = min(a, nb - 1u);
             const uint4 mine = reach[me];
             for (uint32_t j = 0; j < n_b; ++j) {
@@ -371,7 +374,7 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
     phase_mark(T, P_, 1, t0);
     // ── narrowphase: contacts in pair order ──
     for (uint32_t i = T.rank(); i < nb; i += T.size()) R.cnt[i] = 0u;
-    if (kSingle && T.leader()) sh.nan = 0u;
+    if (kPart == kFrameNan && T.leader()) sh.nan = 0u;
     T.sync();
     uint32_t m_true = 0;
     const uint32_t cbase = F.contact_base[s];
@@ -475,12 +478,12 @@ __device__ bool frame_scene(Team& T, uint32_t s, uint32_t f, unsigned char* smem
 
 // All frames of the launch of scene s: scenes do not depend on one another, so
 // a team takes its scene from frame to frame without waiting for the others.
-template <bool kAhead, bool kSingle>
+template <bool kAhead>
 __device__ __forceinline__ void run_scene(Team T, uint32_t s, unsigned char* smem, uint32_t smem_bytes,
                                           SceneShared& sh, const SceneBufs& S, const FrameBufs& F,
                                           const FrameParams& P_) {
     for (uint32_t f = 0; f < P_.n_frames; ++f)
-        if (!frame_scene<false, kAhead, kSingle>(T, s, f, smem, smem_bytes, sh, S, F, P_)) return;
+        if (!frame_scene<false, kAhead>(T, s, f, smem, smem_bytes, sh, S, F, P_)) return;
 }
 
 // Work item i: items[4 i] a large scene solved by the whole block when
@@ -513,23 +516,47 @@ __device__ __forceinline__ ItemTeam item_team(const uint32_t* item, uint32_t sme
 // (128 registers a thread), 5 (96) or 6 (80, a few bytes spilled), or 2 of
 // kSceneWideThreads (128). Which one runs best depends on the batch
 // (dyph_world_autotune picks the budget with the shared memory cap; the wide
-// form's rule is in setup_fused); all compute the same frames. kSingle: one work
-// item, a world's only scene.
-template <int kMinBlocks, int kThreads, bool kSingle = false>
+// form's rule is in setup_fused); all compute the same frames.
+template <int kMinBlocks, int kThreads>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) scene_frame_kernel(SceneBufs S, FrameBufs F, FrameParams P_,
                                                                            const uint32_t* __restrict__ items,
                                                                            uint32_t n_items) {
     extern __shared__ __align__(16) unsigned char scene_smem[];
     __shared__ SceneShared sh[4];
-    if (kSingle) {
-        if (threadIdx.x == 0) sh[0].nan = 0u;
-        __syncthreads();
-    }
     for (uint32_t it = blockIdx.x; it < n_items; it += gridDim.x) {
         const ItemTeam t = item_team(items + 4 * it, S.smem_bytes);
         if (t.scene != kItemEmpty)
-            run_scene<kThreads == kSceneWideThreads, kSingle>(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared], S, F, P_);
+            run_scene<kThreads == kSceneWideThreads>(t.team, t.scene, scene_smem + t.smem, t.bytes, sh[t.shared], S, F, P_);
         __syncthreads();
+    }
+}
+
+// A single scene's frame with a NaN among its boxes, from the pairs on. Apart, so that
+// the frames without one do not carry its code (they took 1.4 us longer with it, of 17
+// on 9 boxes). Returns the team's turn, + 2 when the frame is done.
+__device__ __noinline__ uint32_t nan_frame(Team T, uint32_t f, unsigned char* smem, uint32_t smem_bytes,
+                                           SceneShared& sh, const SceneBufs& S, const FrameBufs& F,
+                                           const FrameParams& P_) {
+    const bool ok = frame_scene<false, true, kFrameNan>(T, 0u, f, smem, smem_bytes, sh, S, F, P_);
+    return T.turn | (ok ? 2u : 0u);
+}
+
+// The frames of a world's only scene, on one block of kThreads.
+template <int kThreads>
+__global__ void __launch_bounds__(kThreads, 2) scene_single_kernel(const __grid_constant__ SceneBufs S,
+                                                                   const __grid_constant__ FrameBufs F,
+                                                                   const __grid_constant__ FrameParams P_) {
+    extern __shared__ __align__(16) unsigned char scene_smem[];
+    __shared__ SceneShared sh;
+    if (threadIdx.x == 0) sh.nan = 0u;
+    __syncthreads();
+    Team T{kThreads, 0u};
+    for (uint32_t f = 0; f < P_.n_frames; ++f) {
+        if (frame_scene<false, true, kFrameSingle>(T, 0u, f, scene_smem, S.smem_bytes, sh, S, F, P_)) continue;
+        if (sh.nan == 0u) return;
+        const uint32_t r = nan_frame(T, f, scene_smem, S.smem_bytes, sh, S, F, P_);
+        T.turn = r & 1u;
+        if ((r & 2u) == 0u) return;
     }
 }
 

@@ -62,9 +62,9 @@ struct dyph_world {
     uint32_t f_n_items = 0;
     unsigned long long* f_phase = nullptr;  // [kFramePhases] phase timing of fused frames (null = off)
     // A small single scene's frames but a call's last (solo_frames): one block of
-    // the fused kernel on one scene. Device words: body, pair and contact ranges,
-    // the work item and counts; then the pair slots and the contact words. Null
-    // when the scene is not small.
+    // the fused frame's code (scene_single_kernel). Device words: body, pair and
+    // contact ranges and counts; then the pair slots and the contact words. Null when
+    // the scene is not small.
     uint32_t* s_buf = nullptr;
     uint32_t s_smem = 0, s_pairs = 0, s_contacts = 0;
     dyph_solver_mode graph_mode = DYPH_SOLVER_REFERENCE;  // the solver mode that the captured frame holds
@@ -291,26 +291,24 @@ dyph_status launch_run(dyph_world* w, const FusedRun& r, cudaStream_t s) {
                 w->frame_smem};
     FrameBufs F{w->f_pair_base, w->f_contact_base, w->f_pair_raw, w->f_contact_raw, w->f_color_raw,
                 w->f_counts, w->f_words, w->f_words_stride, w->f_contact_slots};
-    FusedForm form = fused_form(w);
-    const uint32_t* items = w->f_items;
-    uint32_t n_items = w->f_n_items, smem = w->frame_smem;
     if (solo) {
         uint32_t* h = w->s_buf;
         S = SceneBufs{h, nullptr, nullptr, nullptr, nullptr, 0, 1u, w->s_smem};
-        F = FrameBufs{h + 2, h + 4, h + kSoloHead, nullptr, nullptr, h + 12, h + kSoloHead + w->s_pairs,
+        F = FrameBufs{h + 2, h + 4, h + kSoloHead, nullptr, nullptr, h + 8, h + kSoloHead + w->s_pairs,
                       w->s_contacts + 1u, w->s_contacts};
-        items = h + 8;
-        n_items = 1u;
-        smem = w->s_smem;
-        form = {reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads, true>), kSceneWideThreads};
     }
     FrameParams P{d.bodies, d.shapes, ip.gravity[0], ip.gravity[1], ip.gravity[2], sub_dt, 0.5f * sub_dt,
                   w->sv->friction, ip.dt, ip.n_substeps, static_cast<int>(solo ? w->graph_mode : w->sv->mode),
                   w->sv->n_iters, w->f_run, w->f_run + kAccWords, w->f_phase, r.n_frames,
                   r.keep ? 1u : 0u, r.traj, r.traj_first, std::max(w->traj_every, 1u), r.traj_count, r.ckpt,
                   r.ckpt_first, r.ckpt_every, d.scene_bounds};
-    void* args[] = {&S, &F, &P, &items, &n_items};
-    DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(n_items), dim3(form.threads), args, smem, s));
+    if (solo) {
+        scene_single_kernel<kSceneWideThreads><<<1, kSceneWideThreads, w->s_smem, s>>>(S, F, P);
+    } else {
+        const FusedForm form = fused_form(w);
+        void* args[] = {&S, &F, &P, &w->f_items, &w->f_n_items};
+        DYPH_CUDA_TRY(cudaLaunchKernel(form.kernel, dim3(w->f_n_items), dim3(form.threads), args, w->frame_smem, s));
+    }
     frame_run_stats_kernel<<<1, kMaxRunFrames, 0, s>>>(w->f_run, r.n_frames, w->bp->counts, w->np->counts, w->sv->meta,
                                                       w->bp->max_pairs, w->np->max_contacts, w->stats);
     DYPH_CUDA_TRY(cudaGetLastError());
@@ -483,7 +481,7 @@ void solo_reserve(dyph_world* w) {
     // no more pairs than there are, so that the slots stay small whatever the capacities
     const uint32_t pairs = std::min(w->bp->max_pairs, n * (n - 1u) / 2u), contacts = std::min(w->np->max_contacts, pairs);
     const size_t words = kSoloHead + pairs + static_cast<size_t>(kSceneWords) * (contacts + 1u);
-    const uint32_t head[kSoloHead] = {0u, n, 0u, pairs, 0u, contacts, 0u, 0u, 0u, kItemBlock, kItemEmpty, kItemEmpty};
+    const uint32_t head[kSoloHead] = {0u, n, 0u, pairs, 0u, contacts};
     if (fused_smem_prepare() != DYPH_OK || run_words(w) != DYPH_OK ||
         cudaMalloc(&w->s_buf, words * sizeof(uint32_t)) != cudaSuccess ||
         cudaMemcpy(w->s_buf, head, sizeof(head), cudaMemcpyHostToDevice) != cudaSuccess || setup_done() != DYPH_OK) {
@@ -821,7 +819,7 @@ dyph_status fused_smem_prepare() {
                           reinterpret_cast<const void*>(scene_frame_kernel<5, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_kernel<6, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads>),
-                          reinterpret_cast<const void*>(scene_frame_kernel<2, kSceneWideThreads, true>),
+                          reinterpret_cast<const void*>(scene_single_kernel<kSceneWideThreads>),
                           reinterpret_cast<const void*>(scene_frame_record_kernel<4, kSceneThreads>),
                           reinterpret_cast<const void*>(scene_frame_record_kernel<2, kSceneWideThreads>),
                           reverse_kernel()})
