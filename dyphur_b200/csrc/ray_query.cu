@@ -206,23 +206,45 @@ struct RayRecords {
     uint4* leaves;
     // [0] largest excess (float bits), [1] 1 when the tree or a body is outside the
     // assumptions, [2] complement of the smallest sphere radius's bits (0: no sphere),
-    // [3] leaf boxes out of every finite ray's reach
+    // [3] leaf boxes out of every finite ray's reach, [4] the bodies' hx + hy + hz
+    // summed (float)
     uint32_t* words;
 };
+constexpr size_t kRayWords = 8;
 
-// A tree of fewer bodies is walked as it is. The walk in leaf order and this one:
-// 900 and 252 us for 64 rays at random into a pile of 65,537 bodies, 1,478 and 526
-// for 131,072, 6,364 and 2,676 for a million; 2,790 and 2,730 for a million at
-// 16,385 bodies, 1,852 and 2,474 at 8,193. A million camera rays: 715 and 621 us
-// at 65,537, 464 and 439 at 16,385.
-constexpr uint32_t kRayRecordsBodies = 16384;
+// A tree of fewer bodies, and a query of fewer rays, is walked as it is: the scratch
+// and two more launches cost 8 us at 16,385 bodies and 20 at 65,537 (a query whose
+// rays all miss the pile at once, of 64 or 65,536 rays: 52 and 73, 60 and 94 us). The walk
+// in leaf order and this one, in us by rays (random through the whole pile; short ones,
+// three body lengths; downwards from 3 m above a body; a camera's) and bodies:
+//            1 ray    8       64         4,096      65,536      a million
+//   random   88>80    175>195 378>306    564>293    654>383     3,082>2,867  16,385 bodies
+//            71>73    361>155 1,113>297  1,476>434  1,848>486   8,719>2,937  65,537
+//   short    36>48    80>74   120>101    162>109    189>114       909>667    16,385
+//            64>68    147>124 267>190    339>211    383>215     2,028>1,434  65,537
+//   down     56>59    94>84   150>111    185>114    209>120     1,105>757    16,385
+//            113>103  203>152 332>212    414>227    457>242     2,752>1,697  65,537
+//   camera   37>47    49>58   186>148    224>148    257>204     1,282>1,091  16,385
+// and at 8,193 bodies a million random rays took 1,852 and 2,474 us.
+constexpr uint32_t kRayRecordsBodies = 16384, kRayRecordsRays = 8;
 // Nodes that a ray visits in leaf order before it looks for a bound first. Leaf
 // order is Morton order, which ascends in every coordinate: the more a ray does,
-// the nearer it comes to meeting the near leaves first anyway.
+// the nearer it comes to meeting the near leaves first anyway. A million rays, random
+// (up, across and down that order) and a camera's (across), into 16,385 bodies, and
+// into the burst pile of 65,537:
+//   384/96/24 2,804, 1,307 and 7,870 us; half of each 2,715, 1,804 and 7,110; twice
+//   each 2,939, 1,046 and 7,730; 576 or 768 up as 384; across 192 2,891, 1,040 and
+//   7,950; across 128 2,867, 1,091 and 7,870.
 __device__ __forceinline__ uint32_t ray_steps(const dyph_ray& r) {
     const float s = (r.dx + r.dy + r.dz) / (fabsf(r.dx) + fabsf(r.dy) + fabsf(r.dz));
-    return s > 0.25f ? 384u : (s > -0.25f ? 96u : 24u);
+    return s > 0.25f ? 384u : (s > -0.25f ? 128u : 24u);
 }
+// A ray no longer than this many of the bodies' mean hx + hy + hz goes in leaf order
+// to its end: few leaves lie along it, and the bound and the fold would each visit
+// most of them again. A million short rays as above, all of them to the end and by
+// steps: 667 and 1,315 us into 16,385 bodies, 1,434 and 2,443 into 65,537; with 10 in
+// place of 16 the rays downwards (12 long) took 1,241 and 1,689 instead of 752 and 1,694.
+constexpr float kRayShort = 16.f;
 
 // The node index and the height of the reference's stack share a stack word.
 constexpr uint32_t kRayNodeBits = 26;
@@ -251,7 +273,7 @@ __device__ __forceinline__ bool box_holds(const BoxF& a, const BoxF& b) {
 __global__ void __launch_bounds__(256) ray_records_kernel(dyph_bvh_view bvh, RayScene S, RayRecords R) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint4* boxes = reinterpret_cast<const uint4*>(bvh.aabb);
-    float excess = 0.f;
+    float excess = 0.f, extent = 0.f;
     uint32_t small = 0u;
     bool odd = false, away = false;
     if (i < bvh.n) {
@@ -299,6 +321,7 @@ __global__ void __launch_bounds__(256) ray_records_kernel(dyph_bvh_view bvh, Ray
             // bounds what kRayWide leaves; and the leaf tests' terms in the size
             const float size = type == kShapeSphere ? 5e-3f * hx : 1e-4f * (hx + hy + hz);
             excess = 1.00001f * fmaxf(over, 0.f) + 1e-5f * (ex + ey + ez) + size + 1e-6f;
+            extent = fminf(type == kShapeSphere ? 3.f * hx : hx + hy + hz, 1e6f);
             if (type == kShapeSphere) small = ~bits(fabsf(hx));
             odd = odd || !(hx >= 0.f) || !isfinite(fabsf(px) + fabsf(py) + fabsf(pz) + ex + ey + ez) ||
                   !(excess < 1e6f);
@@ -308,11 +331,14 @@ __global__ void __launch_bounds__(256) ray_records_kernel(dyph_bvh_view bvh, Ray
     const bool any_odd = __any_sync(0xffffffffu, odd);
     const uint32_t n_away = __popc(__ballot_sync(0xffffffffu, away));
     small = __reduce_max_sync(0xffffffffu, small);
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) extent += __shfl_xor_sync(0xffffffffu, extent, d);
     if ((threadIdx.x & 31u) == 0u) {
         if (small) atomicMax(&R.words[2], small);
         if (e) atomicMax(&R.words[0], e);
         if (any_odd) R.words[1] = 1u;
         if (n_away) atomicAdd(&R.words[3], n_away);
+        atomicAdd(reinterpret_cast<float*>(&R.words[4]), extent);  // (a rounded sum only moves the rule's line)
     }
 }
 
@@ -486,14 +512,16 @@ __global__ void __launch_bounds__(kRayThreads) ray_walk_kernel(dyph_bvh_view bvh
     const bool plain = R.words[1] != 0u || !isfinite(fabsf(r.ox) + fabsf(r.oy) + fabsf(r.oz)) ||
                        !isfinite(fabsf(w.ix) + fabsf(w.iy) + fabsf(w.iz)) || !(d2 > 1e-20f && d2 < 1e20f) ||
                        !(r.t_max > 0.f) || (R.words[3] != 0u && !isfinite(r.t_max));
-    if (!w.in_order(root, plain ? ~0u : ray_steps(r))) {
+    const float length = __fsqrt_rn(d2);
+    const bool near = r.t_max * length * static_cast<float>(bvh.n) <= kRayShort * __uint_as_float(R.words[4]);
+    if (!w.in_order(root, plain || near ? ~0u : ray_steps(r))) {
         float W = w.bound(root, w.best_t);
         bool done = !w.deep && W == r.t_max;  // nothing is entered and hit before t_max
         if (done) {
             w.best_t = r.t_max;
             w.best_body = kRayNone;
         }
-        const float slack = __uint_as_float(R.words[0]), length = __fsqrt_rn(d2);
+        const float slack = __uint_as_float(R.words[0]);
         const uint32_t small = R.words[2];
         const float inv_radius = small ? 1.f / __uint_as_float(~small) : 0.f;
         for (int k = 0; k < 8 && !done && !w.deep; ++k) {
@@ -546,8 +574,8 @@ struct RelaxedCapture {
 
 // A captured query takes no scratch: it would put an allocation into the caller's
 // graph, which could then be instantiated only once at a time and not become part of
-// another graph. A million random rays into the settled 65,537-body pile take 6.4 ms
-// so instead of 2.7.
+// another graph. A million random rays into a settled 65,537-body pile take 8.7 ms so
+// instead of 2.9.
 bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(s, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
@@ -650,16 +678,16 @@ extern "C" dyph_status dyph_ray_query(const dyph_bvh_view* bvh, const dyph_bodie
     if (bvh->n > bodies->n) return DYPH_ERR_INVALID;
     const uint32_t grid = (n_rays + kRayThreads - 1) / kRayThreads;
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
-    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies && !capturing(cs)) {
+    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies && n_rays >= kRayRecordsRays && !capturing(cs)) {
         const RelaxedCapture relaxed;
         const size_t node_bytes = 32ull * bvh->n, leaf_bytes = 64ull * bvh->n;
         void* ws = nullptr;
         cudaMemPool_t pool = ray_pool();
-        if (pool && cudaMallocFromPoolAsync(&ws, node_bytes + leaf_bytes + 16, pool, cs) == cudaSuccess) {
+        if (pool && cudaMallocFromPoolAsync(&ws, node_bytes + leaf_bytes + 4 * kRayWords, pool, cs) == cudaSuccess) {
             char* base = static_cast<char*>(ws);
             const RayRecords R{reinterpret_cast<uint4*>(base), reinterpret_cast<uint4*>(base + node_bytes),
                                reinterpret_cast<uint32_t*>(base + node_bytes + leaf_bytes)};
-            cudaError_t e = cudaMemsetAsync(R.words, 0, 16, cs);
+            cudaError_t e = cudaMemsetAsync(R.words, 0, 4 * kRayWords, cs);
             if (e == cudaSuccess) {
                 ray_records_kernel<<<(bvh->n + 255) / 256, 256, 0, cs>>>(*bvh, RayScene{*bodies, *shapes}, R);
                 ray_walk_kernel<<<grid, kRayThreads, 0, cs>>>(*bvh, R, d_rays, d_hits, n_rays);

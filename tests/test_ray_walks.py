@@ -133,3 +133,37 @@ def test_captured_query(n):
         g.replay()
         torch.cuda.synchronize()
         assert torch.equal(t.view(torch.int32), wt.view(torch.int32)) and torch.equal(body, wb)
+
+
+@pytest.mark.parametrize("n_rays", [1, 7, 8, 9, 4000])
+def test_few_and_short_rays(oracle_mod, n_rays):
+    """On both sides of the rules on the number of rays and on a ray's length, which
+    is the same whether the direction or t_max carries it."""
+    from dyphur_b200 import device
+    scene = scenes.random_pile(16400, seed=3)
+    o = oracle_mod.World(scene)
+    assert o.step(20) == 0
+    st = o.state()
+    o.stage(oracle_mod.STAGE_BROADPHASE)
+    b, sh = device.DeviceBodies(scene), device.DeviceShapes(scene)
+    b.set_state(st)
+    bp = device.Broadphase(scene.n_bodies, scene.max_pairs)
+    bp.build_and_query(b, sh, scene.bounds[0])
+    half = scene.shape_half[scene.shape]
+    size = np.where(scene.shape_type[scene.shape] == 1, 3 * half[:, 0], half.sum(1)).mean()
+    rng = np.random.default_rng(n_rays)
+    d = rng.normal(size=(n_rays, 3))
+    d /= np.linalg.norm(d, axis=1, keepdims=True)
+    length = 16 * size * rng.choice([0.1, 0.5, 0.999, 1.0, 1.001, 2.0, 30.0], n_rays)
+    t_max = rng.choice([1e-3, 1.0, 50.0], n_rays)
+    at = st[:3, rng.integers(0, scene.n_bodies, n_rays)].T
+    rays = np.empty((n_rays, 7), np.float32)
+    rays[:, 3:6] = d * (length / t_max)[:, None]
+    rays[:, :3] = at - d * (length * rng.uniform(0, 1, n_rays))[:, None]
+    rays[:, 6] = t_max
+    want_t, want_b = o.ray_query(rays)
+    t, body = device.ray_query(bp.bvh_view(scene.n_bodies), b, sh, rays)
+    assert np.array_equal(bits(t.cpu().numpy()), bits(want_t))
+    assert np.array_equal(body.cpu().numpy().view(np.uint32), want_b)
+    assert (want_b != 0xFFFFFFFF).any()
+    assert device.device_error() == 0
