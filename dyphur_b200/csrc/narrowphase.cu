@@ -189,9 +189,11 @@ dyph_status narrowphase_reserve(dyph_narrowphase* np, uint32_t max_pairs) {
 }
 
 // Bodies of a scene from which on they are packed: one more launch, 3 us. The
-// stage with and without: 127 and 137 us on the settled 65,537-body pile, 31 and
-// 33 on 20,002 bodies.
-constexpr uint32_t kPackedBodies = 8192;
+// stage without and with: 137 and 127 us on the settled 65,537-body pile; called by
+// itself, 55.6 and 53.8 us on a pile of 28,000, 41.8 and 42.4 on 20,002, 38.9 and 42.2
+// on 16,000, 36.5 and 38.8 on 8,193, and 28 and 31 us on bodies apart from one another
+// at each of those sizes.
+constexpr uint32_t kPackedBodies = 32768;
 
 dyph_status narrowphase_reserve_bodies(dyph_narrowphase* np, uint32_t n) {
     if (n < kPackedBodies || n <= np->packed_n) return DYPH_OK;

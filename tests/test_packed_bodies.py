@@ -36,11 +36,33 @@ def test_contacts_match_oracle(oracle_mod, n):
     assert device.device_error() == 0
 
 
-def test_one_handle_grows():
+@pytest.mark.parametrize("n", [32767, 32768, 32769])
+def test_contacts_match_oracle_at_the_line(oracle_mod, n):
+    from dyphur_b200 import device
+    s = scenes.random_pile(n - 1, seed=n)  # and the ground
+    w = device.World(s)
+    w.step(45)
+    st = w.state()
+    o = oracle_mod.World(s)
+    o.set_state(st)
+    o.stage(oracle_mod.STAGE_BROADPHASE)
+    o.stage(oracle_mod.STAGE_NARROWPHASE)
+    ab, p7 = o.contacts()
+    bp, npz = device.Broadphase(n, s.max_pairs), device.Narrowphase(s.max_contacts)
+    bp.build_and_query(w.bodies, w.shapes, s.bounds[0])
+    npz.run(bp, w.bodies, w.shapes)
+    got_ab, got_p7 = npz.contacts()
+    assert len(ab) > 1000
+    assert np.array_equal(got_ab, ab) and np.array_equal(bits(got_p7), bits(p7))
+    assert device.device_error() == 0
+
+
+@pytest.mark.parametrize("sizes", [(8200, 9000), (33000, 36000)])
+def test_one_handle_grows(sizes):
     import torch
     from dyphur_b200 import device
     parts = []
-    for n in (8200, 9000):
+    for n in sizes:
         s = scenes.random_pile(n, seed=n)
         w = device.World(s)
         w.step(45)
