@@ -77,7 +77,8 @@ struct dyph_world {
     std::vector<float*> a_qs;        // [4][n]
     std::vector<uint32_t*> a_words;  // [kSceneWords][f_words_stride]
     std::vector<uint32_t*> a_mg;     // [2 n_scenes]
-    AdjSet* a_sets = nullptr;        // [a_rec.size()] the record sets, for the kernels
+    AdjSet* a_sets = nullptr;        // [a_sets_n] the record sets, for the kernels
+    size_t a_sets_n = 0;
     float* a_g = nullptr;            // [13][n] the state's adjoint
     float* a_seg[2] = {nullptr, nullptr};  // [a_seg_frames][13][n] states of frames 1.. of a segment (double buffer)
     uint32_t a_seg_frames = 0;
@@ -1407,6 +1408,7 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
         w->a_mg.clear();
         if (w->a_sets) cudaFree(w->a_sets);
         w->a_sets = nullptr;
+        w->a_sets_n = 0;
         if (w->a_pairs) cudaFree(w->a_pairs);
         w->a_pairs = nullptr;
         std::fill(w->a_sized, w->a_sized + 4, 0u);
@@ -1414,7 +1416,6 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
             return DYPH_ERR_NOMEM;
         std::copy(sized, sized + 4, w->a_sized);
     }
-    const bool grow = w->a_rec.size() < sets;
     while (w->a_rec.size() < sets) {
         float *rec = nullptr, *pose1 = nullptr, *qs = nullptr;
         uint32_t *words = nullptr, *mg = nullptr;
@@ -1435,16 +1436,19 @@ dyph_status adjoint_buffers(dyph_world* w, uint32_t sets, uint32_t seg_states) {
         w->a_words.push_back(words);
         w->a_mg.push_back(mg);
     }
-    if (grow || !w->a_sets) {
+    // (a call that ran out of memory may have left sets that the table does not have)
+    if (w->a_sets_n != w->a_rec.size()) {
         std::vector<AdjSet> table(w->a_rec.size());
         for (size_t k = 0; k < table.size(); ++k)
             table[k] = AdjSet{w->a_rec[k], w->a_pose1[k], w->a_qs[k], w->a_words[k], w->a_mg[k]};
         if (w->a_sets) cudaFree(w->a_sets);
         w->a_sets = nullptr;
+        w->a_sets_n = 0;
         if (cudaMalloc(&w->a_sets, table.size() * sizeof(AdjSet)) != cudaSuccess) return DYPH_ERR_NOMEM;
         // read by the recordings on a_stream and by the reversals that wait for them
         DYPH_CUDA_TRY(cudaMemcpyAsync(w->a_sets, table.data(), table.size() * sizeof(AdjSet), cudaMemcpyHostToDevice,
                                       w->a_stream));
+        w->a_sets_n = table.size();
     }
     if (seg_states > w->a_seg_frames) {
         for (float*& b : w->a_seg) {
@@ -1491,8 +1495,8 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     for (;;) {
         const uint32_t seg_frames = static_cast<uint32_t>(std::min(group, n_frames));
         st = adjoint_buffers(w, 2u * seg_frames, every > 1 ? seg_frames - 1u : 0u);
+        if (st == DYPH_ERR_NOMEM) cudaGetLastError();  // the failed allocation
         if (st != DYPH_ERR_NOMEM || every > 1 || group == 1) break;
-        cudaGetLastError();  // the failed allocation
         group = 1;
     }
     if (st != DYPH_OK) return st;

@@ -78,3 +78,39 @@ def test_first_backward_pass(every):
         got.append((bits(g_init.cpu().numpy()), bits(g_im.cpu().numpy())))
     assert np.any(got[0][0]) and all(np.array_equal(x, y) for x, y in zip(*got))
     assert device.device_error() == 0
+
+
+def test_backward_pass_after_one_that_ran_out_of_memory():
+    """Some of a pass's record sets were made, then the memory ran out: a smaller pass
+    that finds enough of them there runs on them."""
+    import torch
+    from dyphur_b200 import capi, device
+    s = scenes.push(128)
+    n = s.n_bodies
+
+    def gradients(w, frames):
+        ckpt = torch.zeros((1, 13, n), device="cuda")
+        w.bodies.fbuf[:13, :n] = w.initial_rows()[:13, :n]
+        w.rollout_raw(frames, frames, ckpt.data_ptr(), torch.cuda.current_stream().cuda_stream)
+        g_final, g_init, g_im = torch.ones((13, n), device="cuda"), torch.zeros((13, n), device="cuda"), \
+            torch.zeros(n, device="cuda")
+        w.rollout_backward_raw(frames, frames, ckpt.data_ptr(), g_final.data_ptr(), g_init.data_ptr(), g_im.data_ptr(),
+                               torch.cuda.current_stream().cuda_stream)
+        torch.cuda.synchronize()
+        return bits(g_init.cpu().numpy()), bits(g_im.cpu().numpy())
+
+    w, fresh = device.World(s, mode=1), device.World(s, mode=1)
+    gradients(w, 1)  # two sets
+    before = torch.cuda.mem_get_info()[0]
+    want = gradients(fresh, 2)  # four sets
+    four = before - torch.cuda.mem_get_info()[0]
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    hog = torch.empty(free - four, dtype=torch.uint8, device="cuda")  # room for some four more
+    with pytest.raises(capi.DyphError):
+        gradients(w, 12)
+    del hog
+    torch.cuda.empty_cache()
+    got = gradients(w, 2)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    assert device.device_error() == 0
