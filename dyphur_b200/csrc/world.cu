@@ -379,14 +379,15 @@ dyph_status enqueue_run(dyph_world* w, cudaStream_t s, uint64_t frame0, uint32_t
 
 // One frame; when probe_stage matches a stage (0 integrate, 1 broadphase,
 // 2 narrowphase, 3 solver) the events are recorded around it; probe_stage 4
-// records them around the solver's dataflow kernel alone.
+// records them around the solver's dataflow kernel alone. keep: the last frame of a
+// call (a fused batch stores no lists before it).
 dyph_status enqueue_frame(dyph_world* w, cudaStream_t s, int probe_stage = -1, void* ev0 = nullptr,
-                          void* ev1 = nullptr) {
+                          void* ev1 = nullptr, bool keep = true) {
     const dyph_world_desc& d = w->desc;
     dyph_status st;
     if (w->fused) {
         if (probe_stage >= 0 && (st = probe_record(ev0, s)) != DYPH_OK) return st;
-        if ((st = launch_run(w, FusedRun{1u}, s)) != DYPH_OK) return st;
+        if ((st = launch_run(w, FusedRun{1u, keep}, s)) != DYPH_OK) return st;
         return probe_stage >= 0 ? probe_record(ev1, s) : DYPH_OK;
     }
     w->sv->probe_flow[0] = probe_stage == 4 ? ev0 : nullptr;
@@ -637,7 +638,7 @@ extern "C" dyph_status dyph_world_capture_episode(dyph_world* w, int32_t n_frame
         for (int32_t f = f0; f < n_frames && st == DYPH_OK; ++f) {
             // a probed fused frame is a launch of its own between the events
             st = enqueue_frame(w, w->stream, probe_stage, probe_stage >= 0 ? ev_start[f] : nullptr,
-                               probe_stage >= 0 ? ev_end[f] : nullptr);
+                               probe_stage >= 0 ? ev_end[f] : nullptr, f + 1 == n_frames);
             if (st == DYPH_OK && trajectory_frame(w, static_cast<uint64_t>(f))) {
                 last = static_cast<uint64_t>(f) / w->traj_every;
                 st = enqueue_trajectory_record(w, w->stream, last, last >= 2);
@@ -1186,12 +1187,12 @@ extern "C" dyph_status dyph_world_autotune(dyph_world* w, int32_t frames, dyph_s
                 w->f_variant = variant;
                 st = setup_fused(w, static_cast<uint32_t>(w->h_body_offset.size() - 1), w->h_body_offset.data());
                 if (st != DYPH_OK) break;
-                // one untimed frame, then the timed ones as one run, each trial from the saved state
-                st = launch_run(w, FusedRun{1u}, w->stream);
+                // one untimed frame, then the timed ones launched as a call's, each trial from the saved state
+                st = launch_run(w, FusedRun{1u, false}, w->stream);
                 if (st == DYPH_OK && cudaEventRecord(e0, w->stream) != cudaSuccess) st = DYPH_ERR_CUDA;
-                const uint32_t run = w->f_resident ? kMaxRunFrames : 1u;
-                for (uint32_t f = 0; f < static_cast<uint32_t>(frames) && st == DYPH_OK; f += run)
-                    st = launch_run(w, FusedRun{std::min(static_cast<uint32_t>(frames) - f, run)}, w->stream);
+                const uint32_t all = static_cast<uint32_t>(frames), run = w->f_resident ? kMaxRunFrames : 1u;
+                for (uint32_t f = 0; f < all && st == DYPH_OK; f += run)
+                    st = launch_run(w, FusedRun{std::min(all - f, run), all - f <= run}, w->stream);
                 if (st == DYPH_OK && cudaEventRecord(e1, w->stream) != cudaSuccess) st = DYPH_ERR_CUDA;
                 if (st == DYPH_OK && (copy_rows(false) != cudaSuccess || cudaStreamSynchronize(w->stream) != cudaSuccess))
                     st = DYPH_ERR_CUDA;

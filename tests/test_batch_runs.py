@@ -110,3 +110,18 @@ def test_status_is_the_first_frames_to_overflow(pairs, contacts):
     b.step(8)
     assert (seen[0] != 0) == (min(pairs, contacts) == 1000) and seen[-1] != 0
     assert a.stats() == b.stats()
+
+
+def test_probed_episode_keeps_the_last_frames_lists():
+    """Frames timed one by one store their lists as a call's do: the last one's are kept."""
+    a, b = _world(), _world()
+    a.step(9)
+    b.capture_episode(9, probe_stage=0)
+    b.run_episode()
+    assert (b.probe_ms() > 0).all()
+    assert np.array_equal(bits(a.state()), bits(b.state())) and a.stats() == b.stats()
+    for x, y in zip(a.history(), b.history()):
+        assert np.array_equal(x, y)
+    assert len(a.pairs()) > 0 and np.array_equal(a.pairs(), b.pairs())
+    (ab, pa), (bb, pb) = a.contacts(), b.contacts()
+    assert np.array_equal(ab, bb) and np.array_equal(bits(pa), bits(pb)) and a.solver_stats() == b.solver_stats()
