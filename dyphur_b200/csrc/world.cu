@@ -548,6 +548,11 @@ dyph_status enqueue_solo(dyph_world* w, cudaStream_t s, uint32_t n_frames) {
 // dyph_world_step; a fused batch also writes checkpoints (dyph_world_rollout).
 dyph_status world_step(dyph_world* w, int32_t n_frames, dyph_stream s, float* ckpt = nullptr, uint32_t ckpt_every = 1) {
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
+    // Not in a caller's capture: the host counts the frames of each call, and a new
+    // layout gives back the buffers that recorded launches would go on using.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DYPH_CUDA_TRY(cudaStreamIsCapturing(cs, &capture));
+    if (capture != cudaStreamCaptureStatusNone) DYPH_CUDA_TRY(cudaErrorStreamCaptureUnsupported);
     DYPH_CUDA_TRY(cudaEventRecord(w->ev_in, cs));
     DYPH_CUDA_TRY(cudaStreamWaitEvent(w->stream, w->ev_in, 0));
     uint64_t last = 0;

@@ -362,7 +362,9 @@ typedef struct dyph_world_desc {
 typedef struct dyph_world dyph_world;
 dyph_status dyph_world_create(const dyph_world_desc* desc, dyph_stream s, dyph_world** out);
 void dyph_world_destroy(dyph_world* w);
-/* Queue n_frames frame steps (graph-replayed after the first call). */
+/* Queue n_frames frame steps on the world's own stream, ordered after and
+ * before the work on s. DYPH_ERR_CUDA while s is captured: a world's frames are
+ * not recorded in a caller's graph (dyph_world_capture_episode has its own). */
 dyph_status dyph_world_step(dyph_world* w, int32_t n_frames, dyph_stream s);
 /* Batched scenes in one world (dyph_broadphase_set_scenes; desc.scene_bounds is
  * then unused). No reference counterpart: the reference steps one scene per

@@ -40,6 +40,35 @@ def test_frames_beside_a_capture(n):
     assert device.device_error() == 0
 
 
+@pytest.mark.parametrize("kind", ["small", "single", "batch"])
+def test_steps_are_not_recorded(kind):
+    """A world's frames are refused inside a capture, which goes on without them."""
+    import torch
+    from dyphur_b200 import device
+    s = {"small": scenes.random_pile(40, seed=1), "single": scenes.random_pile(600, seed=1),
+         "batch": scenes.batch(5, 5, 30, seed=1)}[kind]
+    a, b = device.World(s), device.World(s)
+    for w in (a, b):
+        w.step(1)
+    x, ckpt = torch.zeros(64, device="cuda"), torch.zeros((1, 13, s.n_bodies), device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        for frames in (1, 4):
+            with pytest.raises(capi.DyphError):
+                b.step(frames)
+        with pytest.raises(capi.DyphError):
+            b.rollout_raw(2, 2, ckpt.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    g.replay()
+    torch.cuda.synchronize()
+    assert float(x.sum()) == 64
+    a.step(4)
+    b.step(4)
+    assert np.array_equal(bits(a.state()), bits(b.state())) and a.stats() == b.stats()
+    assert device.device_error() == 0
+
+
 FIRST_QUERY = """
 import ctypes as C
 import torch
