@@ -400,12 +400,6 @@ struct SideBody {
 };
 
 template <class Bodies>
-__device__ __forceinline__ SideBody load_side(const Bodies& B, uint32_t i) {
-    return SideBody{B.px(i), B.py(i), B.pz(i), B.qw(i), B.qx(i), B.qy(i), B.qz(i), B.vx(i), B.vy(i), B.vz(i),
-                    B.wx(i), B.wy(i), B.wz(i), B.im(i), B.ixx(i), B.iyy(i), B.izz(i), B.ixy(i), B.ixz(i), B.iyz(i)};
-}
-
-template <class Bodies>
 __device__ __forceinline__ void store_side(const Bodies& B, uint32_t i, const SideBody& s) {
     B.px(i) = s.px; B.py(i) = s.py; B.pz(i) = s.pz;
     B.qw(i) = s.qw; B.qx(i) = s.qx; B.qy(i) = s.qy; B.qz(i) = s.qz;

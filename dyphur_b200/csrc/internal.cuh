@@ -159,7 +159,7 @@ dyph_status sort_prepare();
 
 // The adjoint's reverse kernel (reverse.cu, its own translation unit), for
 // cudaLaunchKernel with the argument list (SceneBufs, FrameBufs, FrameParams,
-// AdjRun, AdjKeep, AdjFrame, const uint32_t* items, uint32_t n_items).
+// AdjSegment, AdjFrame, const uint32_t* items, uint32_t n_items).
 const void* reverse_kernel();
 
 dyph_status integrate_launch(const dyph_bodies* bodies, const dyph_integrator_params* p, cudaStream_t s);

@@ -1,9 +1,9 @@
 // The adjoint's reverse kernel, the library's second translation unit.
 //
-// It is compiled with contracted multiply-adds and approximate division and
-// square root, unlike every other kernel (dyphur_b200.cu keeps each float
-// operation correctly rounded and uncontracted, which the bit-exact forward
-// frame and its recording need). The reverse pass only follows the branches
+// It is compiled with approximate division and square root, unlike every other
+// kernel (dyphur_b200.cu keeps each float operation correctly rounded, which the
+// bit-exact forward frame and its recording need); multiply-adds are contracted
+// where the code says so (__fmaf_rn), as nowhere else. The reverse pass only follows the branches
 // the recording fixed (contact set, narrowphase features, solve flags, clamp
 // bits); the signs it recomputes are of quantities that are zero by
 // construction (their terms cancel) or far from zero, and its gradients are

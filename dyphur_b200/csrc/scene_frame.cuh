@@ -513,7 +513,7 @@ __device__ __forceinline__ ItemTeam item_team(const uint32_t* item, uint32_t sme
 }
 
 // kMinBlocks is the register budget: 4 resident blocks of kSceneThreads per SM
-// (128 registers a thread), 5 (96) or 6 (80, a few bytes spilled), or 2 of
+// (128 registers a thread), 5 (96, 88 bytes of them spilled) or 6 (80, 112), or 2 of
 // kSceneWideThreads (128). Which one runs best depends on the batch
 // (dyph_world_autotune picks the budget with the shared memory cap; the wide
 // form's rule is in setup_fused); all compute the same frames.

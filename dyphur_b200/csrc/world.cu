@@ -468,7 +468,8 @@ dyph_status fused_smem_prepare();
 // A frame, one block against the stage kernels: 17 and 66 us on 9 stacked boxes,
 // 113 and 177 on 201, 156 and 181 on 289, 273 and 208 on 433; in the sequential
 // order, whose chains leave a chip idle, 322 and 725 us on 433; 27 and 82 us on a
-// loose pile of 400.
+// loose pile of 400. The lines stay below the size where a dense stack, whose levels
+// one block takes one after another, is slower on it.
 constexpr uint32_t kSoloBodies = 256, kSoloSequentialBodies = 512;
 bool solo_size(const dyph_world* w) {
     return w->desc.bodies.n <= (w->sv->mode == DYPH_SOLVER_SEQUENTIAL ? kSoloSequentialBodies : kSoloBodies);
@@ -1485,13 +1486,12 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
         !d_grad_inv_mass)
         return DYPH_ERR_INVALID;
     // Frames are recorded in segments on a_stream, one launch a segment and one
-    // record set per frame;
-    // sets alternate between two segments, so segment seg - 1 is recorded
-    // while segment seg is reversed on the caller's stream, last frame first.
-    // With checkpoints every `every` > 1 frames a segment is a checkpoint's
-    // frames, each recorded from the state the one before stored; with a
-    // checkpoint at every frame it is up to kRecordGroup frames, each recorded
-    // from its own checkpoint (one frame when that many sets do not fit).
+    // record set per frame; sets alternate between two segments, so segment
+    // seg - 1 is recorded while segment seg is reversed on the caller's stream,
+    // last frame first. With checkpoints every `every` > 1 frames a segment is a
+    // checkpoint's frames; with a checkpoint at every frame it is up to
+    // kRecordGroup frames (one frame when that many sets do not fit). The
+    // recording loads the segment's first checkpoint and goes on from there.
     int32_t group = every;
     if (every == 1) {
         const size_t sets = kRecordBudget / (2 * record_set_bytes(w));
@@ -1522,9 +1522,10 @@ extern "C" dyph_status dyph_world_rollout_backward(dyph_world* w, int32_t n_fram
     S_rev.smem_bytes = w->r_smem;
     auto seg_len = [&](int32_t seg) { return std::min(group, n_frames - seg * group); };
     auto ckpt = [&](int32_t c) { return d_ckpt + static_cast<size_t>(c) * 13 * n; };
-    // Segment seg's frames. Frame f starts from its segment's checkpoint, or from
-    // the state its predecessor's recording stored (with a checkpoint at every
-    // frame, from its own checkpoint). The kernels only read a checkpoint.
+    // Segment seg's frames. The state that the reversal of frame f starts from is
+    // its segment's checkpoint, or what its predecessor's recording stored (with a
+    // checkpoint at every frame, its own checkpoint, the same bits). The kernels
+    // only read a checkpoint.
     auto segment = [&](int32_t seg) {
         float* state1 = every > 1 ? w->a_seg[seg & 1] : const_cast<float*>(ckpt(seg * group)) + 13 * n;
         const float* state0 = ckpt(every > 1 ? seg : seg * group);
