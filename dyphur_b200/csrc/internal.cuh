@@ -154,6 +154,15 @@ dyph_status xpbd_set_scenes(dyph_xpbd* sv, uint32_t n_scenes, const uint32_t* h_
 // buffers that way ends with this.
 dyph_status setup_done();
 
+// Another stream may be in a capture that forbids calls which could allocate on the
+// way: those of a call that is itself not captured are no part of it, so the thread
+// may make them while this lives.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Pre-set kernel attributes of the sort (call once, outside graph capture).
 dyph_status sort_prepare();
 

@@ -222,6 +222,7 @@ dyph_status narrowphase_run(dyph_narrowphase* np, const dyph_pair* pairs, const 
     bool packed = bodies->n >= kPackedBodies;
     if (packed && bodies->n > np->packed_n) {
         // a capture cannot allocate: its pairs read the bodies' rows
+        const RelaxedCapture relaxed;
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         packed = cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone &&
                  narrowphase_reserve_bodies(np, bodies->n) == DYPH_OK;

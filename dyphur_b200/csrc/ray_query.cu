@@ -19,7 +19,7 @@
 #include <mutex>
 #include <new>
 
-#include "physics.cuh"
+#include "internal.cuh"
 
 namespace dyph {
 namespace {
@@ -562,15 +562,6 @@ cudaMemPool_t ray_pool() {
     }
     return g_ray_pool[dev];
 }
-
-// Another stream may be in a capture that forbids calls which could allocate on the
-// way: those of a query that is itself not captured are no part of it, so the thread
-// may make them while this lives.
-struct RelaxedCapture {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 // A captured query takes no scratch: it would put an allocation into the caller's
 // graph, which could then be instantiated only once at a time and not become part of

@@ -69,6 +69,36 @@ def test_steps_are_not_recorded(kind):
     assert device.device_error() == 0
 
 
+def test_large_narrowphase_beside_a_capture():
+    """A handle's first run on a scene whose bodies it packs, while another stream captures."""
+    import torch
+    from dyphur_b200 import device
+    small, large = scenes.random_pile(50, seed=2), scenes.random_pile(33000, seed=2)
+    npz, other_npz = device.Narrowphase(large.max_contacts), device.Narrowphase(large.max_contacts)
+    parts = []
+    for s in (small, large):
+        w = device.World(s)
+        w.step(45)
+        bp = device.Broadphase(s.n_bodies, 400000)
+        bp.build_and_query(w.bodies, w.shapes, s.bounds[0])
+        parts.append((bp, w.bodies, w.shapes, w))
+    npz.run(*parts[0][:3])
+    other_npz.run(*parts[1][:3])
+    want = other_npz.contacts()
+    x, other = torch.zeros(64, device="cuda"), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        x.add_(1)
+        npz.run(*parts[1][:3], stream=other)
+    g.replay()
+    torch.cuda.synchronize()
+    got = npz.contacts()
+    assert float(x.sum()) == 64 and len(want[0]) > 1000
+    assert np.array_equal(got[0], want[0]) and np.array_equal(bits(got[1]), bits(want[1]))
+    assert device.device_error() == 0
+
+
 FIRST_QUERY = """
 import ctypes as C
 import torch
