@@ -343,9 +343,11 @@ def kernels_per_frame(n: int, n_scenes: int = 1) -> int:
     else:
         sort = 1 if n <= 4096 else 5  # one-block sort, or histogram + 4 onesweep passes
     # integrate, morton, sort, build, finalize, pair search (tiles, or tree walks in two passes), pair
-    # write, narrowphase, solver (dataflow, round-synchronous, sequential: two of them return at once), stats
+    # write, packed bodies, narrowphase, solver (dataflow, round-synchronous, sequential: two of them
+    # return at once), stats
     find = 1 if n_scenes == 1 and n <= 32768 else 2
-    return 1 + 1 + sort + 1 + 1 + find + 1 + 1 + 3 + 1
+    pack = 1 if n >= 32768 else 0
+    return 1 + 1 + sort + 1 + 1 + find + 1 + pack + 1 + 3 + 1
 
 
 def peaks() -> tuple[float, str]:
