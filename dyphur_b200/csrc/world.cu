@@ -465,11 +465,15 @@ dyph_status fused_smem_prepare();
 // block's work instead of a dozen launches that a scene of this size cannot
 // fill. The last frame runs the stage kernels, so the tree, the lists, the
 // colours and the statistics that a program reads after a call are theirs.
-// A frame, one block against the stage kernels: 17 and 66 us on 9 stacked boxes,
-// 113 and 177 on 201, 156 and 181 on 289, 273 and 208 on 433; in the sequential
-// order, whose chains leave a chip idle, 322 and 725 us on 433; 27 and 82 us on a
-// loose pile of 400. The lines stay below the size where a dense stack, whose levels
-// one block takes one after another, is slower on it.
+// A frame in us, one block against the stage kernels, on stacks of boxes and on loose
+// piles, whose few contacts leave the levels short:
+//   reference order   16 / 61 (9)  102 / 138 (201)  148 / 148 (289)  168 / 145 (344)
+//                     pile: 13 / 62 (61)  15 / 68 (201)  25 / 71 (401)  31 / 73 (506)
+//   sequential        128 / 198 (201)  174 / 226 (289)  294 / 291 (433)  280 / 267 (505)
+//                     pile: 25 / 69 (401)  31 / 74 (506)
+// The limits lie where a dense stack breaks even: the count of bodies is all that is
+// known ahead of the frames. A little past it the sequential order still has the pile's
+// gain against 5 % of a stack's time.
 constexpr uint32_t kSoloBodies = 256, kSoloSequentialBodies = 512;
 bool solo_size(const dyph_world* w) {
     return w->desc.bodies.n <= (w->sv->mode == DYPH_SOLVER_SEQUENTIAL ? kSoloSequentialBodies : kSoloBodies);
