@@ -461,7 +461,7 @@ uint32_t fused_smem_floor(uint32_t max_nb);
 dyph_status fused_smem_prepare();
 
 // A single scene of at most this many bodies steps the frames of a call but the
-// last on one block of the fused kernel, in one launch: a frame is then one
+// last on one block (scene_single_kernel), in one launch: a frame is then one
 // block's work instead of a dozen launches that a scene of this size cannot
 // fill. The last frame runs the stage kernels, so the tree, the lists, the
 // colours and the statistics that a program reads after a call are theirs.
@@ -480,8 +480,8 @@ bool solo_size(const dyph_world* w) {
 }
 
 // The one block's buffers, made with the world: a step allocates nothing, since
-// it may run inside a stream capture or beside one. Without them the world steps
-// every frame on the stage kernels.
+// another stream may be in a capture meanwhile. Without them the world steps every
+// frame on the stage kernels.
 void solo_reserve(dyph_world* w) {
     if (!solo_size(w)) return;
     const uint32_t n = w->desc.bodies.n;
