@@ -212,21 +212,23 @@ struct RayRecords {
 };
 constexpr size_t kRayWords = 8;
 
-// A tree of fewer bodies, and a query of fewer rays, is walked as it is: the scratch
-// and two more launches cost 8 us at 16,385 bodies and 20 at 65,537 (a query whose
-// rays all miss the pile at once, of 64 or 65,536 rays: 52 and 73, 60 and 94 us). The walk
-// in leaf order and this one, in us by rays (random through the whole pile; short ones,
+// A tree of fewer bodies is walked as it is, and so is one by few rays, fewer than
+// kRayRecordsWork over its bodies (8 into 16,384, 2 into 65,536): the scratch and two
+// more launches cost 8 us at 16,385 bodies and 20 at 65,537 (a query whose rays all
+// miss the pile at once, of 64 or 65,536 rays: 52 and 73, 60 and 94 us). The walk in
+// leaf order and this one, in us by rays (random through the whole pile; short ones,
 // three body lengths; downwards from 3 m above a body; a camera's) and bodies:
-//            1 ray    8       64         4,096      65,536      a million
-//   random   88>80    175>195 378>306    564>293    654>383     3,082>2,867  16,385 bodies
-//            71>73    361>155 1,113>297  1,476>434  1,848>486   8,719>2,937  65,537
-//   short    36>48    80>74   120>101    162>109    189>114       909>667    16,385
-//            64>68    147>124 267>190    339>211    383>215     2,028>1,434  65,537
-//   down     56>59    94>84   150>111    185>114    209>120     1,105>757    16,385
-//            113>103  203>152 332>212    414>227    457>242     2,752>1,697  65,537
-//   camera   37>47    49>58   186>148    224>148    257>204     1,282>1,091  16,385
+//            1 ray    4       8       64         4,096      65,536      a million
+//   random   88>80    141>135 175>195 378>306    564>293    654>383     3,082>2,867  16,385 bodies
+//            71>73    333>127 361>155 1,113>297  1,476>434  1,848>486   8,719>2,937  65,537
+//   short    36>48    63>62   80>74   120>101    162>109    189>114       909>667    16,385
+//            64>68    104>93  147>124 267>190    339>211    383>215     2,028>1,434  65,537
+//   down     56>59    72>69   94>84   150>111    185>114    209>120     1,105>757    16,385
+//            113>103  147>118 203>152 332>212    414>227    457>242     2,752>1,697  65,537
+//   camera   37>47    49>56   49>58   186>148    224>148    257>204     1,282>1,091  16,385
 // and at 8,193 bodies a million random rays took 1,852 and 2,474 us.
-constexpr uint32_t kRayRecordsBodies = 16384, kRayRecordsRays = 8;
+constexpr uint32_t kRayRecordsBodies = 16384;
+constexpr uint64_t kRayRecordsWork = 1u << 17;  // rays times bodies
 // Nodes that a ray visits in leaf order before it looks for a bound first. Leaf
 // order is Morton order, which ascends in every coordinate: the more a ray does,
 // the nearer it comes to meeting the near leaves first anyway. A million rays, random
@@ -669,7 +671,8 @@ extern "C" dyph_status dyph_ray_query(const dyph_bvh_view* bvh, const dyph_bodie
     if (bvh->n > bodies->n) return DYPH_ERR_INVALID;
     const uint32_t grid = (n_rays + kRayThreads - 1) / kRayThreads;
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(s);
-    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies && n_rays >= kRayRecordsRays && !capturing(cs)) {
+    if (bvh->n >= kRayRecordsBodies && bvh->n <= kRayMaxBodies &&
+        static_cast<uint64_t>(n_rays) * bvh->n >= kRayRecordsWork && !capturing(cs)) {
         const RelaxedCapture relaxed;
         const size_t node_bytes = 32ull * bvh->n, leaf_bytes = 64ull * bvh->n;
         void* ws = nullptr;

@@ -137,8 +137,8 @@ def test_captured_query(n):
 
 @pytest.mark.parametrize("n_rays", [1, 7, 8, 9, 4000])
 def test_few_and_short_rays(oracle_mod, n_rays):
-    """On both sides of the rules on the number of rays and on a ray's length, which
-    is the same whether the direction or t_max carries it."""
+    """On both sides of the rules on the number of rays (8 at this size) and on a ray's
+    length, which is the same whether the direction or t_max carries it."""
     from dyphur_b200 import device
     scene = scenes.random_pile(16400, seed=3)
     o = oracle_mod.World(scene)
